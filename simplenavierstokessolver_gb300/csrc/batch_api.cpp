@@ -1126,7 +1126,7 @@ int sns_batch_diagnostics(sns_batch *b, int slot, double out[11]) {
   BCase t;
   BCUDA(cudaStreamSynchronize(b->stream));
   BCUDA(cudaMemcpy(&t, b->d_cases + slot, sizeof(BCase), cudaMemcpyDeviceToHost));
-  const size_t words = diag_partials_words(t.nx, t.ny);
+  const size_t words = diag_words(t.nx, t.ny);
   if (b->diag_words < words) {
     cudaFree(b->diag);
     b->diag = nullptr;
@@ -1149,13 +1149,11 @@ int sns_batch_diagnostics(sns_batch *b, int slot, double out[11]) {
                           t.uxl[t.par],
                           t.uyl[t.par],
                           t.tl[t.par]};
-  int nb = 0;
-  BCUDA(launch_diag(a, b->diag, &nb, b->stream));
-  count_launches(1);
-  std::vector<double> h(words);
-  BCUDA(cudaMemcpyAsync(h.data(), b->diag, sizeof(double) * words, cudaMemcpyDeviceToHost, b->stream));
+  double *res = nullptr;
+  BCUDA(launch_diag(a, b->diag, &res, b->stream));
+  count_launches(2);
+  BCUDA(cudaMemcpyAsync(out, res, 11 * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   BCUDA(cudaStreamSynchronize(b->stream));
-  diag_finish(h.data(), nb, d.ly, out);
   return SNS_OK;
 }
 

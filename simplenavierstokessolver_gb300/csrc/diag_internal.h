@@ -25,12 +25,15 @@ struct DiagArgs {
   const float *uxl = nullptr, *uyl = nullptr, *tl = nullptr;
 };
 
+constexpr int kDiagOut = 16;  // words kept for the 11 results at the head of the scratch
+// words of device scratch for a grid
+size_t diag_words(int nx, int ny);
+// the block sums and their final sum; *out: the 11 results on the device:
+// divergence max, sum; x, y momentum; kinetic x, y and thermal energy;
+// Nu from wall flux, injection, kinetic dissipation, thermal dissipation.
+// Two launches.
 template <typename F>
-cudaError_t launch_diag(const DiagArgs<F> &a, double *partials, int *nblocks, cudaStream_t st);
-size_t diag_partials_words(int nx, int ny);
-// out: divergence max, sum; x, y momentum; kinetic x, y and thermal energy;
-// Nu from wall flux, injection, kinetic dissipation, thermal dissipation
-void diag_finish(const double *partials, int nblocks, double ly, double out[11]);
+cudaError_t launch_diag(const DiagArgs<F> &a, double *scratch, double **out, cudaStream_t st);
 
 // allocation-free form: block partials in a fixed file-scope device array of
 // kDiagStaticBlocks blocks (672 KiB), the final sum on the device; grids with

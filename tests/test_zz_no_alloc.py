@@ -71,3 +71,30 @@ def test_grids_beyond_the_scratch_are_rejected():
         assert e.value.code == N.SNS_ERR_UNSUPPORTED
         assert "static" in str(e.value) and "4096" in str(e.value)
         assert np.isfinite(_call(c, "sns_diagnostics")).all()  # the allocating form still serves it
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 2), (63, 16), (64, 32), (65, 8), (130, 64)])
+def test_diagnostics_at_block_edges(nx, ny):
+    """both entry points against the oracle's log quantities on seeded fields:
+    columns and rows below, at and past a block's 64 and 16; the tolerance is
+    the sums' round-off, at most n eps of the summed magnitudes"""
+    from oracle.bindings import Config, OracleCase
+    from simplenavierstokessolver_gb300.solver import Case
+
+    rng = np.random.default_rng(4)
+    su, sc = (ny + 2, nx + 1), (ny + 2, nx + 2)
+    cfg = Config(nx, ny, ly=1.5, Ra=1e6, Pr=0.7)
+    o = OracleCase(cfg)
+    o.set_state(rng.uniform(-1, 1, su), rng.uniform(-1, 1, sc), np.zeros(sc), rng.uniform(-0.5, 0.5, sc))
+    o.call("update_boundaries")
+    s = o.get_state()
+    with Case(nx, ny, ly=1.5, Ra=1e6, Pr=0.7) as c:
+        c.set_state(s["ux"], s["uy"], s["p"], s["temp"])
+        got, static = c.diagnostics(), _call(c, "sns_diagnostics_static")
+    want = o.diagnostics()
+    assert np.array_equal(got, static)
+    assert got[0] == want[0]  # the maximum is exact
+    # sum |term| <= cells * max |term|: divergence up to 4 / spacing, momenta 1, Nusselt terms of the wall flux's size
+    eps = np.finfo(float).eps
+    atol = np.array([0, 8 * max(nx, ny) * nx * ny, 2, 2, 2, 2, 2, 2 * nx, 2000, 0, 0]) * nx * ny * eps
+    assert np.all(np.abs(got - want) <= atol + nx * ny * eps * np.abs(want)), (got, want)
