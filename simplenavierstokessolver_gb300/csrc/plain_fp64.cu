@@ -3,9 +3,10 @@
 // Compiled with --fmad=false: every expression below is evaluated with the
 // same IEEE binary64 operations, in the same order, as the reference's C
 // (cited per kernel), so results are bit-identical to it. Divisions by grid
-// spacings become multiplications by exact reciprocals only when every such
-// spacing is a power of two (DevGrid::rcp), where both give the same
-// correctly rounded result.
+// spacings become multiplications by exact reciprocals when every such
+// spacing is a power of two (DevGrid::rcp), and a product and a fused
+// multiply-add that are proven to round like the division otherwise
+// (DevGrid::dv2): the same correctly rounded result either way.
 //
 // On GB300 the FP64 pipe (~0.5 Tops/s) rather than HBM bounds this path, so
 // the kernels minimise FP64 instructions: y-face quantities are carried from
@@ -48,7 +49,10 @@ __device__ __forceinline__ double dv(double a, double d, double rd) {
 __device__ __forceinline__ int wrap_up(int y, int ny) { return y + 1 == ny ? 0 : y + 1; }
 __device__ __forceinline__ int wrap_dn(int y, int ny) { return y == 0 ? ny - 1 : y - 1; }
 
-constexpr int kRows = 8;     // rows marched by one thread in the stencil kernels
+constexpr int kRows = 8;     // rows marched by one thread in the stencil kernels on large grids
+// warps a launch has before its threads march more rows: two per sub-partition
+// (152 SMs of 4)
+constexpr int kMarchWarps = 1216;
 constexpr int kBlockX = 64;  // columns per block: ~6-7 blocks per SM at 512 x 1024 for load balance
 
 // ------------------------------------------------- exact power-of-two products
@@ -69,6 +73,16 @@ constexpr unsigned kP2Span = (0x7feu - 2u * kP2Margin) << 20;
 // c == 2^e: e in the position of the exponent field of the high word
 __device__ __forceinline__ int p2_field(double c) { return (((__double2hiint(c) >> 20) & 0x7ff) - 1023) * (1 << 20); }
 
+// Division by a spacing that is no power of two: x zh + RN(x zl) in one fused
+// multiply-add equals RN(x / y) for the pairs that the host has proven
+// (invariant_divisor): 2 FP64 instructions instead of a division's ~10. The
+// Measured with the marches below: 400 x 512, velocity update 80 -> 45 us. The
+// proof needs numerators away from the ends of the exponent range; others
+// (below 2^-723 and not zero, from 2^877 up, infinities, NaN) clear the row's
+// flag like the products above.
+constexpr unsigned kDivLo = 300u << 20;
+constexpr unsigned kDivSpan = 1600u << 20;
+
 template <bool FAST>
 struct Mul {
   bool ok = true;
@@ -85,7 +99,56 @@ struct Mul {
     }
   }
   __device__ __forceinline__ double half(double x) { return by(x, 0.5, -(1 << 20)); }
+  // x / y by its pair (zh, zl); FAST only
+  __device__ __forceinline__ double div(double x, double zh, double zl) {
+    const unsigned m = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    ok &= ((m | (unsigned)__double2loint(x)) == 0u) | (m - kDivLo < kDivSpan);
+    return __fma_rn(x, zh, __dmul_rn(x, zl));
+  }
 };
+
+// what a row's divisions by the spacings use: (d) the spacing, (r) its
+// reciprocal, (l) the pair's low word, (e) the exponent of a power of two
+struct Spacing {
+  double d, r, l;
+  int e;
+};
+template <bool RCP, bool FAST>
+__device__ __forceinline__ Spacing spacing(double d, double r, const double *l, int i) {
+  Spacing s;
+  s.d = d;
+  s.r = r;
+  s.l = !RCP && FAST ? l[i] : 0.0;
+  s.e = RCP && FAST ? p2_field(r) : 0;
+  return s;
+}
+template <bool RCP, bool FAST>
+__device__ __forceinline__ Spacing spacing_y(double d, double r, double l) {
+  return spacing<RCP, FAST>(d, r, &l, 0);
+}
+// v / spacing
+template <bool RCP, bool FAST>
+__device__ __forceinline__ double over(Mul<FAST> &m, double v, const Spacing &s) {
+  if constexpr (!FAST) {
+    return dv<RCP>(v, s.d, s.r);
+  } else if constexpr (RCP) {
+    return m.by(v, s.r, s.e);
+  } else {
+    return m.div(v, s.r, s.l);
+  }
+}
+// the same outside a row: FAST falls back by itself
+template <bool RCP, bool FAST>
+__device__ __forceinline__ double over_checked(double v, const Spacing &s) {
+  Mul<FAST> m;
+  const double q = over<RCP, FAST>(m, v, s);
+  if constexpr (FAST) {
+    if (!m.ok) return dv<RCP>(v, s.d, s.r);
+  }
+  return q;
+}
+// a column's spacing has no pair: its rows divide
+__device__ __forceinline__ bool no_pair(const Spacing &s) { return (__double2hiint(s.l) & 0x7ff00000) == 0x7ff00000; }
 
 // ---------------------------------------------------------------- temperature
 struct TempArgs {
@@ -101,37 +164,36 @@ struct TempArgs {
 struct TempRow {
   double A, q, gyp, pyp;
 };
+// metrics of column x; bad: a spacing without its pair
+struct TempCol {
+  Spacing cm, cp, f, y;  // DXC(i), DXC(i+1), DXF(i), dy
+  double am, ap;         // advective coefficients and their exponents
+  int e_am, e_ap;
+  bool bad;
+};
 
 template <int IMPX, int IMPY, bool RCP, bool FAST>
-__device__ __forceinline__ bool temp_row(const TempArgs &a, double tc, double gym, double pym, double tp, double tl,
-                                         double tr, double uyp, double uxm, double uxp, double atr, double dcm,
-                                         double dcp, double df, double rcm, double rcp, double rf, double cm,
-                                         double cp, const int *e, TempRow &o) {
+__device__ __forceinline__ bool temp_row(const TempArgs &a, const TempCol &k, double tc, double gym, double pym,
+                                         double tp, double tl, double tr, double uyp, double uxm, double uxp,
+                                         double atr, TempRow &o) {
   Mul<FAST> m;
-  const double dy = a.g.dy, rdy = a.g.rdy, kappa = a.s.kappa;
-  auto D = [&](double v, double d, double rd, int E) {
-    if constexpr (FAST) {
-      return m.by(v, rd, E);
-    } else {
-      return dv<RCP>(v, d, rd);
-    }
-  };
+  const double kappa = a.s.kappa;
+  auto D = [&](double v, const Spacing &s) { return over<RCP, FAST>(m, v, s); };
   auto Cf = [&](double c, double v, int E) {
-    if constexpr (FAST) {
+    if constexpr (FAST && RCP) {
       return m.by(v, c, E);
     } else {
       return c * v;
     }
   };
-  // e: exponents of rcm, rcp, rdy, rf, cm, cp
-  const double gxm = D(tc - tl, dcm, rcm, e[0]);
-  const double gxp = D(tr - tc, dcp, rcp, e[1]);
-  const double gyp = D(tp - tc, dy, rdy, e[2]);
+  const double gxm = D(tc - tl, k.cm);
+  const double gxp = D(tr - tc, k.cp);
+  const double gyp = D(tp - tc, k.y);
   const double pyp = m.half(uyp) * gyp;
-  const double adv1 = -(Cf(cm, uxm, e[4]) * gxm) - (Cf(cp, uxp, e[5]) * gxp);
+  const double adv1 = -(Cf(k.am, uxm, k.e_am) * gxm) - (Cf(k.ap, uxp, k.e_ap) * gxp);
   const double adv2 = -pym - pyp;
-  const double dif1 = D(kappa * (gxp - gxm), df, rf, e[3]);
-  const double dif2 = D(kappa * (gyp - gym), dy, rdy, e[2]);
+  const double dif1 = D(kappa * (gxp - gxm), k.f);
+  const double dif2 = D(kappa * (gyp - gym), k.y);
   double A = adv1 + adv2;
   if (!IMPX) A = A + dif1;
   if (!IMPY) A = A + dif2;
@@ -149,30 +211,28 @@ __device__ __forceinline__ bool temp_row(const TempArgs &a, double tc, double gy
 }
 
 // src/temperature/update.c:11-87 (sources) and :114-122, :221-226 (RK3 update)
-// for column x, rows y0 .. y0+kRows-1. FAST: the products by powers of two in
-// the integer unit, a row outside their range recomputed with FP64 products.
+// for column x, rows y0 .. y0+rows-1. FAST: the products by powers of two in
+// the integer unit and the divisions by their pairs, a row outside their range
+// recomputed with FP64 products and divisions.
 template <int IMPX, int IMPY, bool RCP, bool FAST>
-__device__ __forceinline__ void temp_column(const TempArgs &a, int x, int y0) {
+__device__ __forceinline__ void temp_column(const TempArgs &a, int x, int y0, int rows) {
   const int nx = a.g.nx, ny = a.g.ny;
-  const int y1 = min(y0 + kRows, ny);
+  const int y1 = min(y0 + rows, ny);
   const double *T = a.t_in;
-  const double dcm = a.g.dxc[x], dcp = a.g.dxc[x + 1], df = a.g.dxf[x];
-  const double rcm = a.g.rdxc[x], rcp = a.g.rdxc[x + 1], rf = a.g.rdxf[x];
-  const double cm = a.g.c_cm[x], cp = a.g.c_cp[x];
-  const double dy = a.g.dy, rdy = a.g.rdy;
-  int e[6] = {0, 0, 0, 0, 0, 0};
-  if constexpr (FAST) {
-    e[0] = p2_field(rcm);
-    e[1] = p2_field(rcp);
-    e[2] = p2_field(rdy);
-    e[3] = p2_field(rf);
-    e[4] = p2_field(cm);
-    e[5] = p2_field(cp);
-  }
+  TempCol k;
+  k.cm = spacing<RCP, FAST>(a.g.dxc[x], a.g.rdxc[x], a.g.rdxc_l, x);
+  k.cp = spacing<RCP, FAST>(a.g.dxc[x + 1], a.g.rdxc[x + 1], a.g.rdxc_l, x + 1);
+  k.f = spacing<RCP, FAST>(a.g.dxf[x], a.g.rdxf[x], a.g.rdxf_l, x);
+  k.y = spacing_y<RCP, FAST>(a.g.dy, a.g.rdy, a.g.rdyl);
+  k.am = a.g.c_cm[x];
+  k.ap = a.g.c_cp[x];
+  k.e_am = RCP && FAST ? p2_field(k.am) : 0;
+  k.e_ap = RCP && FAST ? p2_field(k.ap) : 0;
+  k.bad = !RCP && FAST && (no_pair(k.cm) | no_pair(k.cp) | no_pair(k.f));
   const bool left = x == 0, right = x == nx - 1;
   double tc = T[(size_t)y0 * nx + x];
   // y-face between rows y0-1 and y0 (periodic halo, src/temperature/boundary_conditions.c:13-14)
-  double gym = dv<RCP>(tc - T[(size_t)wrap_dn(y0, ny) * nx + x], dy, rdy);
+  double gym = over_checked<RCP, FAST>(tc - T[(size_t)wrap_dn(y0, ny) * nx + x], k.y);
   double pym = (0.5 * a.uy[(size_t)y0 * nx + x]) * gym;
   for (int y = y0; y < y1; ++y) {
     const int yp = wrap_up(y, ny);
@@ -186,13 +246,10 @@ __device__ __forceinline__ void temp_column(const TempArgs &a, int x, int y0) {
     const double atr = a.s.has_b ? a.at[r] : 0.0;
     TempRow o;
     if constexpr (FAST) {
-      if (!temp_row<IMPX, IMPY, RCP, true>(a, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, dcm, dcp, df, rcm, rcp, rf,
-                                           cm, cp, e, o))
-        temp_row<IMPX, IMPY, RCP, false>(a, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, dcm, dcp, df, rcm, rcp, rf,
-                                         cm, cp, e, o);
+      if (!temp_row<IMPX, IMPY, RCP, true>(a, k, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, o) || k.bad)
+        temp_row<IMPX, IMPY, RCP, false>(a, k, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, o);
     } else {
-      temp_row<IMPX, IMPY, RCP, false>(a, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, dcm, dcp, df, rcm, rcp, rf, cm,
-                                       cp, e, o);
+      temp_row<IMPX, IMPY, RCP, false>(a, k, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, o);
     }
     a.at[r] = o.A;
     if (IMPX || IMPY) {
@@ -207,10 +264,10 @@ __device__ __forceinline__ void temp_column(const TempArgs &a, int x, int y0) {
 }
 
 template <int IMPX, int IMPY, bool RCP, bool FAST>
-__global__ void __launch_bounds__(128) k_temp(const TempArgs a) {
+__global__ void __launch_bounds__(128) k_temp(const TempArgs a, int rows) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.g.nx) return;
-  temp_column<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * kRows);
+  temp_column<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
 }
 
 // ------------------------------------------------------------------ velocity
@@ -221,13 +278,14 @@ struct VelArgs {
   double *ux_out, *uy_out, *aux, *auy, *qx, *qy;
 };
 
-// metrics of column x: ux at i = x+1 (DXF(i-1), DXF(i), DXC(i)), uy at
-// i = x+1 (DXC(i), DXC(i+1), DXF(i)), with the exponents of the power-of-two
-// factors when they are taken in the integer unit
+// metrics of column x: ux at i = x+1 divides by DXF(i-1), DXF(i), DXC(i), uy
+// by DXC(i), DXC(i+1), DXF(i), both by dy; the advective coefficients with the
+// exponents of those that are powers of two; bad: a spacing without its pair
 struct VelCol {
-  double uf_m, uf_p, uc_c, ruf_m, ruf_p, ruc_c, fm, fp;
-  double vc_m, vc_p, vf_c, rvc_m, rvc_p, rvf_c, cm, cp;
-  int e_ruf_m, e_ruf_p, e_ruc_c, e_fm, e_fp, e_rvc_m, e_rvc_p, e_rvf_c, e_cm, e_cp, e_rdy;
+  Spacing f_m, f, c, c_p, y;  // DXF(i-1), DXF(i), DXC(i), DXC(i+1), dy
+  double fm, fp, cm, cp;
+  int e_fm, e_fp, e_cm, e_cp;
+  bool bad;
 };
 
 // one row: the values carried from the row below, and this row's loads
@@ -249,18 +307,12 @@ template <int IMPX, int IMPY, bool RCP, bool FAST>
 __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const VelIn &in, bool has_ux,
                                         VelOut &o) {
   Mul<FAST> m;
-  const double dy = a.g.dy, rdy = a.g.rdy, nu = a.s.nu;
+  const double nu = a.s.nu;
   // difference / spacing
-  auto D = [&](double v, double d, double rd, int E) {
-    if constexpr (FAST) {
-      return m.by(v, rd, E);
-    } else {
-      return dv<RCP>(v, d, rd);
-    }
-  };
+  auto D = [&](double v, const Spacing &s) { return over<RCP, FAST>(m, v, s); };
   // coefficient * value
   auto C = [&](double c, double v, int E) {
-    if constexpr (FAST) {
+    if constexpr (FAST && RCP) {
       return m.by(v, c, E);
     } else {
       return c * v;
@@ -270,17 +322,17 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
   o.pym_u = in.pym_u;
   // ---- ux(i, j), i = x+1 >= 2
   if (has_ux) {
-    const double gxm = D(in.u0 - in.ul, k.uf_m, k.ruf_m, k.e_ruf_m);
-    const double gxp = D(in.u1 - in.u0, k.uf_p, k.ruf_p, k.e_ruf_p);
-    const double gyp = D(in.u0n - in.u0, dy, rdy, k.e_rdy);
+    const double gxm = D(in.u0 - in.ul, k.f_m);
+    const double gxp = D(in.u1 - in.u0, k.f);
+    const double gyp = D(in.u0n - in.u0, k.y);
     const double vxm = m.half(in.ul) + m.half(in.u0);
     const double vxp = m.half(in.u0) + m.half(in.u1);
     const double adv1 = -(C(k.fm, vxm, k.e_fm) * gxm) - (C(k.fp, vxp, k.e_fp) * gxp);
     const double pyp = m.half(C(k.fm, in.vln, k.e_fm) + C(k.fp, in.v0n, k.e_fp)) * gyp;
     const double adv2 = -in.pym_u - pyp;
-    const double dif1 = D(nu * (gxp - gxm), k.uc_c, k.ruc_c, k.e_ruc_c);
-    const double dif2 = D(nu * (gyp - in.gym_u), dy, rdy, k.e_rdy);
-    const double pre = -D(in.pc - in.pl, k.uc_c, k.ruc_c, k.e_ruc_c);
+    const double dif1 = D(nu * (gxp - gxm), k.c);
+    const double dif2 = D(nu * (gyp - in.gym_u), k.y);
+    const double pre = -D(in.pc - in.pl, k.c);
     double A = adv1 + adv2;
     if (!IMPX) A = A + dif1;
     if (!IMPY) A = A + dif2;
@@ -306,17 +358,17 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
   }
   // ---- uy(i, j), i = x+1 >= 1
   {
-    const double gxm = D(in.v0 - in.vl, k.vc_m, k.rvc_m, k.e_rvc_m);
-    const double gxp = D(in.vr - in.v0, k.vc_p, k.rvc_p, k.e_rvc_p);
-    const double gyp = D(in.v0n - in.v0, dy, rdy, k.e_rdy);
+    const double gxm = D(in.v0 - in.vl, k.c);
+    const double gxp = D(in.vr - in.v0, k.c_p);
+    const double gyp = D(in.v0n - in.v0, k.y);
     const double wxm = m.half(in.um0) + m.half(in.u0);
     const double wxp = m.half(in.um1) + m.half(in.u1);
     const double adv1 = -(C(k.cm, wxm, k.e_cm) * gxm) - (C(k.cp, wxp, k.e_cp) * gxp);
     const double pyp = m.half(m.half(in.v0) + m.half(in.v0n)) * gyp;
     const double adv2 = -in.pym_v - pyp;
-    const double dif1 = D(nu * (gxp - gxm), k.vf_c, k.rvf_c, k.e_rvf_c);
-    const double dif2 = D(nu * (gyp - in.gym_v), dy, rdy, k.e_rdy);
-    const double pre = -D(in.pc - in.pm, dy, rdy, k.e_rdy);
+    const double dif1 = D(nu * (gxp - gxm), k.f);
+    const double dif2 = D(nu * (gyp - in.gym_v), k.y);
+    const double pre = -D(in.pc - in.pm, k.y);
     double A = adv1 + adv2;
     if (!IMPX) A = A + dif1;
     if (!IMPY) A = A + dif2;
@@ -343,48 +395,33 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
 }
 
 template <int IMPX, int IMPY, bool RCP, bool FAST>
-__global__ void __launch_bounds__(128) k_vel(const VelArgs a) {
+__global__ void __launch_bounds__(128) k_vel(const VelArgs a, int rows) {
   const int nx = a.g.nx, ny = a.g.ny;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= nx) return;
-  const int y0 = blockIdx.y * kRows;
-  const int y1 = min(y0 + kRows, ny);
+  const int y0 = blockIdx.y * rows;
+  const int y1 = min(y0 + rows, ny);
   const bool left = x == 0, right = x == nx - 1;
   const bool has_ux = x >= 1;  // ux is updated for i = 2..itot
-  const double dy = a.g.dy, rdy = a.g.rdy;
   VelCol k;
-  k.uf_m = has_ux ? a.g.dxf[x - 1] : 1.0;
-  k.uf_p = a.g.dxf[x];
-  k.uc_c = a.g.dxc[x];
-  k.ruf_m = has_ux ? a.g.rdxf[x - 1] : 1.0;
-  k.ruf_p = a.g.rdxf[x];
-  k.ruc_c = a.g.rdxc[x];
+  const int xm = has_ux ? x - 1 : x;
+  k.f_m = spacing<RCP, FAST>(a.g.dxf[xm], a.g.rdxf[xm], a.g.rdxf_l, xm);
+  k.f = spacing<RCP, FAST>(a.g.dxf[x], a.g.rdxf[x], a.g.rdxf_l, x);
+  k.c = spacing<RCP, FAST>(a.g.dxc[x], a.g.rdxc[x], a.g.rdxc_l, x);
+  k.c_p = spacing<RCP, FAST>(a.g.dxc[x + 1], a.g.rdxc[x + 1], a.g.rdxc_l, x + 1);
+  k.y = spacing_y<RCP, FAST>(a.g.dy, a.g.rdy, a.g.rdyl);
   k.fm = a.g.c_fm[x];
   k.fp = a.g.c_fp[x];
-  k.vc_m = a.g.dxc[x];
-  k.vc_p = a.g.dxc[x + 1];
-  k.vf_c = a.g.dxf[x];
-  k.rvc_m = a.g.rdxc[x];
-  k.rvc_p = a.g.rdxc[x + 1];
-  k.rvf_c = a.g.rdxf[x];
   k.cm = a.g.c_cm[x];
   k.cp = a.g.c_cp[x];
-  if constexpr (FAST) {
-    k.e_ruf_m = p2_field(k.ruf_m);
-    k.e_ruf_p = p2_field(k.ruf_p);
-    k.e_ruc_c = p2_field(k.ruc_c);
+  k.e_fm = k.e_fp = k.e_cm = k.e_cp = 0;
+  if constexpr (RCP && FAST) {
     k.e_fm = p2_field(k.fm);
     k.e_fp = p2_field(k.fp);
-    k.e_rvc_m = p2_field(k.rvc_m);
-    k.e_rvc_p = p2_field(k.rvc_p);
-    k.e_rvf_c = p2_field(k.rvf_c);
     k.e_cm = p2_field(k.cm);
     k.e_cp = p2_field(k.cp);
-    k.e_rdy = p2_field(rdy);
-  } else {
-    k.e_ruf_m = k.e_ruf_p = k.e_ruc_c = k.e_fm = k.e_fp = k.e_rvc_m = k.e_rvc_p = k.e_rvf_c = k.e_cm = k.e_cp =
-        k.e_rdy = 0;
   }
+  k.bad = !RCP && FAST && (no_pair(k.f_m) | no_pair(k.f) | no_pair(k.c) | no_pair(k.c_p));
   const double *ux = a.ux, *uy = a.uy, *p = a.p;
 
   VelIn in;
@@ -398,11 +435,11 @@ __global__ void __launch_bounds__(128) k_vel(const VelArgs a) {
   in.vl = left ? 0.0 : uy[r0 - 1];
   in.pm = p[rm];
   // y-faces between rows y0-1 and y0
-  in.gym_u = dv<RCP>(in.u0 - in.um0, dy, rdy);
+  in.gym_u = over_checked<RCP, FAST>(in.u0 - in.um0, k.y);
   in.pym_u = 0.0;
   if (has_ux) in.pym_u = (0.5 * (k.fm * in.vl + k.fp * in.v0)) * in.gym_u;
   const double vm = uy[rm];
-  in.gym_v = dv<RCP>(in.v0 - vm, dy, rdy);
+  in.gym_v = over_checked<RCP, FAST>(in.v0 - vm, k.y);
   in.pym_v = (0.5 * (0.5 * vm + 0.5 * in.v0)) * in.gym_v;
   in.ul = in.pl = in.tfl = in.tfr = in.aux = in.auy = 0.0;
 
@@ -427,7 +464,8 @@ __global__ void __launch_bounds__(128) k_vel(const VelArgs a) {
     if (a.s.has_b) in.auy = a.auy[r];
     VelOut o;
     if constexpr (FAST) {
-      if (!vel_row<IMPX, IMPY, RCP, true>(a, k, in, has_ux, o)) vel_row<IMPX, IMPY, RCP, false>(a, k, in, has_ux, o);
+      if (!vel_row<IMPX, IMPY, RCP, true>(a, k, in, has_ux, o) || k.bad)
+        vel_row<IMPX, IMPY, RCP, false>(a, k, in, has_ux, o);
     } else {
       vel_row<IMPX, IMPY, RCP, false>(a, k, in, has_ux, o);
     }
@@ -653,6 +691,7 @@ __device__ __forceinline__ void poisson_fwd_cols(const PoissonArgs &a, int x0, d
   const int nx = a.g.nx, ny = a.g.ny, M = ny / 2, C = a.cols;
   double *zd = reinterpret_cast<double *>(z);
   const double dy = a.g.dy, rdy = a.g.rdy;
+  const Spacing sy = spacing_y<RCP, true>(dy, rdy, a.g.rdyl);
   for (int e = threadIdx.x; e < C * ny; e += blockDim.x) {
     const int c = e % C, y = e / C, x = x0 + c;
     double d = 0.0;
@@ -662,7 +701,15 @@ __device__ __forceinline__ void poisson_fwd_cols(const PoissonArgs &a, int x0, d
       const double uxp = x == nx - 1 ? 0.0 : a.ux[r + 1];
       const double uym = a.uy[r];
       const double uyp = a.uy[(size_t)wrap_up(y, ny) * nx + x];
-      d = a.s.rgdt * (dv<RCP>(uxp - uxm, a.g.dxf[x], a.g.rdxf[x]) + dv<RCP>(uyp - uym, dy, rdy));
+      Mul<true> m;
+      bool fast = RCP ? a.g.p2 : a.g.dv2;
+      if (fast) {
+        const Spacing sx = spacing<RCP, true>(a.g.dxf[x], a.g.rdxf[x], a.g.rdxf_l, x);
+        d = over<RCP, true>(m, uxp - uxm, sx) + over<RCP, true>(m, uyp - uym, sy);
+        fast = m.ok && (RCP || !no_pair(sx));
+      }
+      if (!fast) d = dv<RCP>(uxp - uxm, a.g.dxf[x], a.g.rdxf[x]) + dv<RCP>(uyp - uym, dy, rdy);
+      d = a.s.rgdt * d;
     }
     zd[2 * (c * M + fft_slot(y >> 1, M, a.g.fft_nst, a.g.fft_first2)) + (y & 1)] = d;
   }
@@ -1106,10 +1153,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_poisson_fused(const FusedA
     for (int u = wk; u < xb * yb; u += W) {
       const int x = (u % xb) * kFusedThreads + threadIdx.x;
       if (x < nx) {
-        if (RCP && g.p2) {
-          temp_column<0, 0, RCP, RCP>(a.t, x, (u / xb) * kRows);
+        if (RCP ? g.p2 : g.dv2) {
+          temp_column<0, 0, RCP, true>(a.t, x, (u / xb) * kRows, kRows);
         } else {
-          temp_column<0, 0, RCP, false>(a.t, x, (u / xb) * kRows);
+          temp_column<0, 0, RCP, false>(a.t, x, (u / xb) * kRows, kRows);
         }
       }
     }
@@ -1157,7 +1204,7 @@ __device__ __forceinline__ bool nonfinite(double v) {
   return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
 }
 
-constexpr int kCorrRows = 4;  // rows per thread in the (memory-latency bound) correction kernels
+constexpr int kCorrRows = 4;  // rows per thread in the (memory-latency bound) correction kernels on large grids
 
 __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
 #pragma unroll
@@ -1165,12 +1212,56 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
   return v;
 }
 
+// one cell of the correction and the pressure: psi here (sc), west, east,
+// south and north of it, the cell's old values; gm_y: the psi gradient
+// between rows y-1 and y (implicit y), replaced by that between y and y+1
+struct CorrCell {
+  double u, v, p;
+};
+struct CorrCol {
+  Spacing cm, cp, f, y;  // DXC(i), DXC(i+1), DXF(i), dy
+  double dxi;            // 1./DXC(i)
+  bool bad;
+};
+template <int IMPX, int IMPY, bool RCP, bool FAST, bool CORR, bool PRES>
+__device__ __forceinline__ bool corr_cell(const StageScalars &t, const CorrCol &k, double sc, double sw, double se,
+                                          double ss, double sn, double &gm_y, CorrCell &o) {
+  Mul<FAST> m;
+  auto D = [&](double v, const Spacing &s) { return over<RCP, FAST>(m, v, s); };
+  if (CORR) {
+    const double dx = t.gdt * (sc - sw);
+    if constexpr (RCP && FAST) {
+      o.u = o.u - m.by(dx, k.dxi, k.cm.e);
+    } else {
+      o.u = o.u - (dx * k.dxi);
+    }
+    o.v = o.v - D(t.gdt * (sc - ss), k.y);
+  }
+  if (PRES) {
+    double pv = o.p + sc;
+    if (IMPX) {
+      const double gm = D(sc - sw, k.cm), gp = D(se - sc, k.cp);
+      pv = pv + t.pcorr * D(gp - gm, k.f);
+    }
+    if (IMPY) {
+      const double gp = D(sn - sc, k.y);
+      pv = pv + t.pcorr * D(gp - gm_y, k.y);
+      gm_y = gp;
+    }
+    o.p = pv;
+  }
+  return m.ok;
+}
+
 // src/fluid/correct_velocity.c:6-42 and src/fluid/update_pressure.c:7-60, per
 // cell in the reference's order; with colmax set, also max |ux| per column and
 // max |uy| for the next src/param/decide_dt.c (exact: division is monotonic).
 // Every lane of a block stays alive to the warp reduction (blockDim is a
-// multiple of 32); lanes past the last column only contribute zero.
-template <int IMPX, int IMPY, bool RCP, bool CORR, bool PRES>
+// multiple of 32); lanes past the last column only contribute zero. A thread
+// takes CR rows and loads every operand of theirs before its first store (the
+// stores could alias later loads for the compiler): one memory round trip per
+// thread instead of CR.
+template <int IMPX, int IMPY, bool RCP, bool CORR, bool PRES, int CR>
 __global__ void __launch_bounds__(128) k_corr(const CorrArgs a) {
   const int nx = a.g.nx, ny = a.g.ny;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1178,103 +1269,84 @@ __global__ void __launch_bounds__(128) k_corr(const CorrArgs a) {
   unsigned long long mx = 0ull, my = 0ull;
   bool nf = false;  // a NaN or infinity among the values written
   if (live) {
-    const int y0 = blockIdx.y * kCorrRows;
-    int y1 = min(y0 + kCorrRows, ny);
-    const double gdt = a.s.gdt, dy = a.g.dy, rdy = a.g.rdy;
-    const double dxi = a.g.dxi[x];
-    const double dcm = a.g.dxc[x], dcp = a.g.dxc[x + 1], df = a.g.dxf[x];
-    const double rcm = a.g.rdxc[x], rcp = a.g.rdxc[x + 1], rf = a.g.rdxf[x];
+    const int y0 = blockIdx.y * CR, n = min(CR, ny - y0);
     const bool left = x == 0, right = x == nx - 1;
-    const double *psi = a.psi;
-    double sm = psi[(size_t)wrap_dn(y0, ny) * nx + x];
-    if constexpr (!IMPX && !IMPY && CORR && PRES) {
-      if (y1 - y0 == kCorrRows) {
-        // every operand of the rows loaded before the first store (the
-        // stores could alias later loads for the compiler): one memory round
-        // trip per thread instead of kCorrRows
-        double ps[kCorrRows], pw[kCorrRows], u[kCorrRows], v[kCorrRows], pp[kCorrRows];
-#pragma unroll
-        for (int k = 0; k < kCorrRows; ++k) {
-          const size_t r = (size_t)(y0 + k) * nx + x;
-          ps[k] = psi[r];
-          pw[k] = left ? 0.0 : psi[r - 1];
-          u[k] = left ? 0.0 : a.ux[r];
-          v[k] = a.uy[r];
-          pp[k] = a.p[r];
-        }
-        // the rows' new values; FAST: the products by 1/dx and 1/dy (powers of
-        // two on such grids) in the integer unit, false when out of range
-        auto rows = [&](auto fast, double *un, double *vn) -> bool {
-          Mul<decltype(fast)::value> m;
-          double s0 = sm;
-#pragma unroll
-          for (int k = 0; k < kCorrRows; ++k) {
-            const double sc = ps[k];
-            const double sl = left ? sc : pw[k];  // Neumann psi(0) = psi(1)
-            if constexpr (decltype(fast)::value) {
-              un[k] = u[k] - m.by(gdt * (sc - sl), dxi, p2_field(dxi));
-              vn[k] = v[k] - m.by(gdt * (sc - s0), rdy, p2_field(rdy));
-            } else {
-              un[k] = u[k] - ((gdt * (sc - sl)) * dxi);
-              vn[k] = v[k] - dv<RCP>(gdt * (sc - s0), dy, rdy);
-            }
-            s0 = sc;
-          }
-          return m.ok;
-        };
-        double un[kCorrRows], vn[kCorrRows];
-        if (!(RCP && a.g.p2 && rows(std::true_type{}, un, vn))) rows(std::false_type{}, un, vn);
-#pragma unroll
-        for (int k = 0; k < kCorrRows; ++k) {
-          const size_t r = (size_t)(y0 + k) * nx + x;
-          if (!left) {
-            a.ux[r] = un[k];
-            mx = max(mx, abs_bits(un[k]));
-            nf |= nonfinite(un[k]);
-          }
-          a.uy[r] = vn[k];
-          my = max(my, abs_bits(vn[k]));
-          const double pv = pp[k] + ps[k];
-          a.p[r] = pv;
-          nf |= nonfinite(vn[k]) | nonfinite(pv);
-        }
-        y1 = y0;  // done: skip the row loop below
-      }
+    const bool fast = RCP ? a.g.p2 : a.g.dv2;
+    CorrCol k;
+    k.dxi = a.g.dxi[x];
+    k.cm = spacing<RCP, false>(a.g.dxc[x], a.g.rdxc[x], nullptr, 0);
+    k.cp = spacing<RCP, false>(a.g.dxc[x + 1], a.g.rdxc[x + 1], nullptr, 0);
+    k.f = spacing<RCP, false>(a.g.dxf[x], a.g.rdxf[x], nullptr, 0);
+    k.y = spacing_y<RCP, false>(a.g.dy, a.g.rdy, 0.0);
+    k.bad = false;
+    if (fast) {
+      k.cm = spacing<RCP, true>(k.cm.d, k.cm.r, a.g.rdxc_l, x);
+      k.cp = spacing<RCP, true>(k.cp.d, k.cp.r, a.g.rdxc_l, x + 1);
+      k.f = spacing<RCP, true>(k.f.d, k.f.r, a.g.rdxf_l, x);
+      k.y = spacing_y<RCP, true>(k.y.d, k.y.r, a.g.rdyl);
+      k.bad = !RCP && IMPX && (no_pair(k.cm) | no_pair(k.cp) | no_pair(k.f));
     }
-    for (int y = y0; y < y1; ++y) {
-      const size_t r = (size_t)y * nx + x;
-      const double sc = psi[r];
-      const double sl = left ? sc : psi[r - 1];  // Neumann psi(0) = psi(1)
+    const double *psi = a.psi;
+    const double s0 = psi[(size_t)wrap_dn(y0, ny) * nx + x];
+    double ps[CR + 1], pw[CR], pe[CR];
+    CorrCell old[CR];
+#pragma unroll
+    for (int i = 0; i <= CR; ++i) {
+      if (i < n || (IMPY && i == n)) ps[i] = psi[(size_t)(y0 + i == ny ? 0 : y0 + i) * nx + x];
+      if (i == CR || i >= n) continue;
+      const size_t r = (size_t)(y0 + i) * nx + x;
+      pw[i] = left ? 0.0 : psi[r - 1];
+      if (IMPX) pe[i] = right ? 0.0 : psi[r + 1];
+      if (CORR) {
+        old[i].u = left ? 0.0 : a.ux[r];
+        old[i].v = a.uy[r];
+      }
+      if (PRES) old[i].p = a.p[r];
+    }
+    // the rows' new values; FAST: the products by 1/dx and 1/dy (powers of two
+    // on such grids) in the integer unit and the divisions by their pairs,
+    // false when an operand is out of range
+    auto rows = [&](auto ff, CorrCell *o) -> bool {
+      constexpr bool F = decltype(ff)::value;
+      bool ok = true;
+      double sm = s0, gm = 0.0;
+      if (IMPY) {
+        Mul<F> m;
+        gm = over<RCP, F>(m, ps[0] - sm, k.y);
+        ok &= m.ok;
+      }
+#pragma unroll
+      for (int i = 0; i < CR; ++i) {
+        if (i >= n) break;
+        o[i] = old[i];
+        const double sc = ps[i];
+        // Neumann psi(0) = psi(1), psi(nx+1) = psi(nx)
+        ok &= corr_cell<IMPX, IMPY, RCP, F, CORR, PRES>(a.s, k, sc, left ? sc : pw[i], IMPX && !right ? pe[i] : sc, sm,
+                                                        IMPY ? ps[i + 1] : 0.0, gm, o[i]);
+        sm = sc;
+      }
+      return ok;
+    };
+    CorrCell now[CR];
+    if (!(fast && !k.bad && rows(std::true_type{}, now))) rows(std::false_type{}, now);
+#pragma unroll
+    for (int i = 0; i < CR; ++i) {
+      if (i >= n) break;
+      const size_t r = (size_t)(y0 + i) * nx + x;
       if (CORR) {
         if (!left) {
-          const double u = a.ux[r] - ((gdt * (sc - sl)) * dxi);
-          a.ux[r] = u;
-          mx = max(mx, abs_bits(u));
-          nf |= nonfinite(u);
+          a.ux[r] = now[i].u;
+          mx = max(mx, abs_bits(now[i].u));
+          nf |= nonfinite(now[i].u);
         }
-        const double v = a.uy[r] - dv<RCP>(gdt * (sc - sm), dy, rdy);
-        a.uy[r] = v;
-        my = max(my, abs_bits(v));
-        nf |= nonfinite(v);
+        a.uy[r] = now[i].v;
+        my = max(my, abs_bits(now[i].v));
+        nf |= nonfinite(now[i].v);
       }
       if (PRES) {
-        double pv = a.p[r] + sc;
-        if (IMPX) {
-          const double sr = right ? sc : psi[r + 1];  // Neumann psi(nx+1) = psi(nx)
-          const double gm = dv<RCP>(sc - sl, dcm, rcm);
-          const double gp = dv<RCP>(sr - sc, dcp, rcp);
-          pv = pv + a.s.pcorr * dv<RCP>(gp - gm, df, rf);
-        }
-        if (IMPY) {
-          const double sn = psi[(size_t)wrap_up(y, ny) * nx + x];
-          const double gm = dv<RCP>(sc - sm, dy, rdy);
-          const double gp = dv<RCP>(sn - sc, dy, rdy);
-          pv = pv + a.s.pcorr * dv<RCP>(gp - gm, dy, rdy);
-        }
-        a.p[r] = pv;
-        nf |= nonfinite(pv);
+        a.p[r] = now[i].p;
+        nf |= nonfinite(now[i].p);
       }
-      sm = sc;
     }
   }
   if (CORR && a.colmax) {
@@ -1311,8 +1383,26 @@ __global__ void __launch_bounds__(128) k_umax(int nx, int ny, const double *ux, 
   if (__any_sync(0xffffffffu, nf) && (threadIdx.x & 31) == 0) atomicOr(colmax, 1ull);
 }
 
-dim3 march_grid(const DevGrid &g, int rows = kRows) {
+dim3 march_grid(const DevGrid &g, int rows) {
   return dim3((g.nx + kBlockX - 1) / kBlockX, (g.ny + rows - 1) / rows);
+}
+
+// Rows marched by a thread of the velocity and temperature updates. Fewer
+// rows form more y-faces twice (2 to 9 FP64 instructions a thread) but give
+// more warps; a sub-partition issues an FP64 instruction every ~70 cycles from
+// one warp and hardly more from several, so a small grid needs its
+// sub-partitions filled before it needs long marches. Velocity update, us per
+// launch (events; 1, 2, 4, 8 rows; the rule's choice in brackets):
+//   64 x 128:  [8.5] 10.9 16.5 26.6     128 x 256: [10.6] 12.4 16.9 26.9
+//   256 x 512: 25.2 [20.9] 22.9 27.4    512 x 512: 40.7 35.2 [34.5] 38.1
+//   512 x 1024: 69.8 65.4 61.6 [61.1]
+// (two warps per sub-partition against one: 256 x 512 20.8 / 22.9, 512 x 512
+// 34.6 / 37.8, 300 x 256 stretched 24.7 / 26.6 us)
+int march_rows(const DevGrid &g) {
+  const long warps1 = (long)((g.nx + 31) / 32) * g.ny;  // warps with one row each
+  int rows = 1;
+  while (rows < kRows && warps1 / (2 * rows) >= kMarchWarps) rows *= 2;
+  return rows;
 }
 
 // one thread per radix-4 butterfly of a stage, 64..256 per block
@@ -1335,8 +1425,9 @@ cudaError_t launch_temp_update(const DevGrid &g, const StageScalars &s, int impx
                                const double *t_in, double *t_out, double *at, double *qt,
                                const double *ux, const double *uy, cudaStream_t st) {
   const TempArgs a{g, s, t_in, t_out, at, qt, ux, uy};
-  const dim3 grid = march_grid(g), block(kBlockX);
-#define SNS_T(X, Y, R, F) k_temp<X, Y, R, F><<<grid, block, 0, st>>>(a)
+  const int rows = march_rows(g);
+  const dim3 grid = march_grid(g, rows), block(kBlockX);
+#define SNS_T(X, Y, R, F) k_temp<X, Y, R, F><<<grid, block, 0, st>>>(a, rows)
   if (g.p2) {
     if (impx && impy) SNS_T(1, 1, true, true);
     else if (impx) SNS_T(1, 0, true, true);
@@ -1347,6 +1438,11 @@ cudaError_t launch_temp_update(const DevGrid &g, const StageScalars &s, int impx
     else if (impx) SNS_T(1, 0, true, false);
     else if (impy) SNS_T(0, 1, true, false);
     else SNS_T(0, 0, true, false);
+  } else if (g.dv2) {
+    if (impx && impy) SNS_T(1, 1, false, true);
+    else if (impx) SNS_T(1, 0, false, true);
+    else if (impy) SNS_T(0, 1, false, true);
+    else SNS_T(0, 0, false, true);
   } else {
     if (impx && impy) SNS_T(1, 1, false, false);
     else if (impx) SNS_T(1, 0, false, false);
@@ -1363,8 +1459,9 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
                                    double *ux_out, double *uy_out, double *aux, double *auy,
                                    double *qx, double *qy, cudaStream_t st) {
   const VelArgs a{g, s, ux, uy, p, tforce, ux_out, uy_out, aux, auy, qx, qy};
-  const dim3 grid = march_grid(g), block(kBlockX);
-#define SNS_V(X, Y, R, F) k_vel<X, Y, R, F><<<grid, block, 0, st>>>(a)
+  const int rows = march_rows(g);
+  const dim3 grid = march_grid(g, rows), block(kBlockX);
+#define SNS_V(X, Y, R, F) k_vel<X, Y, R, F><<<grid, block, 0, st>>>(a, rows)
   if (g.p2) {
     if (impx && impy) SNS_V(1, 1, true, true);
     else if (impx) SNS_V(1, 0, true, true);
@@ -1375,6 +1472,11 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
     else if (impx) SNS_V(1, 0, true, false);
     else if (impy) SNS_V(0, 1, true, false);
     else SNS_V(0, 0, true, false);
+  } else if (g.dv2) {
+    if (impx && impy) SNS_V(1, 1, false, true);
+    else if (impx) SNS_V(1, 0, false, true);
+    else if (impy) SNS_V(0, 1, false, true);
+    else SNS_V(0, 0, false, true);
   } else {
     if (impx && impy) SNS_V(1, 1, false, false);
     else if (impx) SNS_V(1, 0, false, false);
@@ -1739,8 +1841,15 @@ static cudaError_t launch_corr_t(const DevGrid &g, const StageScalars &s, int im
                                  double *ux, double *uy, double *p, unsigned long long *colmax,
                                  unsigned long long *uymax, cudaStream_t st) {
   const CorrArgs a{g, s, psi, ux, uy, p, colmax, uymax};
-  const dim3 grid = march_grid(g, kCorrRows), block(kBlockX);
-#define SNS_C(X, Y, R) k_corr<X, Y, R, CORR, PRES><<<grid, block, 0, st>>>(a)
+  // one row per thread on grids that march fewer than kCorrRows rows (128 x 256:
+  // 6.7 us per launch against 8.0 with four; 512 x 1024: four, 16.4 us)
+  const bool small = march_rows(g) < kCorrRows;
+  const dim3 grid = march_grid(g, small ? 1 : kCorrRows), block(kBlockX);
+#define SNS_C(X, Y, R)                                                \
+  do {                                                                \
+    if (small) k_corr<X, Y, R, CORR, PRES, 1><<<grid, block, 0, st>>>(a); \
+    else k_corr<X, Y, R, CORR, PRES, kCorrRows><<<grid, block, 0, st>>>(a); \
+  } while (0)
   if (g.rcp) {
     if (impx && impy) SNS_C(1, 1, true);
     else if (impx) SNS_C(1, 0, true);
@@ -1775,7 +1884,7 @@ cudaError_t launch_correct_pressure(const DevGrid &g, const StageScalars &s, int
 
 cudaError_t launch_umax(const DevGrid &g, const double *ux, const double *uy, unsigned long long *colmax,
                         unsigned long long *uymax, cudaStream_t st) {
-  k_umax<<<march_grid(g), kBlockX, 0, st>>>(g.nx, g.ny, ux, uy, colmax, uymax);
+  k_umax<<<march_grid(g, kRows), kBlockX, 0, st>>>(g.nx, g.ny, ux, uy, colmax, uymax);
   count_launches(1);
   return cudaGetLastError();
 }

@@ -329,6 +329,27 @@ static int build_context(Context *c, const param_t *param) {
     g.p2 = ok;
   }
   int rc = SNS_OK;
+  g.dv2 = false;
+  g.rdyl = 0.0;
+  if (!rcp) {
+    // divisions by the spacings in two instructions (plain_fp64.cu, Mul::div);
+    // a spacing without such a pair (one in some thousands) keeps its division
+    const double nan = std::nan("");
+    double zh;
+    auto pair = [&](double v, double *zl) {
+      int e;
+      return std::isnormal(v) && (std::frexp(v, &e), std::abs(e - 1) <= 64) && invariant_divisor(v, &zh, zl);
+    };
+    g.dv2 = pair(g.dy, &g.rdyl);
+    std::vector<double> lf(nx), lc(nx + 1);
+    for (int i = 0; i < nx; i++)
+      if (i > 0 && c->dxf[i] == c->dxf[i - 1]) lf[i] = lf[i - 1];
+      else if (!pair(c->dxf[i], &lf[i])) lf[i] = nan;
+    for (int i = 0; i <= nx; i++)
+      if (i > 0 && c->dxc[i] == c->dxc[i - 1]) lc[i] = lc[i - 1];
+      else if (!pair(c->dxc[i], &lc[i])) lc[i] = nan;
+    if ((rc = upload(c, &g.rdxf_l, lf)) || (rc = upload(c, &g.rdxc_l, lc))) return rc;
+  }
   if ((rc = upload(c, &g.dxf, c->dxf)) || (rc = upload(c, &g.dxc, c->dxc)) || (rc = upload(c, &g.rdxf, rdxf)) ||
       (rc = upload(c, &g.rdxc, rdxc)) || (rc = upload(c, &g.dxi, dxi)) || (rc = upload(c, &g.c_cm, ccm)) ||
       (rc = upload(c, &g.c_cp, ccp)) || (rc = upload(c, &g.c_fm, cfm)) || (rc = upload(c, &g.c_fp, cfp)) ||

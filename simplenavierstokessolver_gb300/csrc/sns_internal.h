@@ -28,11 +28,13 @@ struct DevGrid {
   int nx, ny, nh, jpitch;  // nh = ny/2 + 1 Fourier modes; jpitch >= nh
   bool rcp;                // every metric divisor is a power of two
   bool p2;                 // rcp, and every reciprocal spacing, advective and Poisson coefficient is 2^e, |e| <= 64
-  double dy, rdy;
+  bool dv2;                // not rcp, and division by dy takes two instructions (invariant_divisor in host_common.h)
+  double dy, rdy, rdyl;    // rdyl, rdxf_l, rdxc_l: with the reciprocal the pair that divides (NaN where none does)
   const double *dxf;    // [nx]    DXF(i)
   const double *dxc;    // [nx+1]  DXC(i), i = 1..nx+1
   const double *rdxf;   // [nx]    1/DXF(i) (exact when rcp)
   const double *rdxc;   // [nx+1]  1/DXC(i) (exact when rcp)
+  const double *rdxf_l, *rdxc_l;  // [nx], [nx+1] (null when rcp)
   const double *dxi;    // [nx+1]  1./DXC(i) as src/fluid/correct_velocity.c:13
   const double *c_cm;   // [nx]    DXC(i)/(2.*DXF(i))     (T and uy advection)
   const double *c_cp;   // [nx]    DXC(i+1)/(2.*DXF(i))
