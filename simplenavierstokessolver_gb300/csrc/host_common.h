@@ -100,12 +100,14 @@ inline std::vector<double> twiddle_table(int n) {
 // and zl close to 1/y - zh, RN(x zh + RN(x zl)), a product and a fused
 // multiply-add, is RN(x/y) for every x (no over- or underflow) unless x/y lies
 // very close to the midpoint of two neighbouring doubles. Before its last
-// rounding that sum is off by at most 8 2^-54 ulp of the quotient (RN(x zl):
-// 2^-54, as |x zl| < 1 ulp; zl, within 3.5 ulp of 1/y - zh: 7 2^-54). With
-// 53-bit integer significands X and Y a midpoint M (odd, 54 bits) is
-// |X 2^53 - M Y| / 2Y ulp away if X >= Y, |X 2^54 - M Y| / 2Y if X < Y, so only
-// numerators X for which that integer is at most 8 can fail. They solve
-// M Y = -D (mod 2^53 or 2^54), a few X per D: all are formed here and tried.
+// rounding that sum is off by at most 2 2^-54 ulp of the quotient with
+// zl = RN(1/y - zh) (RN(x zl): 2^-54, as |x zl| < 1 ulp; zl: 2^-54) and by
+// (2 + 2 k) 2^-54 ulp with a zl k ulps further. With 53-bit integer
+// significands X and Y a midpoint M (odd, 54 bits) is |X 2^53 - M Y| / 2Y ulp
+// away if X >= Y, |X 2^54 - M Y| / 2Y if X < Y, so only numerators X for which
+// that integer is at most 2 + 2 k can fail. They solve M Y = -D (mod 2^53 or
+// 2^54), a few X per D: all are formed here and tried, for zl and, where it
+// fails (one divisor in 200), its neighbours up to k = 3.
 // Returns false when no zl passes (or y is not normal and positive).
 inline bool invariant_divisor(double y, double *zh_out, double *zl_out) {
   int ey;
@@ -116,30 +118,32 @@ inline bool invariant_divisor(double y, double *zh_out, double *zl_out) {
   const uint64_t Yo = Y >> t;
   uint64_t yinv = Yo;  // inverse of Yo modulo 2^64 by Newton's iteration
   for (int k = 0; k < 5; k++) yinv *= 2 - Yo * yinv;
-  std::vector<double> hard;
-  for (int w = 53; w <= 54; w++)  // X >= Y, X < Y
-    for (int D = -8; D <= 8; D++) {
-      // M Y = -D (mod 2^w) needs 2^t | D
-      if (D == 0 || t > 3 || D % (1 << t)) continue;
-      // M = -(D / 2^t) / Yo modulo 2^(w - t), odd, in [2^53, 2^54)
-      const uint64_t mod = 1ull << (w - t);
-      const uint64_t m0 = ((uint64_t)(-(int64_t)(D / (1 << t))) * yinv) & (mod - 1);
-      for (uint64_t M = m0 + ((1ull << 53) - m0 + mod - 1) / mod * mod * (m0 < (1ull << 53)); M < (1ull << 54); M += mod) {
-        if (!(M & 1)) continue;
-        const __int128 n = (__int128)M * Y + D;
-        if (n <= 0 || (n & (((__int128)1 << w) - 1)) != 0) continue;
-        const uint64_t X = (uint64_t)(n >> w);
-        if (X >> 52 != 1 || (w == 53) != (X >= Y)) continue;
-        hard.push_back((double)X);
-      }
-    }
   const double zl0 = std::fma(-zh, ys, 1.0) / ys;  // the residual is exact
+  // whether the pair (zh, zl) divides every X with a midpoint at most Dmax away
+  auto divides = [&](double zl, int Dmax) {
+    for (int w = 53; w <= 54; w++)  // X >= Y, X < Y
+      for (int D = -Dmax; D <= Dmax; D++) {
+        // M Y = -D (mod 2^w) needs 2^t | D
+        if (D == 0 || t > 3 || D % (1 << t)) continue;
+        // M = -(D / 2^t) / Yo modulo 2^(w - t), odd, in [2^53, 2^54)
+        const uint64_t mod = 1ull << (w - t), lo = 1ull << 53;
+        const uint64_t m0 = ((uint64_t)(-(int64_t)(D / (1 << t))) * yinv) & (mod - 1);
+        for (uint64_t M = m0 >= lo ? m0 : m0 + (lo - m0 + mod - 1) / mod * mod; M < 2 * lo; M += mod) {
+          if (!(M & 1)) continue;
+          const __int128 n = (__int128)M * Y + D;
+          if (n <= 0 || (n & (((__int128)1 << w) - 1)) != 0) continue;
+          const uint64_t X = (uint64_t)(n >> w);
+          if (X >> 52 != 1 || (w == 53) != (X >= Y)) continue;
+          const double x = (double)X;
+          if (std::fma(x, zh, x * zl) != x / ys) return false;
+        }
+      }
+    return true;
+  };
   for (int k = 0; k < 7; k++) {  // zl0, then one, two, three ulps up and down
     double zl = zl0;
     for (int i = 0; i < (k + 1) / 2; i++) zl = std::nextafter(zl, k % 2 ? 1.0 : -1.0);
-    bool ok = true;
-    for (double x : hard) ok = ok && std::fma(x, zh, x * zl) == x / ys;
-    if (ok) {
+    if (divides(zl, 2 + 2 * ((k + 1) / 2))) {
       *zh_out = std::ldexp(zh, 53 - ey);
       *zl_out = std::ldexp(zl, 53 - ey);
       return true;
