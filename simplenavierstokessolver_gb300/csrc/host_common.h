@@ -152,6 +152,67 @@ inline bool invariant_divisor(double y, double *zh_out, double *zl_out) {
   return false;
 }
 
+// exp(-2 pi i t / n), t < n (a power of two), scaled by 2^62 and split for the
+// fixed-point DFT (fft_fixed.cuh, Tw): four words per t, real high and low,
+// imaginary high and low, the low ones in (-2^31, 2^31). Sine and cosine of an
+// angle in [0, pi/4] by their Taylor series in 112-bit fixed point, so the
+// words are the same on every host.
+inline std::vector<int32_t> fixed_twiddles(int n) {
+  typedef unsigned __int128 u128;
+  auto mulq = [](u128 a, u128 b) -> u128 {  // a b / 2^112 (truncated), a, b <= 2^112
+    a <<= 8;
+    b <<= 8;
+    const u128 m = ((u128)1 << 64) - 1, ah = a >> 64, al = a & m, bh = b >> 64, bl = b & m;
+    const u128 mid = ah * bl, mid2 = al * bh;
+    return ah * bh + (mid >> 64) + (mid2 >> 64) + (((mid & m) + (mid2 & m) + ((al * bl) >> 64)) >> 64);
+  };
+  const u128 one = (u128)1 << 112;
+  const u128 pi4 = ((u128)0xC90FDAA22168C234ull << 48) | (0xC4C6628B80DC1CD1ull >> 16);  // pi/4 in units of 2^-112
+  auto sincos = [&](int num, u128 *s, u128 *c) {  // angle (pi/4) num / n, num <= n
+    const u128 x = pi4 / (unsigned)n * (unsigned)num, x2 = mulq(x, x);
+    u128 ts = x, tc = one, ss = x, cc = one;
+    for (int k = 1; k < 16 && tc; k++) {
+      tc = mulq(tc, x2) / (unsigned)((2 * k - 1) * (2 * k));
+      ts = mulq(ts, x2) / (unsigned)((2 * k) * (2 * k + 1));
+      if (k & 1) {
+        cc -= tc;
+        ss -= ts;
+      } else {
+        cc += tc;
+        ss += ts;
+      }
+    }
+    *s = ss;
+    *c = cc;
+  };
+  std::vector<int32_t> out(4 * (size_t)n);
+  for (int t = 0; t < n; t++) {
+    const long q = 4L * t / n, r = 4L * t - q * n;  // quadrant and (pi/2) r / n inside it
+    u128 s, c;
+    if (2 * r <= n) {
+      sincos((int)(2 * r), &s, &c);
+    } else {
+      sincos((int)(2 * (n - r)), &c, &s);
+    }
+    const int64_t si = (int64_t)((s + ((u128)1 << 49)) >> 50), ci = (int64_t)((c + ((u128)1 << 49)) >> 50);
+    int64_t re = 0, im = 0;
+    switch (q & 3) {
+      case 0: re = ci; im = -si; break;
+      case 1: re = -si; im = -ci; break;
+      case 2: re = -ci; im = si; break;
+      default: re = si; im = ci; break;
+    }
+    auto split = [](int64_t v, int32_t *h, int32_t *l) {
+      if ((int32_t)(uint32_t)v == INT32_MIN) v++;  // keeps the low part's negative representable
+      *l = (int32_t)(uint32_t)v;
+      *h = (int32_t)((v - *l) / (int64_t)4294967296);
+    };
+    split(re, &out[4 * (size_t)t], &out[4 * (size_t)t + 1]);
+    split(im, &out[4 * (size_t)t + 2], &out[4 * (size_t)t + 3]);
+  }
+  return out;
+}
+
 // Fourier eigenvalue of mode J of the periodic second difference
 // (src/fluid/compute_potential.c:112-115)
 inline double poisson_eigenvalue(double dy, int jtot, int J) {

@@ -19,9 +19,9 @@
 // mode line in the interleaved order p = (x % m) * 32 + x / m (m = nx / 32):
 // lane k walks segment k, and at every step the 32 lanes touch 32
 // consecutive elements, in global and in shared memory alike. The forward
-// and inverse DFTs write and read that order: a radix-8 Stockham FFT in
-// registers for 16 <= jtot <= 8192 (fft_stockham.cuh), the Thomas form's
-// radix-2/4 FFT otherwise.
+// and inverse DFTs write and read that order: in 64-bit fixed point for
+// 16 <= jtot <= 8192 (fft_fixed.cuh), by the Thomas form's radix-2/4 FFT
+// otherwise.
 //
 // The Crank-Nicolson lines (src/linalg.c:9-108) are solved by the same
 // partition method: one warp per row along x (k_par_cn), one thread per
@@ -32,7 +32,7 @@
 #include <cstdint>
 
 #include "fft_dev.cuh"
-#include "fft_stockham.cuh"
+#include "fft_fixed.cuh"
 #include "host_common.h"
 #include "sns_gpu.h"
 #include "sns_internal.h"
@@ -115,110 +115,84 @@ __global__ void __launch_bounds__(256) k_par_bwd(const ParArgs a) {
   }
 }
 
-// ---- the same two transforms by the radix-8 Stockham FFT (fft_stockham.cuh),
-// for 16 <= jtot <= 8192. The solve is linear, so this pair moves two
-// constant factors to the inverse's final scale: the forward transforms
-// div u* without the factor 1/(gamma dt) and leaves the real FFT's split
-// step unhalved (2 X), and the inverse multiplies by 1/(gamma dt) / (2 jtot)
-// (an exact power-of-two scaling of 1/(gamma dt)). Both kernels run C
-// columns per block on C jtot / 16 threads, 8 complex values per thread.
+// ---- the same two transforms in 64-bit fixed point (fft_fixed.cuh), for
+// 16 <= jtot <= 8192: 3 FP64 instructions per value forward and 2 inverse, the
+// rest integer, where the FP64 transforms took about 20 each. The solve is
+// linear, so this pair moves two constant
+// factors to the inverse's final scale: the forward transforms div u* without
+// the factor 1/(gamma dt) and leaves the real FFT's split step unhalved
+// (2 X), and the inverse multiplies by 1/(gamma dt) / (2 jtot).
+
+struct FixArgs {
+  DevGrid g;
+  const double *ux, *uy;
+  double2 *spec;  // [nh][nx], interleaved rows
+  double *psi;
+  double scale;   // of the inverse
+  int lgC;        // 2^lgC adjacent x columns per block
+  int m;          // rows per segment, nx / 32
+};
 
 // src/fluid/compute_potential.c:69-92: div u* along two rows per complex
-// element (z[m] = d[2m] + i d[2m+1]), its FFT, and 2 X[k] of the real
-// transform at the columns' line positions
-__global__ void __launch_bounds__(512) k_par_fwd8(const ParArgs a) {
-  extern __shared__ double2 z[];
-  const int nx = a.g.nx, ny = a.g.ny, M = ny / 2, C = a.cols;
-  const int x0 = blockIdx.x * C;
+// element (z[m] = d[2m] + i d[2m+1]) and 2 X[k] of its real transform at the
+// columns' line positions. On uniform grids whose spacings are powers of two
+// (DevGrid::p2u) the divergence is formed without the factor 1/dx, which joins the exponent:
+// the same bits in 3 FP64 instructions per value instead of 4.
+template <int V>
+__global__ void __launch_bounds__(512, 1) k_par_fwd_fx(const FixArgs a) {
+  extern __shared__ __align__(16) unsigned char fx_sm[];
+  __shared__ fx::Slots slots;
+  const int nx = a.g.nx, ny = a.g.ny, x0 = blockIdx.x << a.lgC;
   const double rdy = a.g.rdy;
-  const double2 *tw = reinterpret_cast<const double2 *>(a.g.tw);
-  for (int e = threadIdx.x; e < C * M; e += blockDim.x) {
-    const int c = e % C, mm = e / C, x = x0 + c;
-    double2 d = make_double2(0.0, 0.0);
-    if (x < nx) {
-      const size_t r0 = (size_t)(2 * mm) * nx + x, r1 = r0 + nx;
-      const size_t r2 = (size_t)(2 * mm + 2 == ny ? 0 : 2 * mm + 2) * nx + x;
-      const bool right = x == nx - 1;
-      const double rdx = a.g.rdxf[x];
-      const double u0m = a.ux[r0], u0p = right ? 0.0 : a.ux[r0 + 1];
-      const double u1m = a.ux[r1], u1p = right ? 0.0 : a.ux[r1 + 1];
-      const double v0 = a.uy[r0], v1 = a.uy[r1], v2 = a.uy[r2];
-      d.x = (u0p - u0m) * rdx + (v1 - v0) * rdy;
-      d.y = (u1p - u1m) * rdx + (v2 - v1) * rdy;
-    }
-    z[c * M + fft8::swz(mm)] = d;
-  }
-  __syncthreads();
-  fft8::transform<true, 1>(z, C, M, tw);
-  // split step for the bin pair (k, M-k): 2 X[k] = (Z[k] + conj Z[M-k]) +
-  // w^k (Z[k] - conj Z[M-k]) / i, w = exp(-2 pi i / jtot)
-  const int half = M / 2 + 1;
-  for (int e = threadIdx.x; e < C * half; e += blockDim.x) {
-    const int c = e % C, k = e / C, x = x0 + c;
-    if (x >= nx) continue;
-    const double2 *zc = z + c * M;
-    double2 *out = a.spec + par_p(x, a.m);
-    const size_t os = (size_t)nx;
-    if (k == 0) {
-      const double2 z0 = zc[0];
-      const double s = z0.x + z0.y, t = z0.x - z0.y;
-      out[0] = make_double2(s + s, 0.0);
-      out[(size_t)M * os] = make_double2(t + t, 0.0);
+  const bool p2 = a.g.p2u;
+  const int eoff = p2 ? ((__double2hiint(a.g.rdxf[0]) >> 20) & 0x7ff) - 1023 : 0;
+  const double ratio = p2 ? rdy * a.g.dxf[0] : 0.0;
+  auto in = [&](int c, int mm, double *d) {
+    const int x = x0 + c;
+    d[0] = d[1] = 0.0;
+    if (x >= nx) return;
+    const size_t r0 = (size_t)(2 * mm) * nx + x, r1 = r0 + nx;
+    const size_t r2 = (size_t)(2 * mm + 2 == ny ? 0 : 2 * mm + 2) * nx + x;
+    const bool right = x == nx - 1;
+    const double u0m = a.ux[r0], u0p = right ? 0.0 : a.ux[r0 + 1];
+    const double u1m = a.ux[r1], u1p = right ? 0.0 : a.ux[r1 + 1];
+    const double v0 = a.uy[r0], v1 = a.uy[r1], v2 = a.uy[r2];
+    if (p2) {
+      d[0] = fma(v1 - v0, ratio, u0p - u0m);
+      d[1] = fma(v2 - v1, ratio, u1p - u1m);
     } else {
-      const double2 A = zc[fft8::swz(k)], B = zc[fft8::swz(M - k)];
-      const double sre = A.x + B.x, dim = A.y - B.y, dre = A.x - B.x, sim = A.y + B.y;
-      const double2 w = tw[k];
-      const double wor = w.x * sim + w.y * dre;
-      const double woi = w.y * sim - w.x * dre;
-      out[(size_t)k * os] = make_double2(sre + wor, dim + woi);
-      if (2 * k != M) out[(size_t)(M - k) * os] = make_double2(sre - wor, woi - dim);
+      const double rdx = a.g.rdxf[x];
+      d[0] = (u0p - u0m) * rdx + (v1 - v0) * rdy;
+      d[1] = (u1p - u1m) * rdx + (v2 - v1) * rdy;
     }
-  }
+  };
+  auto out = [&](int c, int k, double2 X) {
+    const int x = x0 + c;
+    if (x < nx) a.spec[(size_t)k * nx + par_p(x, a.m)] = X;
+  };
+  fx::forward<V>(reinterpret_cast<fx::C64 *>(fx_sm), &slots, a.lgC, ny / 2, reinterpret_cast<const fx::Tw *>(a.g.twx),
+              eoff, in, out);
 }
 
-// src/fluid/compute_potential.c:146-157: the inverse (2 Z[k] from the bin
-// pair, FFT, psi rows 2m and 2m+1 from element m) and the final scale
-__global__ void __launch_bounds__(512) k_par_bwd8(const ParArgs a) {
-  extern __shared__ double2 z[];
-  const int nx = a.g.nx, ny = a.g.ny, M = ny / 2, C = a.cols;
-  const int x0 = blockIdx.x * C;
-  const double2 *tw = reinterpret_cast<const double2 *>(a.g.tw);
-  const int half = M / 2 + 1;
-  for (int e = threadIdx.x; e < C * half; e += blockDim.x) {
-    const int c = e % C, k = e / C, x = x0 + c;
-    double2 *zc = z + c * M;
-    if (x >= nx) {
-      zc[fft8::swz(k)] = make_double2(0.0, 0.0);
-      if (k > 0) zc[fft8::swz(M - k)] = make_double2(0.0, 0.0);
-      continue;
-    }
-    const double2 *in = a.spec + par_p(x, a.m);
-    const size_t is = (size_t)nx;
-    if (k == 0) {
-      // imaginary parts of X[0] and X[M] ignored (FFTW's c2r convention)
-      const double x0r = in[0].x, xmr = in[(size_t)M * is].x;
-      zc[0] = make_double2(x0r + xmr, x0r - xmr);
-    } else {
-      const double2 A = in[(size_t)k * is], B = in[(size_t)(M - k) * is];
-      const double er = A.x + B.x, ei = A.y - B.y, dr = A.x - B.x, di = A.y + B.y;
-      const double2 w = tw[k];
-      const double orr = dr * w.x + di * w.y;
-      const double oi = di * w.x - dr * w.y;
-      zc[fft8::swz(k)] = make_double2(er - oi, ei + orr);
-      if (2 * k != M) zc[fft8::swz(M - k)] = make_double2(er + oi, orr - ei);
-    }
-  }
-  __syncthreads();
-  fft8::transform<false, 1>(z, C, M, tw);
-  const double scale = a.s.rgdt * (0.5 * a.s.rny);
-  for (int e = threadIdx.x; e < C * M; e += blockDim.x) {
-    const int c = e % C, mm = e / C, x = x0 + c;
-    if (x >= nx) continue;
-    const double2 v = z[c * M + fft8::swz(mm)];
+// src/fluid/compute_potential.c:146-157: the inverse into psi
+template <int V>
+__global__ void __launch_bounds__(512, 1) k_par_bwd_fx(const FixArgs a) {
+  extern __shared__ __align__(16) unsigned char fx_sm[];
+  __shared__ fx::Slots slots;
+  const int nx = a.g.nx, x0 = blockIdx.x << a.lgC;
+  auto in = [&](int c, int k) -> double2 {
+    const int x = x0 + c;
+    return x < nx ? a.spec[(size_t)k * nx + par_p(x, a.m)] : make_double2(0.0, 0.0);
+  };
+  auto out = [&](int c, int mm, const double *d) {
+    const int x = x0 + c;
+    if (x >= nx) return;
     const size_t r0 = (size_t)(2 * mm) * nx + x;
-    a.psi[r0] = v.x * scale;
-    a.psi[r0 + nx] = v.y * scale;
-  }
+    a.psi[r0] = d[0];
+    a.psi[r0 + nx] = d[1];
+  };
+  fx::inverse<V>(reinterpret_cast<fx::C64 *>(fx_sm), &slots, a.lgC, a.g.ny / 2,
+              reinterpret_cast<const fx::Tw *>(a.g.twx), a.scale, in, out);
 }
 
 struct ParTriArgs {
@@ -680,10 +654,7 @@ __global__ void __launch_bounds__(32 * kCnCols) k_par_cn_cols(const ParCnArgs a)
   }
 }
 
-// adjacent columns per block of the DFT kernels, where the shared memory
-// allows it. Measured at 512 x 1024 (parallel-form step, CUDA events): 1, 2,
-// 4 and 8 columns 0.513, 0.511, 0.538 and 0.724 ms per step: whole sectors
-// of the velocity rows (4 and more) cost more in blocks per SM than they save
+// adjacent columns per block of the FP64 DFT kernels
 constexpr int kParCols = 2;
 int par_cols(const DevGrid &g) {
   int c = kParCols;
@@ -717,35 +688,61 @@ bool parallel_tri_supported(int nx, int ny) {
 }
 
 namespace {
-// the radix-8 Stockham pair: 16 <= jtot <= 8192 (at most 512 threads a block)
-bool par_fft8(const DevGrid &g) { return g.ny >= 16 && g.ny <= 8192; }
+// the fixed-point pair: 16 <= jtot <= 8192 (at most 512 threads a block)
+bool par_fixed(const DevGrid &g) { return g.ny >= 16 && g.ny <= 8192; }
 
 void par_dft_attributes() {
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_par_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     cudaFuncSetAttribute(k_par_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    cudaFuncSetAttribute(k_par_fwd8, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    cudaFuncSetAttribute(k_par_bwd8, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+    cudaFuncSetAttribute(k_par_fwd_fx<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+    cudaFuncSetAttribute(k_par_bwd_fx<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+    cudaFuncSetAttribute(k_par_fwd_fx<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
+    cudaFuncSetAttribute(k_par_bwd_fx<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
     attr = true;
   }
 }
 
-// columns per block of the radix-8 pair: C jtot / 16 threads, C jtot 8 bytes
-int par_cols8(const DevGrid &g) {
-  int c = kParCols;
-  while (c > 1 && ((size_t)c * g.ny * sizeof(double) > 128 * 1024 || c * g.ny / 16 > 512)) c /= 2;
-  return c;
+// values per thread, columns per block (log2) and threads of the fixed-point
+// pair: jtot / 2V threads a column. One warp's instruction latency bounds the
+// pair on small grids, the instruction count on large ones: 4 values per
+// thread below kFix8Warps warps of 8. us per launch, forward (beside the
+// temperature update) / inverse, 8 against 4 values:
+//   128 x 256   19.9 / 14.3, 14.3 / 12.2    512 x 512   23.9 / 14.9, 18.2 / 12.9
+//   512 x 1024  27.7 / 17.0, 26.2 / 18.2    1024 x 2048 64.8 / 43.2, 86.2 / 61.3
+//   2048 x 4096 234 / 168, 341 / 257
+// (the FP64 radix-8 pair: 22.4 / 19.9 at 128 x 256, 45 / 30 at 512 x 1024,
+// 410 / 364 at 2048 x 4096). Columns per block 1, 2, 4: within 5% at 512 x 1024,
+// 2 the best from 256 x 512 to 1024 x 2048.
+constexpr long kFix8Warps = 1024;
+constexpr int kFixLg = 1;
+struct FixShape {
+  int v, lgC, threads;
+  size_t smem;
+};
+FixShape fix_shape(const DevGrid &g) {
+  FixShape f;
+  f.v = (long)g.nx * (g.ny / 16) / 32 >= kFix8Warps || g.ny > 4096 ? 8 : 4;
+  f.lgC = kFixLg;
+  const int n = g.ny / 2 / f.v;
+  while (f.lgC < 4 && (n << f.lgC) < 32) f.lgC++;
+  while (f.lgC > 0 && (n << f.lgC) > 512) f.lgC--;
+  f.threads = std::max(32, n << f.lgC);
+  f.smem = ((size_t)fx::column_stride(g.ny / 2, f.lgC) << f.lgC) * sizeof(fx::C64);
+  return f;
 }
 }  // namespace
 
 cudaError_t launch_par_fwd(const DevGrid &g, const StageScalars &s, const double *ux, const double *uy,
                            double2 *spec, cudaStream_t st) {
   par_dft_attributes();
-  if (par_fft8(g)) {
-    const int C = par_cols8(g);
-    const ParArgs a{g, s, ux, uy, spec, nullptr, C, g.nx / kPartSeg};
-    k_par_fwd8<<<(g.nx + C - 1) / C, C * g.ny / 16, (size_t)C * g.ny * sizeof(double), st>>>(a);
+  if (par_fixed(g)) {
+    const FixShape f = fix_shape(g);
+    const FixArgs a{g, ux, uy, spec, nullptr, 0.0, f.lgC, g.nx / kPartSeg};
+    const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
+    if (f.v == 8) k_par_fwd_fx<8><<<blocks, f.threads, f.smem, st>>>(a);
+    else k_par_fwd_fx<4><<<blocks, f.threads, f.smem, st>>>(a);
   } else {
     const int C = par_cols(g);
     const ParArgs a{g, s, ux, uy, spec, nullptr, C, g.nx / kPartSeg};
@@ -817,10 +814,13 @@ cudaError_t launch_par_cn(bool columns, ParCnArgs a, cudaStream_t st) {
 cudaError_t launch_par_bwd(const DevGrid &g, const StageScalars &s, const double2 *spec, double *psi,
                            cudaStream_t st) {
   par_dft_attributes();
-  if (par_fft8(g)) {
-    const int C = par_cols8(g);
-    const ParArgs a{g, s, nullptr, nullptr, const_cast<double2 *>(spec), psi, C, g.nx / kPartSeg};
-    k_par_bwd8<<<(g.nx + C - 1) / C, C * g.ny / 16, (size_t)C * g.ny * sizeof(double), st>>>(a);
+  if (par_fixed(g)) {
+    const FixShape f = fix_shape(g);
+    const FixArgs a{g,     nullptr, nullptr, const_cast<double2 *>(spec), psi, s.rgdt * (0.5 * s.rny),
+                    f.lgC, g.nx / kPartSeg};
+    const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
+    if (f.v == 8) k_par_bwd_fx<8><<<blocks, f.threads, f.smem, st>>>(a);
+    else k_par_bwd_fx<4><<<blocks, f.threads, f.smem, st>>>(a);
   } else {
     const int C = par_cols(g);
     const ParArgs a{g, s, nullptr, nullptr, const_cast<double2 *>(spec), psi, C, g.nx / kPartSeg};

@@ -327,6 +327,8 @@ static int build_context(Context *c, const param_t *param) {
     for (int i = 0; i <= nx; i++) ok = ok && p2(rdxc[i]);
     for (int i = 1; i < nx; i++) ok = ok && p2(cfm[i]) && p2(cfp[i]);
     g.p2 = ok;
+    g.p2u = ok;
+    for (double v : c->dxf) g.p2u = g.p2u && v == c->dxf[0];
   }
   int rc = SNS_OK;
   g.dv2 = false;
@@ -1170,6 +1172,7 @@ static int parallel_prepare(Context *c) {
     std::copy(blk.begin() + nx, blk.end(), o + 2 * (size_t)nx);         // up v w alpha beta rD
   }
   int rc = SNS_OK;
+  if ((rc = upload(c, &c->g.twx, fixed_twiddles(ny)))) return rc;
   if ((rc = upload(c, &c->par.fac, fac)) || (rc = upload(c, &c->par.lo, lo)) || (rc = upload(c, &c->par.hi, hi)))
     return rc;
   if ((rc = dev_alloc(c, &c->par.err, (size_t)1))) return rc;

@@ -28,6 +28,7 @@ struct DevGrid {
   int nx, ny, nh, jpitch;  // nh = ny/2 + 1 Fourier modes; jpitch >= nh
   bool rcp;                // every metric divisor is a power of two
   bool p2;                 // rcp, and every reciprocal spacing, advective and Poisson coefficient is 2^e, |e| <= 64
+  bool p2u;                // p2, and every DXF(i) is the same
   bool dv2;                // not rcp, and division by dy takes two instructions (invariant_divisor in host_common.h)
   double dy, rdy, rdyl;    // rdyl, rdxf_l, rdxc_l: with the reciprocal the pair that divides (NaN where none does)
   const double *dxf;    // [nx]    DXF(i)
@@ -46,6 +47,7 @@ struct DevGrid {
   const double *pinv;   // [nx * jpitch]   1./pivot; 0 where |pivot| < DBL_EPSILON (row forced to 0)
   const double *pup;    // [nx * jpitch]   normalised upper diagonal
   const double *tw;     // [2*ny]          twiddles exp(-2 pi i t/ny), t < ny
+  const int *twx;       // [4*ny]  the same for the fixed-point DFTs (fft_fixed.cuh; set with the parallel form)
   int fft_nst;          // stages of the length-ny/2 complex FFT
   int fft_first2;       // first stage radix 2 (else all radix 4)
 };
