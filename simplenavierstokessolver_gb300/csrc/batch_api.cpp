@@ -53,7 +53,7 @@ static size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 // byte layout of one case inside its arena block
 struct CaseLayout {
   size_t rdxf_f, rdxc_f, ccm_f, ccp_f, cfm_f, cfp_f, rdxf_l;
-  size_t rdxf, rdxc, dxi, dxf, dxc, tw, lo, hi, pfac, ccm, ccp, cfm, cfp;
+  size_t rdxf, rdxc, dxi, dxf, dxc, tw, twx, lo, hi, pfac, ccm, ccp, cfm, cfp;
   size_t ux[2], uy[2], t[2], uxl[2], uyl[2], tl[2], aux, auy, at, auxl, auyl, atl, p, psi, spec;
   size_t total;
   size_t pstride;
@@ -84,6 +84,7 @@ static CaseLayout layout_for(int nx, int ny, bool x2) {
   L.dxf = take(sizeof(double) * nx);
   L.dxc = take(sizeof(double) * (nx + 1));
   L.tw = take(sizeof(double) * 2 * ny);
+  L.twx = take(sizeof(int32_t) * 4 * ny);
   L.lo = take(sizeof(double) * nx);
   L.hi = take(sizeof(double) * nx);
   L.pstride = 4 * (size_t)nx + 2 * kPcrLevels * kSeg + kSeg;
@@ -168,7 +169,6 @@ struct CaseHost {
   sns_case_desc d{};
   size_t off = 0, bytes = 0;
   long long steps_done = 0;  // host mirror: every unfinished case advances one step per batch step
-  int fcols = 1;
 };
 
 }  // namespace sns
@@ -257,15 +257,18 @@ static int ensure_device_list(T **ptr, size_t *cap, size_t need) {
 }
 
 // work lists for the current case set and the graph of one step
-// DFT columns per block for a case under the current tuning: the admission
-// default scaled by 2^fcols_shift, within [1, 16], nx and 160 KiB of shared memory
-static int tuned_fcols(const sns_batch *b, const CaseHost &h) {
-  int fc = h.fcols;
-  if (b->tune.fcols_shift > 0) fc <<= b->tune.fcols_shift;
-  if (b->tune.fcols_shift < 0) fc >>= -b->tune.fcols_shift;
-  fc = std::max(1, std::min(fc, 16));
-  while (fc > 1 && (fc > h.d.itot || sizeof(double) * (size_t)fc * h.d.jtot > 160 * 1024)) fc >>= 1;
-  return fc;
+// threads of a column DFT block under the current tuning: kFftThreads times
+// 2^fcols_shift, enough for one column of the longest resident case; the
+// persistent launch's 256 threads otherwise. 128 threads take 2 columns of
+// jtot 1024, 16 of jtot 128; 512 x 1024 alone steps in 221 us with 128 and 214
+// with 256, twelve mixed cases in 244 with 128 (the autotuner's choice)
+constexpr int kFftThreads = 128;
+static int tuned_fft_threads(const sns_batch *b, int ny_max) {
+  if (b->persistent) return 256;
+  int t = kFftThreads;
+  if (b->tune.fcols_shift > 0) t <<= b->tune.fcols_shift;
+  if (b->tune.fcols_shift < 0) t >>= -b->tune.fcols_shift;
+  return std::max(std::max(32, std::min(t, 512)), ny_max / 16);
 }
 
 static int rebuild(sns_batch *b) {
@@ -273,13 +276,16 @@ static int rebuild(sns_batch *b) {
   std::vector<BCols> cols;
   std::vector<BModes> modes;
   size_t smem = 0;
-  int threads = 64;
   const int tx = b->tune.tile_x, ty = b->tune.tile_rows;
   // the tridiagonal launch stages each warp's line in shared memory: fewer
   // warps per block when the longest line would not fit
-  int nmax = 32;
+  int nmax = 32, ny_max = 8;
   for (const CaseHost &h : b->hc)
-    if (h.used && !(h.d.steps > 0 && h.steps_done >= h.d.steps)) nmax = std::max(nmax, h.d.itot);
+    if (h.used && !(h.d.steps > 0 && h.steps_done >= h.d.steps)) {
+      nmax = std::max(nmax, h.d.itot);
+      ny_max = std::max(ny_max, h.d.jtot);
+    }
+  const int threads = tuned_fft_threads(b, ny_max);
   int mpb = b->tune.modes_per_block;
   while (mpb > 1 && batch_tri_smem(nmax, mpb) > 200 * 1024) mpb /= 2;
   if (b->persistent) mpb = std::min(mpb, 4);  // the persistent launch's four line slots per block
@@ -288,7 +294,7 @@ static int rebuild(sns_batch *b) {
     if (!h.used) continue;
     if (h.d.steps > 0 && h.steps_done >= h.d.steps) continue;
     const int nx = h.d.itot, ny = h.d.jtot, nh = ny / 2 + 1;
-    const int fc = tuned_fcols(b, h);
+    const int fc = batch_fft_cols(ny, threads);
     if (b->table[c].fcols != fc) {  // the kernels read a case's column count from its table entry
       b->table[c].fcols = fc;
       BCUDA(cudaMemcpyAsync(reinterpret_cast<char *>(b->d_cases + c) + offsetof(BCase, fcols), &b->table[c].fcols,
@@ -298,8 +304,7 @@ static int rebuild(sns_batch *b) {
       for (int x0 = 0; x0 < nx; x0 += tx) (h.d.compensated ? tiles_x2 : tiles).push_back({c, x0, y0});
     for (int x0 = 0; x0 < nx; x0 += fc) cols.push_back({c, x0});
     for (int j0 = 0; j0 < nh; j0 += mpb) modes.push_back({c, j0});
-    smem = std::max(smem, sizeof(double) * (size_t)fc * ny);
-    threads = std::max(threads, std::min(256, (fc * (ny / 2) / 4 + 31) / 32 * 32));
+    smem = std::max(smem, batch_fft_smem(ny, fc, threads));
   }
   const int nx2 = (int)tiles_x2.size();
   tiles.insert(tiles.end(), tiles_x2.begin(), tiles_x2.end());
@@ -359,7 +364,7 @@ static int rebuild(sns_batch *b) {
     if ((err = launch_batch_tri(b->d_cases, b->d_modes, b->nmodes, mpb, nmax, b->d_err, b->tri_spin,
                                 rk == 0 ? b->tri_stale : 0, b->stream)) != cudaSuccess)
       break;
-    if ((err = launch_batch_bwd(b->d_cases, b->d_cols, b->ncols, b->fft_smem, b->fft_threads, b->stream)) !=
+    if ((err = launch_batch_bwd(b->d_cases, b->d_cols, b->ncols, rk, b->fft_smem, b->fft_threads, b->stream)) !=
         cudaSuccess)
       break;
     if ((err = launch_batch_corr(b->d_cases, b->d_tiles, b->ntiles, rk, tx, ty, b->stream)) != cudaSuccess) break;
@@ -517,6 +522,7 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
     partition_factors(nx, lo.data(), hi.data(), l_raw.data(), u_raw.data(), poisson_eigenvalue(dy, ny, J), J == 0,
                       false, pfac.data() + L.pstride * J);
   const std::vector<double> tw = twiddle_table(ny);
+  const std::vector<int32_t> twx = fixed_twiddles(ny);
   std::vector<double> temp((size_t)(nx + 2) * (ny + 2));
   if (st) temp_init = st->temp;
   if (temp_init) {
@@ -553,6 +559,7 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
   chk(put(L.dxf, dxf.data(), sizeof(double) * nx));
   chk(put(L.dxc, dxc.data(), sizeof(double) * (nx + 1)));
   chk(put(L.tw, tw.data(), sizeof(double) * tw.size()));
+  chk(put(L.twx, twx.data(), sizeof(int32_t) * twx.size()));
   chk(put(L.lo, lo.data(), sizeof(double) * nx));
   chk(put(L.hi, hi.data(), sizeof(double) * nx));
   chk(put(L.pfac, pfac.data(), sizeof(double) * pfac.size()));
@@ -620,9 +627,23 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
   t.ny = ny;
   t.nh = nh;
   fft_layout(ny, &t.fft_nst, &t.fft_first2);
-  int fc = std::min(8192 / ny, nx / 128);
-  fc = std::max(1, std::min(8, fc));
-  t.fcols = fc;
+  t.fcols = 0;  // set with the work lists
+  t.p2 = 0;
+  {
+    // uniform with power-of-two spacings: the divergence as a sum of two floats
+    auto pow2 = [](double v) {
+      int e;
+      return std::frexp(v, &e) == 0.5;
+    };
+    const double rdy = 1.0 / dy, ratio = rdy * dxf[0];
+    bool ok = pow2(rdy) && pow2(rdxf[0]) && ratio >= 0x1p-20 && ratio <= 0x1p20;
+    for (int i = 1; i < nx; i++) ok = ok && dxf[i] == dxf[0];
+    int e;
+    std::frexp(rdxf[0], &e);
+    t.p2 = ok ? 1 : 0;
+    t.eoff = e - 1;
+    t.ratio_f = (float)ratio;
+  }
   t.with_t = d->with_temperature ? 1 : 0;
   t.with_force = d->with_thermal_forcing ? 1 : 0;
   t.seg = nx / kSeg;
@@ -661,6 +682,7 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
   t.dxf = reinterpret_cast<const double *>(base + L.dxf);
   t.dxc = reinterpret_cast<const double *>(base + L.dxc);
   t.tw = reinterpret_cast<const double *>(base + L.tw);
+  t.twx = reinterpret_cast<const int *>(base + L.twx);
   t.lo = reinterpret_cast<const double *>(base + L.lo);
   t.hi = reinterpret_cast<const double *>(base + L.hi);
   t.pfac = reinterpret_cast<const double *>(base + L.pfac);
@@ -715,7 +737,6 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
   h.off = off;
   h.bytes = L.total;
   h.steps_done = t.step;
-  h.fcols = fc;
   b->dirty = true;
   if (slot_out) *slot_out = slot;
   return SNS_OK;

@@ -7,7 +7,8 @@
 // significant bits) so that the per-substage rounding of the stored state
 // does not accumulate, while every stencil reads the hi words only; the pressure gradient, the divergence, the FFTs, the
 // tridiagonal solves, psi and p are FP64 (multiply-adds allowed: this form is
-// compared with the FP64 reference by error norms, not bits). The equations
+// compared with the FP64 reference by error norms, not bits), the FFTs in
+// 64-bit fixed point, below FP64's rounding. The equations
 // are the reference's (src/temperature/update.c:11-87, src/fluid/
 // update_velocity.c:11-192, src/fluid/compute_potential.c:69-157,
 // src/fluid/correct_velocity.c:6-42, src/fluid/update_pressure.c:7-60) with
@@ -25,7 +26,7 @@
 
 #include "batch_internal.h"
 #include "fft_dev.cuh"
-#include "fft_stockham.cuh"
+#include "fft_fixed.cuh"
 
 namespace sns {
 namespace {
@@ -370,116 +371,168 @@ __global__ void __launch_bounds__(kBTileXMax) k_b_stencil(const BCase *__restric
 }
 
 // ------------------------------------------------------------------- Poisson
-// The column DFTs run the radix-8 Stockham FFT (fft_stockham.cuh, 8 values
-// per thread) where the block's threads cover the column group that way, the
-// radix-2/4 stages otherwise (the block size is set by the largest case of
-// the batch)
-__device__ __forceinline__ bool stockham8(int M, int nc) { return M >= 8 && nc * M <= 8 * (int)blockDim.x; }
+// The column DFTs run in 64-bit fixed point (fft_fixed.cuh, radix 8: 8 values
+// per thread), where the block has jtot / 16 threads for each of its columns,
+// and by the radix-2/4 FP64 stages otherwise (jtot 8; jtot 8192 in the
+// persistent launch). Both move 1/(gamma dt) to the inverse's final scale.
+// Always 8 values per thread: the rounding of a case must not depend on what
+// it shares a launch with. 512 x 1024, forward / inverse, us per launch: 44 /
+// 31 in FP64 -> 20 / 14.
+__device__ __forceinline__ bool fixed_dft(int M, int nc) { return M >= 8 && nc * (M >> 3) <= (int)blockDim.x; }
 
-// FP64 divergence of the FP32 predicted velocity (src/fluid/compute_potential.c:74-86)
-// and the forward real DFT along y of `fcols` columns.
-// the block's column group x0 .. x0+fcols-1 (every thread of the block)
-__device__ __forceinline__ void fwd_cols(const BCase &C, int x0, int rk, double2 *zs) {
+// The divergence of the predicted velocity (src/fluid/compute_potential.c:74-86),
+// as what fx::forward reads: the sum of two floats where that is exact or to
+// the pairs' 48 bits (compensated cases, and FP32 cases on uniform grids whose
+// spacings are powers of two: no FP64 instruction), a double otherwise.
+struct DivIn {
+  const BCase &C;
+  const float *__restrict__ ux, *__restrict__ uy, *__restrict__ uxl, *__restrict__ uyl;
+  int x0;
+  bool pair;
+  static constexpr int kUnroll = 2;
+  __device__ __forceinline__ DivIn(const BCase &c, int pu, int x)
+      : C(c), ux(c.ux[pu]), uy(c.uy[pu]), uxl(c.uxl[pu]), uyl(c.uyl[pu]), x0(x), pair(c.x2 || c.p2) {}
+  // the differences at (x, y) as pairs; v0, v1: uy at rows y and y+1
+  __device__ __forceinline__ F2 dx(int x, size_t r) const {
+    const F2 u0{ux[r], uxl[r]};
+    const F2 u1 = x == C.nx - 1 ? F2{0.f, 0.f} : F2{ux[r + 1], uxl[r + 1]};
+    if (C.x2) return u1 - u0;
+    return F2{(u1.h - u0.h) + (u1.l - u0.l), 0.f};
+  }
+  __device__ __forceinline__ F2 dy(F2 v0, F2 v1) const {
+    if (C.x2) return v1 - v0;
+    return F2{(v1.h - v0.h) + (v1.l - v0.l), 0.f};
+  }
+  __device__ __forceinline__ F2 sum(int x, F2 du, F2 dv) const {
+    if (C.x2) return du * F2{C.rdxf_f[x], C.rdxf_l[x]} + dv * F2{C.rdy_f, C.rdy_l};
+    return F2{du.h, dv.h * C.ratio_f};
+  }
+  __device__ __forceinline__ double value(int x, F2 du, F2 dv) const {  // FP32 cases on other grids
+    return (double)du.h * C.rdxf[x] + (double)dv.h * C.rdy;
+  }
+  __device__ __forceinline__ unsigned load(int c, int mm, double2 &raw) const {
+    const int nx = C.nx, x = x0 + c;
+    raw = make_double2(0.0, 0.0);
+    if (x >= nx) return 0u;
+    const size_t r0 = (size_t)(2 * mm) * nx + x, r1 = r0 + nx;
+    const size_t r2 = (size_t)(2 * mm + 2 == C.ny ? 0 : 2 * mm + 2) * nx + x;
+    const F2 v0{uy[r0], uyl[r0]}, v1{uy[r1], uyl[r1]}, v2{uy[r2], uyl[r2]};
+    const F2 du0 = dx(x, r0), du1 = dx(x, r1), dv0 = dy(v0, v1), dv1 = dy(v1, v2);
+    if (pair) {
+      const F2 a = sum(x, du0, dv0), b = sum(x, du1, dv1);
+      raw = make_double2(__hiloint2double(__float_as_int(a.l), __float_as_int(a.h)),
+                         __hiloint2double(__float_as_int(b.l), __float_as_int(b.h)));
+      const unsigned e = max(max(fx::exponent_key(a.h), fx::exponent_key(a.l)),
+                             max(fx::exponent_key(b.h), fx::exponent_key(b.l)));
+      return e == 0u || e == 0x7ffu ? e : e + 1u;  // room for the sums
+    }
+    raw = make_double2(value(x, du0, dv0), value(x, du1, dv1));
+    return max(fx::exponent_key(raw.x), fx::exponent_key(raw.y));
+  }
+  __device__ __forceinline__ fx::C64 fixed(double2 d, int E, bool tiny) const {
+    if (pair) {
+      auto q = [&](double v) {
+        return fx::quantise(__int_as_float(__double2loint(v)), E) + fx::quantise(__int_as_float(__double2hiint(v)), E);
+      };
+      return fx::C64{q(d.x), q(d.y)};
+    }
+    return fx::C64{fx::quantise(fx::lift(d.x, tiny), E), fx::quantise(fx::lift(d.y, tiny), E)};
+  }
+  // the FP64 stages' input: row y of column x
+  __device__ __forceinline__ double at(int x, int y) const {
+    const size_t r = (size_t)y * C.nx + x, rn = (size_t)wup(y, C.ny) * C.nx + x;
+    const F2 du = dx(x, r), dv = dy(F2{uy[r], uyl[r]}, F2{uy[rn], uyl[rn]});
+    if (!C.x2) return value(x, du, dv);
+    const F2 v = sum(x, du, dv);
+    return (double)v.h + (double)v.l;
+  }
+};
+
+// the forward real DFT along y of the block's column group x0 ..
+// x0+fcols-1 (every thread of the block)
+__device__ __forceinline__ void fwd_cols(const BCase &C, int x0, int rk, double2 *zs, fx::Slots *slots) {
   const int nx = C.nx, ny = C.ny, M = ny / 2, nc = C.fcols;
-  const int pu = C.par ^ (rk & 1) ^ 1;
-  const float *__restrict__ ux = C.ux[pu];
-  const float *__restrict__ uy = C.uy[pu];
-  const float *__restrict__ uxl = C.uxl[pu];
-  const float *__restrict__ uyl = C.uyl[pu];
-  const double rgdt = C.rgdt[rk], rdy = C.rdy;
-  const F2 rg2 = ff(rgdt);
+  const DivIn in(C, C.par ^ (rk & 1) ^ 1, x0);
+  if (fixed_dft(M, nc)) {
+    auto out = [&](int c, int k, double2 X) {
+      if (x0 + c < nx) C.spec[(size_t)k * nx + x0 + c] = X;
+    };
+    fx::forward<8>(reinterpret_cast<fx::C64 *>(zs), slots, 31 - __clz(nc), M, reinterpret_cast<const fx::Tw *>(C.twx),
+                   C.p2 && !C.x2 ? C.eoff : 0, in, out);
+    return;
+  }
   double *zd = reinterpret_cast<double *>(zs);
-  const bool s8 = stockham8(M, nc);
   for (int e = threadIdx.x; e < nc * ny; e += blockDim.x) {
     const int c = e % nc, y = e / nc, x = x0 + c;
-    double d = 0.0;
-    if (x < nx) {
-      const size_t r = (size_t)y * nx + x;
-      const size_t ry = (size_t)wup(y, ny) * nx + x;
-      if (C.x2) {  // float-float on the FP32 pipes, one conversion pair at the end
-        const F2 u0{ux[r], uxl[r]};
-        const F2 dux = x == nx - 1 ? -u0 : F2{ux[r + 1], uxl[r + 1]} - u0;
-        const F2 duy = F2{uy[ry], uyl[ry]} - F2{uy[r], uyl[r]};
-        const F2 v = (dux * F2{C.rdxf_f[x], C.rdxf_l[x]} + duy * F2{C.rdy_f, C.rdy_l}) * rg2;
-        d = (double)v.h + (double)v.l;
-      } else {
-        const float dux = x == nx - 1 ? -(ux[r] + uxl[r]) : (ux[r + 1] - ux[r]) + (uxl[r + 1] - uxl[r]);
-        const float duy = (uy[ry] - uy[r]) + (uyl[ry] - uyl[r]);
-        d = rgdt * ((double)dux * C.rdxf[x] + (double)duy * rdy);
-      }
-    }
-    const int m = y >> 1;
-    zd[2 * (c * M + (s8 ? fft8::swz(m) : fft::fft_slot(m, M, C.fft_nst, C.fft_first2))) + (y & 1)] = d;
+    zd[2 * (c * M + fft::fft_slot(y >> 1, M, C.fft_nst, C.fft_first2)) + (y & 1)] = x < nx ? in.at(x, y) : 0.0;
   }
   __syncthreads();
   const double2 *tw = reinterpret_cast<const double2 *>(C.tw);
-  if (s8) {
-    fft8::transform<true, 1>(zs, nc, M, tw);
-  } else {
-    fft::fft_stages<true>(zs, nc, M, ny, C.fft_nst, C.fft_first2, tw);
-  }
+  fft::fft_stages<true>(zs, nc, M, ny, C.fft_nst, C.fft_first2, tw);
   const int half = M / 2 + 1;
   for (int e = threadIdx.x; e < nc * half; e += blockDim.x) {
     const int c = e % nc, k = e / nc, x = x0 + c;
-    if (x >= nx) continue;
-    if (s8) {
-      fft8::rfft_post(zs + c * M, C.spec + x, M, k, tw, (size_t)nx);
-    } else {
-      fft::rfft_post(zs + c * M, C.spec + x, M, k, tw, (size_t)nx);
-    }
+    if (x < nx) fft::rfft_post(zs + c * M, C.spec + x, M, k, tw, (size_t)nx);
   }
 }
 
-__global__ void __launch_bounds__(256) k_b_fwd(const BCase *__restrict__ cases, const BCols *__restrict__ cols,
-                                               int rk) {
+__global__ void __launch_bounds__(512, 1) k_b_fwd(const BCase *__restrict__ cases, const BCols *__restrict__ cols,
+                                                  int rk) {
   extern __shared__ double2 zs[];
+  __shared__ fx::Slots slots;
   const BCols it = cols[blockIdx.x];
   const BCase &C = cases[it.c];
   if (C.done) return;
-  fwd_cols(C, it.x0, rk, zs);
+  fwd_cols(C, it.x0, rk, zs, &slots);
 }
 
-// inverse DFT and 1/jtot (src/fluid/compute_potential.c:146-157)
-__device__ __forceinline__ void bwd_cols(const BCase &C, int x0, double2 *zs) {
+// inverse DFT with the factors 1/(gamma dt) and 1/jtot (src/fluid/compute_potential.c:146-157)
+__device__ __forceinline__ void bwd_cols(const BCase &C, int x0, int rk, double2 *zs, fx::Slots *slots) {
   const int nx = C.nx, ny = C.ny, M = ny / 2, nc = C.fcols;
+  const double scale = C.rgdt[rk] / ny;  // exact: jtot is a power of two
+  if (fixed_dft(M, nc)) {
+    auto in = [&](int c, int k) -> double2 {
+      return x0 + c < nx ? C.spec[(size_t)k * nx + x0 + c] : make_double2(0.0, 0.0);
+    };
+    auto out = [&](int c, int mm, const double *d) {
+      if (x0 + c >= nx) return;
+      const size_t r = (size_t)(2 * mm) * nx + x0 + c;
+      C.psi[r] = d[0];
+      C.psi[r + nx] = d[1];
+    };
+    fx::inverse<8>(reinterpret_cast<fx::C64 *>(zs), slots, 31 - __clz(nc), M, reinterpret_cast<const fx::Tw *>(C.twx),
+                   0.5 * scale, in, out);
+    return;
+  }
   const double2 *tw = reinterpret_cast<const double2 *>(C.tw);
-  const bool s8 = stockham8(M, nc);
   const int half = M / 2 + 1;
   for (int e = threadIdx.x; e < nc * half; e += blockDim.x) {
     const int c = e % nc, k = e / nc, x = x0 + c;
     double2 *zc = zs + c * M;
     if (x >= nx) {
-      zc[s8 ? fft8::swz(k) : fft::fft_slot(k, M, C.fft_nst, C.fft_first2)] = make_double2(0.0, 0.0);
-      if (k > 0) zc[s8 ? fft8::swz(M - k) : fft::fft_slot(M - k, M, C.fft_nst, C.fft_first2)] = make_double2(0.0, 0.0);
+      zc[fft::fft_slot(k, M, C.fft_nst, C.fft_first2)] = make_double2(0.0, 0.0);
+      if (k > 0) zc[fft::fft_slot(M - k, M, C.fft_nst, C.fft_first2)] = make_double2(0.0, 0.0);
       continue;
     }
-    if (s8) {
-      fft8::rfft_pre(C.spec + x, zc, M, k, tw, (size_t)nx);
-    } else {
-      fft::rfft_pre(C.spec + x, zc, M, k, tw, C.fft_nst, C.fft_first2, (size_t)nx);
-    }
+    fft::rfft_pre(C.spec + x, zc, M, k, tw, C.fft_nst, C.fft_first2, (size_t)nx);
   }
   __syncthreads();
-  if (s8) {
-    fft8::transform<false, 1>(zs, nc, M, tw);
-  } else {
-    fft::fft_stages<false>(zs, nc, M, ny, C.fft_nst, C.fft_first2, tw);
-  }
+  fft::fft_stages<false>(zs, nc, M, ny, C.fft_nst, C.fft_first2, tw);
   const double *zd = reinterpret_cast<const double *>(zs);
-  const double rny = 1.0 / ny;
   for (int e = threadIdx.x; e < nc * ny; e += blockDim.x) {
     const int c = e % nc, y = e / nc, x = x0 + c;
-    const int m = y >> 1;
-    if (x < nx) C.psi[(size_t)y * nx + x] = zd[2 * (c * M + (s8 ? fft8::swz(m) : m)) + (y & 1)] * rny;
+    if (x < nx) C.psi[(size_t)y * nx + x] = zd[2 * (c * M + (y >> 1)) + (y & 1)] * scale;
   }
 }
 
-__global__ void __launch_bounds__(256) k_b_bwd(const BCase *__restrict__ cases, const BCols *__restrict__ cols) {
+__global__ void __launch_bounds__(512, 1) k_b_bwd(const BCase *__restrict__ cases, const BCols *__restrict__ cols,
+                                                  int rk) {
   extern __shared__ double2 zs[];
+  __shared__ fx::Slots slots;
   const BCols it = cols[blockIdx.x];
   const BCase &C = cases[it.c];
   if (C.done) return;
-  bwd_cols(C, it.x0, zs);
+  bwd_cols(C, it.x0, rk, zs, &slots);
 }
 
 // Partition-method solve of the mode lines J = j0 .. j0+w-1 (one warp each).
@@ -763,6 +816,7 @@ struct SubstageArgs {
 
 __global__ void __launch_bounds__(256, 2) k_b_substage(const SubstageArgs a) {
   extern __shared__ __align__(128) unsigned char sm[];
+  __shared__ fx::Slots slots;
   const int tid = threadIdx.x, nthr = blockDim.x;
   // 1) stencils: nthr / tile_x tiles per block at a time (FP32 tiles first,
   //    then compensated ones)
@@ -791,7 +845,7 @@ __global__ void __launch_bounds__(256, 2) k_b_substage(const SubstageArgs a) {
   for (int i = blockIdx.x; i < a.ncols; i += gridDim.x) {
     const BCols it = a.cols[i];
     const BCase &C = a.cases[it.c];
-    if (!C.done) fwd_cols(C, it.x0, a.rk, zs);
+    if (!C.done) fwd_cols(C, it.x0, a.rk, zs, &slots);
     __syncthreads();
   }
   grid_barrier(a.bar, a.bar + 1, a.err);
@@ -814,7 +868,7 @@ __global__ void __launch_bounds__(256, 2) k_b_substage(const SubstageArgs a) {
   for (int i = blockIdx.x; i < a.ncols; i += gridDim.x) {
     const BCols it = a.cols[i];
     const BCase &C = a.cases[it.c];
-    if (!C.done) bwd_cols(C, it.x0, zs);
+    if (!C.done) bwd_cols(C, it.x0, a.rk, zs, &slots);
     __syncthreads();
   }
   grid_barrier(a.bar, a.bar + 1, a.err);
@@ -889,6 +943,19 @@ cudaError_t launch_batch_stencil(const BCase *cases, const BTile *tiles, int nti
   return cudaGetLastError();
 }
 
+int batch_fft_cols(int ny, int threads) {
+  int c = 1;
+  while (c < fx::kMaxCols && 2 * c * (ny / 16) <= threads) c *= 2;
+  return c;
+}
+
+size_t batch_fft_smem(int ny, int cols, int threads) {
+  if (ny < 16 || cols * (ny / 16) > threads) return sizeof(double) * (size_t)cols * ny;
+  int lg = 0;
+  while (1 << lg < cols) lg++;
+  return sizeof(fx::C64) * ((size_t)fx::column_stride(ny / 2, lg) << lg);
+}
+
 cudaError_t launch_batch_fwd(const BCase *cases, const BCols *cols, int ncols, int rk, size_t smem, int threads,
                              cudaStream_t st) {
   if (ncols == 0) return cudaSuccess;
@@ -896,10 +963,10 @@ cudaError_t launch_batch_fwd(const BCase *cases, const BCols *cols, int ncols, i
   return cudaGetLastError();
 }
 
-cudaError_t launch_batch_bwd(const BCase *cases, const BCols *cols, int ncols, size_t smem, int threads,
+cudaError_t launch_batch_bwd(const BCase *cases, const BCols *cols, int ncols, int rk, size_t smem, int threads,
                              cudaStream_t st) {
   if (ncols == 0) return cudaSuccess;
-  k_b_bwd<<<ncols, threads, smem, st>>>(cases, cols);
+  k_b_bwd<<<ncols, threads, smem, st>>>(cases, cols, rk);
   return cudaGetLastError();
 }
 

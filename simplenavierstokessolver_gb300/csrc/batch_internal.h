@@ -20,7 +20,7 @@ constexpr int kPcrLevels = 5; // log2(kSeg)
 struct BCase {
   // ---- static
   int nx, ny, nh;
-  int fft_nst, fft_first2, fcols;  // FFT stage layout, columns per FFT block
+  int fft_nst, fft_first2, fcols;  // FFT stage layout, columns per DFT block (a power of two)
   int with_t, with_force;
   int seg;                         // rows per segment = nx / kSeg
   double dy, rdy;
@@ -39,6 +39,9 @@ struct BCase {
   const double *ccm, *ccp, *cfm, *cfp;  // the advective coefficients above in FP64 (compensated cases)
   const double *dxf, *dxc;         // DXF(i), DXC(i) (diagnostics)
   const double *tw;                // [2*ny]
+  const int *twx;                  // [4*ny] twiddles of the fixed-point DFTs (fft_fixed.cuh)
+  int p2, eoff;                    // 1/DXF is 2^eoff everywhere and 1/dy a power of two; then
+  float ratio_f;                   // (1/dy) / (1/DXF)
   const double *lo, *hi;           // Poisson sub/super diagonals a_i, c_i (mode independent) [nx]
   const double *pfac;              // per mode: inv[nx] up[nx] v[nx] w[nx] alpha[5*32] beta[5*32] rD[32]
   size_t pstride;                  // doubles per mode in pfac
@@ -82,6 +85,10 @@ cudaError_t batch_kernels_init();
 // tiles[ntiles - ntiles_x2 ..] belong to compensated cases
 cudaError_t launch_batch_stencil(const BCase *cases, const BTile *tiles, int ntiles, int ntiles_x2, int rk,
                                  int tile_x, int rows, cudaStream_t st);
+// column DFTs: jtot / 16 threads a column where the block has them (then in
+// fixed point), any number otherwise
+int batch_fft_cols(int ny, int threads);          // columns per block
+size_t batch_fft_smem(int ny, int cols, int threads);
 cudaError_t launch_batch_fwd(const BCase *cases, const BCols *cols, int ncols, int rk, size_t smem, int threads,
                              cudaStream_t st);
 // shared memory of the tridiagonal launch for lines up to nmax long
@@ -91,7 +98,7 @@ size_t batch_tri_smem(int nmax, int modes_per_block);
 // the error path)
 cudaError_t launch_batch_tri(const BCase *cases, const BModes *modes, int nmodes, int modes_per_block, int nmax,
                              unsigned *err, unsigned spin, int stale, cudaStream_t st);
-cudaError_t launch_batch_bwd(const BCase *cases, const BCols *cols, int ncols, size_t smem, int threads,
+cudaError_t launch_batch_bwd(const BCase *cases, const BCols *cols, int ncols, int rk, size_t smem, int threads,
                              cudaStream_t st);
 // the five phases of substage rk in one persistent cooperative launch of
 // `blocks` blocks of 256 threads (batch_substage_blocks: every block resident)

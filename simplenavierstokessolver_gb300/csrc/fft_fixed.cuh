@@ -194,6 +194,31 @@ FX_HD long long quantise(double d, int E) {
   const long long q = (long long)(((m >> (s < 63 ? s : 63)) + 1) >> 1), n = (long long)b >> 63;
   return (q ^ n) - n;
 }
+// the same for a float; E at least its double exponent
+FX_HD long long quantise(float f, int E) {
+  unsigned b;
+#ifdef __CUDA_ARCH__
+  b = __float_as_uint(f);
+#else
+  __builtin_memcpy(&b, &f, 4);
+#endif
+  const int e = (int)(b >> 23) & 0xff;
+  const unsigned long long m = (unsigned long long)(((b & 0x7fffffu) | (e ? 1u << 23 : 0u)) << 4) << 32;  // 60 bits
+  const int s = E - ((e ? e : 1) + 896);
+  const long long q = (long long)(((m >> (s < 63 ? s : 63)) + 1) >> 1), n = (long long)((int)b >> 31);
+  return (q ^ n) - n;
+}
+// 0 for 0, a float's biased exponent as a double, 0x7ff for infinities and NaN
+FX_HD unsigned exponent_key(float f) {
+  unsigned b;
+#ifdef __CUDA_ARCH__
+  b = __float_as_uint(f);
+#else
+  __builtin_memcpy(&b, &f, 4);
+#endif
+  const unsigned e = (b >> 23) & 0xff;
+  return e == 255u ? 0x7ffu : (b & 0x7fffffffu) == 0u ? 0u : (e ? e : 1u) + 896u;
+}
 // a column whose largest exponent is below kTiny is taken times 2^512 (exact)
 FX_HD double lift(double d, bool tiny) { return tiny ? d * 0x1p512 : d; }
 FX_HD int column_scale(unsigned top, bool *tiny, int *eoff) {
@@ -268,7 +293,6 @@ FX_HD void merge(C64 A, C64 B, Tw w, C64 &zk, C64 &zm) {
   zm = C64{er + o.y, o.x - ei};
 }
 
-#ifdef __CUDACC__
 // elements of 16 bytes a column takes: M and its padding, and what brings the
 // stride to 8 / C modulo 8, so that the C columns' lanes fall on different banks
 FX_HD int column_stride(int M, int lgC) {
@@ -276,6 +300,7 @@ FX_HD int column_stride(int M, int lgC) {
   return n + ((want - n) & 7);
 }
 
+#ifdef __CUDACC__
 constexpr int kMaxWarps = 32, kMaxCols = 16;
 // per warp and column: the largest exponent, or the bits of a pass's magnitudes
 struct Slots {
@@ -420,23 +445,47 @@ __device__ __forceinline__ void passes(Place<V> &p, C64 *z, const Tw *tw, int &S
   }
 }
 
+// What forward() reads. load(c, mm, raw): rows 2 mm and 2 mm + 1 of the
+// block's column c into 16 bytes, and a key of 0 or the largest biased exponent
+// that the magnitudes stay below 2^(key - 1022) with (0x7ff: not finite);
+// fixed(raw, E, tiny): the two values times 2^(1081 - E) as integers (times
+// 2^512 before that when tiny). kUnroll: loads in flight per thread.
+template <typename F>
+struct Doubles {
+  F f;  // f(c, mm, d): d[0], d[1]
+  static constexpr int kUnroll = 8;
+  __device__ __forceinline__ unsigned load(int c, int mm, double2 &raw) const {
+    double d[2];
+    f(c, mm, d);
+    raw = make_double2(d[0], d[1]);
+    return max(exponent_key(d[0]), exponent_key(d[1]));
+  }
+  __device__ __forceinline__ C64 fixed(double2 d, int E, bool tiny) const {
+    return C64{quantise(lift(d.x, tiny), E), quantise(lift(d.y, tiny), E)};
+  }
+};
+template <typename F>
+__device__ __forceinline__ Doubles<F> doubles(F f) {
+  return Doubles<F>{f};
+}
+
 // Forward real DFT of a block's columns (M = jtot / 2 complex values each,
-// M >= 8, C M / V threads or more). in(c, mm, d): d[0], d[1] = rows 2 mm and
-// 2 mm + 1 of the block's column c; eoff: the values stand for 2^eoff times
-// themselves. out(c, k, X): 2 X[k] of the unnormalised transform (FFTW's
+// M >= 8, C M / V threads or more) of the values that `in` gives times
+// 2^eoff. out(c, k, X): 2 X[k] of the unnormalised transform (FFTW's
 // conventions), k = 0 .. M. A column with a NaN or an infinity gives NaN.
 template <int V, typename In, typename Out>
 __device__ __forceinline__ void forward(C64 *z, Slots *slots, int lgC, int M, const Tw *tw, int eoff, In in, Out out) {
   Place<V> p(lgC, M, slots);
   unsigned top = 0u;
   if (p.on) {
-    double d[2 * V];
+    constexpr int U = In::kUnroll < V ? In::kUnroll : V;
+#pragma unroll 1
+    for (int r0 = 0; r0 < V; r0 += U) {
+      double2 d[U];
 #pragma unroll
-    for (int r = 0; r < V; ++r) in(p.c, p.j + r * p.nv, d + 2 * r);
+      for (int r = 0; r < U; ++r) top = max(top, in.load(p.c, p.j + (r0 + r) * p.nv, d[r]));
 #pragma unroll
-    for (int r = 0; r < V; ++r) {
-      top = max(top, max(exponent_key(d[2 * r]), exponent_key(d[2 * r + 1])));
-      std2(z, p.at(p.j + r * p.nv), make_double2(d[2 * r], d[2 * r + 1]));
+      for (int r = 0; r < U; ++r) std2(z, p.at(p.j + (r0 + r) * p.nv), d[r]);
     }
   }
   p.template put<true>(top);
@@ -445,10 +494,7 @@ __device__ __forceinline__ void forward(C64 *z, Slots *slots, int lgC, int M, co
   const int E = column_scale(p.template get<true>(), &tiny, &eoff);
   if (p.on) {  // each thread its own elements, which its first butterfly reads
 #pragma unroll 1
-    for (int i = p.j; i < M; i += p.nv) {
-      const double2 d = ldd(z, p.at(i));
-      stz(z, p.at(i), C64{quantise(lift(d.x, tiny), E), quantise(lift(d.y, tiny), E)});
-    }
+    for (int i = p.j; i < M; i += p.nv) stz(z, p.at(i), in.fixed(ldd(z, p.at(i)), E, tiny));
   }
   p.template put<false>(0u);
   __syncthreads();

@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(512, 1) k_par_fwd_fx(const FixArgs a) {
     if (x < nx) a.spec[(size_t)k * nx + par_p(x, a.m)] = X;
   };
   fx::forward<V>(reinterpret_cast<fx::C64 *>(fx_sm), &slots, a.lgC, ny / 2, reinterpret_cast<const fx::Tw *>(a.g.twx),
-              eoff, in, out);
+              eoff, fx::doubles(in), out);
 }
 
 // src/fluid/compute_potential.c:146-157: the inverse into psi

@@ -65,3 +65,33 @@ def test_a_non_finite_column_makes_the_potential_non_finite(value):
     ux, uy = np.zeros((ny + 2, nx + 1)), np.ones((ny + 2, nx + 2))
     uy[10, 20] = value
     assert not np.isfinite(_solve(nx, ny, True, ux, uy, 1e-3)).any()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,stretch", [(64, 8, 1e9), (64, 16, 1e9), (96, 32, 1e9), (64, 64, 3), (64, 2048, 1e9),
+                                           (64, 8192, 1e9)])
+@pytest.mark.parametrize("compensated", [False, True], ids=["fp32", "compensated"])
+def test_batched_steps_match_the_plain_path(nx, ny, stretch, compensated):
+    """the batched form's column groups of 1 to 16, its FP64 stages (jtot 8) and
+    its divergences as pairs and as doubles (grids of no powers of two): three
+    steps of a fixed dt against the exact form from the same start, within the
+    forms' stated errors (1e-5 and 1e-10)"""
+    from simplenavierstokessolver_gb300 import Case
+    from simplenavierstokessolver_gb300.batch import Batch, Desc, initial_temperature
+
+    d = Desc(nx, ny, ly=2.0, stretch=stretch, Ra=1e6, Pr=1.0, seed=3, fixed_dt=1e-4, compensated=compensated)
+    with Batch(1 << 30, max_cases=2) as b:
+        s = b.add(d)
+        b.step(3)
+        got = b.state(s)
+    z = np.zeros((ny + 2, nx + 2))
+    with Case(nx, ny, ly=2.0, stretch=stretch, Ra=1e6, Pr=1.0) as c:
+        c.set_state(np.zeros((ny + 2, nx + 1)), z, z, initial_temperature(d))
+        c.set_dt(1e-4, 0, 0)
+        for _ in range(3):
+            c.integrate()
+        want = c.get_state()
+    for k in ("ux", "uy", "temp"):
+        w = want[k][1:-1, 1:-1]
+        err = np.linalg.norm(got[k][1:-1, 1:-1] - w) / np.linalg.norm(w)
+        assert err < (1e-10 if compensated else 1e-5), (k, err)
