@@ -167,7 +167,7 @@ class Batch:
     def state(self, slot: int):
         d = self.descs[slot]
         su, sc = (d.jtot + 2, d.itot + 1), (d.jtot + 2, d.itot + 2)
-        out = {"ux": np.zeros(su), "uy": np.zeros(sc), "p": np.zeros(sc), "psi": np.zeros(sc), "temp": np.zeros(sc)}
+        out = {"ux": np.empty(su), "uy": np.empty(sc), "p": np.empty(sc), "psi": np.empty(sc), "temp": np.empty(sc)}
         N.check(self.lib.sns_batch_state(self.h, slot, _ptr(out["ux"]), _ptr(out["uy"]), _ptr(out["p"]),
                                          _ptr(out["psi"]), _ptr(out["temp"])), "sns_batch_state")
         return out
@@ -191,7 +191,7 @@ def diagnostics_of(batch_handle, slot: int) -> np.ndarray:
 
 def state_of(batch_handle, slot: int, desc: Desc):
     su, sc = (desc.jtot + 2, desc.itot + 1), (desc.jtot + 2, desc.itot + 2)
-    out = {"ux": np.zeros(su), "uy": np.zeros(sc), "p": np.zeros(sc), "psi": np.zeros(sc), "temp": np.zeros(sc)}
+    out = {"ux": np.empty(su), "uy": np.empty(sc), "p": np.empty(sc), "psi": np.empty(sc), "temp": np.empty(sc)}
     N.check(_lib().sns_batch_state(batch_handle, slot, _ptr(out["ux"]), _ptr(out["uy"]), _ptr(out["p"]),
                                    _ptr(out["psi"]), _ptr(out["temp"])), "sns_batch_state")
     return out

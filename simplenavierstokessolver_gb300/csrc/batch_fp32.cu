@@ -920,7 +920,19 @@ __global__ void k_b_dt(BCase *cases, int ncases, RkCoefs rk) {
   }
 }
 
+// compensated pairs to doubles
+__global__ void __launch_bounds__(256) k_b_widen(const float *__restrict__ hi, const float *__restrict__ lo,
+                                                 double *__restrict__ out, size_t n) {
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
+    out[k] = (double)hi[k] + (double)lo[k];
+}
+
 }  // namespace
+
+cudaError_t launch_batch_widen(const float *hi, const float *lo, double *out, size_t n, cudaStream_t st) {
+  k_b_widen<<<(int)std::min<size_t>((n + 255) / 256, 152 * 8), 256, 0, st>>>(hi, lo, out, n);
+  return cudaGetLastError();
+}
 
 // kernel attributes, set once outside any stream capture
 cudaError_t batch_kernels_init() {

@@ -110,6 +110,8 @@ cudaError_t launch_batch_substage(BCase *cases, const BTile *tiles, int ntiles, 
                                   cudaStream_t st);
 cudaError_t launch_batch_corr(const BCase *cases, const BTile *tiles, int ntiles, int rk, int tile_x, int rows,
                               cudaStream_t st);
+// out = hi + lo, exact in FP64
+cudaError_t launch_batch_widen(const float *hi, const float *lo, double *out, size_t n, cudaStream_t st);
 cudaError_t launch_batch_dt(BCase *cases, int ncases, const double *rk_a, const double *rk_b, cudaStream_t st);
 
 void count_launches(long long n);

@@ -153,7 +153,7 @@ inline bool invariant_divisor(double y, double *zh_out, double *zl_out) {
 }
 
 // exp(-2 pi i t / n), t < n (a power of two), scaled by 2^62 and split for the
-// fixed-point DFT (fft_fixed.cuh, Tw): four words per t, real high and low,
+// fixed-point DFT (fft_fixed.cuh, Tw; n >= 8): four words per t, real high and low,
 // imaginary high and low, the low ones in (-2^31, 2^31). Sine and cosine of an
 // angle in [0, pi/4] by their Taylor series in 112-bit fixed point, so the
 // words are the same on every host.
@@ -185,16 +185,20 @@ inline std::vector<int32_t> fixed_twiddles(int n) {
     *s = ss;
     *c = cc;
   };
+  // one octant: angles (pi/2) r / n, r = 4 t' <= n / 2 (r = 0, n / 2 alone below n = 8)
+  const int noct = n / 8 + 1;
+  std::vector<int64_t> so(noct), co(noct);
+  for (int k = 0; k < noct; k++) {
+    u128 s, c;
+    sincos(8 * k, &s, &c);
+    so[k] = (int64_t)((s + ((u128)1 << 49)) >> 50);
+    co[k] = (int64_t)((c + ((u128)1 << 49)) >> 50);
+  }
   std::vector<int32_t> out(4 * (size_t)n);
   for (int t = 0; t < n; t++) {
     const long q = 4L * t / n, r = 4L * t - q * n;  // quadrant and (pi/2) r / n inside it
-    u128 s, c;
-    if (2 * r <= n) {
-      sincos((int)(2 * r), &s, &c);
-    } else {
-      sincos((int)(2 * (n - r)), &c, &s);
-    }
-    const int64_t si = (int64_t)((s + ((u128)1 << 49)) >> 50), ci = (int64_t)((c + ((u128)1 << 49)) >> 50);
+    const bool low = 2 * r <= n;
+    const int64_t si = low ? so[r / 4] : co[(n - r) / 4], ci = low ? co[r / 4] : so[(n - r) / 4];
     int64_t re = 0, im = 0;
     switch (q & 3) {
       case 0: re = ci; im = -si; break;
