@@ -24,6 +24,7 @@
 #include "diag_internal.h"
 #include "host_common.h"
 #include "npy.h"
+#include "setup_internal.h"
 #include "sns_batch.h"
 #include "sns_gpu.h"
 
@@ -55,6 +56,7 @@ struct CaseLayout {
   size_t rdxf_f, rdxc_f, ccm_f, ccp_f, cfm_f, cfp_f, rdxf_l;
   size_t rdxf, rdxc, dxi, dxf, dxc, tw, twx, lo, hi, pfac, ccm, ccp, cfm, cfp;
   size_t ux[2], uy[2], t[2], uxl[2], uyl[2], tl[2], aux, auy, at, auxl, auyl, atl, p, psi, spec;
+  size_t small;  // bytes of the host-computed arrays at the head
   size_t total;
   size_t pstride;
 };
@@ -71,6 +73,7 @@ static CaseLayout layout_for(int nx, int ny, bool x2) {
     return o;
   };
   const size_t cells = (size_t)nx * ny;
+  // what the host computes, in one block and one upload
   L.rdxf_f = take(sizeof(float) * nx);
   L.rdxf_l = take(sizeof(float) * nx);
   L.rdxc_f = take(sizeof(float) * (nx + 1));
@@ -87,12 +90,13 @@ static CaseLayout layout_for(int nx, int ny, bool x2) {
   L.twx = take(sizeof(int32_t) * 4 * ny);
   L.lo = take(sizeof(double) * nx);
   L.hi = take(sizeof(double) * nx);
-  L.pstride = 4 * (size_t)nx + 2 * kPcrLevels * kSeg + kSeg;
-  L.pfac = take(sizeof(double) * L.pstride * nh);
   L.ccm = take(sizeof(double) * nx);
   L.ccp = take(sizeof(double) * nx);
   L.cfm = take(sizeof(double) * nx);
   L.cfp = take(sizeof(double) * nx);
+  L.small = off;
+  L.pstride = 4 * (size_t)nx + 2 * kPcrLevels * kSeg + kSeg;
+  L.pfac = take(sizeof(double) * L.pstride * nh);
   for (int k = 0; k < 2; k++) {
     L.ux[k] = take(sizeof(float) * cells);
     L.uy[k] = take(sizeof(float) * cells);
@@ -514,27 +518,30 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
     rdxc_f[i - 1] = (float)rdxc[i - 1];
     dxi[i - 1] = 1. / DXC(i);
   }
-  std::vector<double> pfac(L.pstride * nh);
-  for (int J = 0; J < nh; J++)
-    partition_factors(nx, lo.data(), hi.data(), l_raw.data(), u_raw.data(), poisson_eigenvalue(dy, ny, J), J == 0,
-                      false, pfac.data() + L.pstride * J);
   const std::vector<double> tw = twiddle_table(ny);
   const std::vector<int32_t> twx = fixed_twiddles(ny);
-  std::vector<double> temp((size_t)(nx + 2) * (ny + 2));
-  if (st) temp_init = st->temp;
-  if (temp_init) {
-    std::memcpy(temp.data(), temp_init, sizeof(double) * temp.size());
-  } else {
-    initial_temperature(d, xc.data(), temp.data());
-  }
-  std::vector<float> t_dense((size_t)nx * ny), t_low((size_t)nx * ny);
-  for (int j = 1; j <= ny; j++)
-    for (int i = 1; i <= nx; i++) {
-      const double v = temp[(size_t)j * (nx + 2) + i];
-      const float hi = (float)v;
-      t_dense[(size_t)(j - 1) * nx + (i - 1)] = hi;
-      t_low[(size_t)(j - 1) * nx + (i - 1)] = (float)(v - (double)hi);
-    }
+  std::vector<char> small(L.small, 0);
+  auto keep = [&](size_t o, const void *src, size_t bytes) { std::memcpy(small.data() + o, src, bytes); };
+  keep(L.rdxf_f, rdxf_f.data(), sizeof(float) * nx);
+  keep(L.rdxf_l, rdxf_l.data(), sizeof(float) * nx);
+  keep(L.rdxc_f, rdxc_f.data(), sizeof(float) * (nx + 1));
+  keep(L.ccm_f, ccm.data(), sizeof(float) * nx);
+  keep(L.ccp_f, ccp.data(), sizeof(float) * nx);
+  keep(L.cfm_f, cfm.data(), sizeof(float) * nx);
+  keep(L.cfp_f, cfp.data(), sizeof(float) * nx);
+  keep(L.rdxf, rdxf.data(), sizeof(double) * nx);
+  keep(L.rdxc, rdxc.data(), sizeof(double) * (nx + 1));
+  keep(L.dxi, dxi.data(), sizeof(double) * (nx + 1));
+  keep(L.dxf, dxf.data(), sizeof(double) * nx);
+  keep(L.dxc, dxc.data(), sizeof(double) * (nx + 1));
+  keep(L.tw, tw.data(), sizeof(double) * tw.size());
+  keep(L.twx, twx.data(), sizeof(int32_t) * twx.size());
+  keep(L.lo, lo.data(), sizeof(double) * nx);
+  keep(L.hi, hi.data(), sizeof(double) * nx);
+  keep(L.ccm, ccm_d.data(), sizeof(double) * nx);
+  keep(L.ccp, ccp_d.data(), sizeof(double) * nx);
+  keep(L.cfm, cfm_d.data(), sizeof(double) * nx);
+  keep(L.cfp, cfp_d.data(), sizeof(double) * nx);
   auto put = [&](size_t o, const void *src, size_t bytes) {
     return cudaMemcpyAsync(base + o, src, bytes, cudaMemcpyHostToDevice, b->stream);
   };
@@ -543,31 +550,37 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
   auto chk = [&](cudaError_t x) {
     if (e == cudaSuccess) e = x;
   };
-  chk(put(L.rdxf_f, rdxf_f.data(), sizeof(float) * nx));
-  chk(put(L.rdxf_l, rdxf_l.data(), sizeof(float) * nx));
-  chk(put(L.rdxc_f, rdxc_f.data(), sizeof(float) * (nx + 1)));
-  chk(put(L.ccm_f, ccm.data(), sizeof(float) * nx));
-  chk(put(L.ccp_f, ccp.data(), sizeof(float) * nx));
-  chk(put(L.cfm_f, cfm.data(), sizeof(float) * nx));
-  chk(put(L.cfp_f, cfp.data(), sizeof(float) * nx));
-  chk(put(L.rdxf, rdxf.data(), sizeof(double) * nx));
-  chk(put(L.rdxc, rdxc.data(), sizeof(double) * (nx + 1)));
-  chk(put(L.dxi, dxi.data(), sizeof(double) * (nx + 1)));
-  chk(put(L.dxf, dxf.data(), sizeof(double) * nx));
-  chk(put(L.dxc, dxc.data(), sizeof(double) * (nx + 1)));
-  chk(put(L.tw, tw.data(), sizeof(double) * tw.size()));
-  chk(put(L.twx, twx.data(), sizeof(int32_t) * twx.size()));
-  chk(put(L.lo, lo.data(), sizeof(double) * nx));
-  chk(put(L.hi, hi.data(), sizeof(double) * nx));
-  chk(put(L.pfac, pfac.data(), sizeof(double) * pfac.size()));
-  chk(put(L.ccm, ccm_d.data(), sizeof(double) * nx));
-  chk(put(L.ccp, ccp_d.data(), sizeof(double) * nx));
-  chk(put(L.cfm, cfm_d.data(), sizeof(double) * nx));
-  chk(put(L.cfp, cfp_d.data(), sizeof(double) * nx));
-  for (int k = 0; k < 2; k++) {
-    chk(cudaMemsetAsync(base + L.ux[k], 0, sizeof(float) * cells, b->stream));
-    chk(cudaMemsetAsync(base + L.uy[k], 0, sizeof(float) * cells, b->stream));
+  chk(put(0, small.data(), L.small));
+  chk(cudaMemsetAsync(base + L.ux[0], 0, L.total - L.ux[0], b->stream));  // every field
+  // the modes' eigenvalues and the centres through the spectrum's memory (the
+  // first step writes it before it reads it)
+  std::vector<double> scratch(nh + nx);
+  for (int J = 0; J < nh; J++) scratch[J] = poisson_eigenvalue(dy, ny, J);
+  std::copy(xc.begin() + 1, xc.begin() + 1 + nx, scratch.begin() + nh);
+  chk(put(L.spec, scratch.data(), sizeof(double) * scratch.size()));
+  double *dscratch = reinterpret_cast<double *>(base + L.spec);
+  chk(launch_partition_factors(PoissonLines{nx, nh, reinterpret_cast<const double *>(base + L.lo),
+                                            reinterpret_cast<const double *>(base + L.hi), dscratch, l_raw[0],
+                                            u_raw[nx - 1], reinterpret_cast<double *>(base + L.pfac), L.pstride, false,
+                                            false},
+                               b->stream));
+  count_launches(1);
+  float *t_hi = reinterpret_cast<float *>(base + L.t[0]), *t_lo = reinterpret_cast<float *>(base + L.tl[0]);
+  std::vector<double> temp;
+  if (st) temp_init = st->temp;
+  if (!temp_init && d->seed != 0) {
+    chk(launch_seeded_temperature(nx, ny, d->seed, dscratch + nh, TEMP_XM, TEMP_XP, t_hi, t_lo, b->stream));
+  } else {
+    if (!temp_init) {  // the reference's own noise
+      temp.resize((size_t)(nx + 2) * (ny + 2));
+      initial_temperature(d, xc.data(), temp.data());
+      temp_init = temp.data();
+    }
+    chk(cudaMemcpy2DAsync(dscratch, sizeof(double) * nx, temp_init + (nx + 2) + 1, sizeof(double) * (nx + 2),
+                          sizeof(double) * nx, ny, cudaMemcpyHostToDevice, b->stream));
+    chk(launch_split(cells, dscratch, t_hi, t_lo, b->stream));
   }
+  count_launches(1);
   // restart: velocity as compensated pairs, pressure as is; and the first dt
   // from its maximum exactly as the correction kernel and k_b_dt form it
   std::vector<float> ux_h, ux_l, uy_h, uy_l;
@@ -599,24 +612,7 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
     chk(put(L.uy[0], uy_h.data(), sizeof(float) * cells));
     chk(put(L.uyl[0], uy_l.data(), sizeof(float) * cells));
   }
-  chk(put(L.t[0], t_dense.data(), sizeof(float) * cells));
-  chk(put(L.tl[0], t_low.data(), sizeof(float) * cells));
-  chk(cudaMemsetAsync(base + L.tl[1], 0, sizeof(float) * cells, b->stream));
-  for (int k = st ? 1 : 0; k < 2; k++) {
-    chk(cudaMemsetAsync(base + L.uxl[k], 0, sizeof(float) * cells, b->stream));
-    chk(cudaMemsetAsync(base + L.uyl[k], 0, sizeof(float) * cells, b->stream));
-  }
-  chk(cudaMemsetAsync(base + L.t[1], 0, sizeof(float) * cells, b->stream));
-  for (size_t o : {L.aux, L.auy, L.at}) chk(cudaMemsetAsync(base + o, 0, sizeof(float) * cells, b->stream));
-  if (x2)
-    for (size_t o : {L.auxl, L.auyl, L.atl}) chk(cudaMemsetAsync(base + o, 0, sizeof(float) * cells, b->stream));
-  if (st) {
-    chk(put(L.p, p_d.data(), sizeof(double) * cells));
-  } else {
-    chk(cudaMemsetAsync(base + L.p, 0, sizeof(double) * cells, b->stream));
-  }
-  chk(cudaMemsetAsync(base + L.psi, 0, sizeof(double) * cells, b->stream));
-  chk(cudaMemsetAsync(base + L.spec, 0, sizeof(double2) * (size_t)nh * nx, b->stream));
+  if (st) chk(put(L.p, p_d.data(), sizeof(double) * cells));
   // ---- table entry
   BCase t;
   std::memset(&t, 0, sizeof t);
@@ -796,6 +792,8 @@ int sns_batch_remove(sns_batch *b, int slot) {
 
 int sns_batch_step(sns_batch *b, int nsteps) {
   if (!b || nsteps < 0) return bfail(SNS_ERR_ARG, "sns_batch_step: bad argument");
+  constexpr int kRebuildSteps = 16;
+  bool drop = false;
   std::lock_guard<std::mutex> lk(b->mu);
   for (int s = 0; s < nsteps; s++) {
     if (b->dirty)
@@ -813,8 +811,15 @@ int sns_batch_step(sns_batch *b, int nsteps) {
       h.steps_done++;
       if (h.d.steps > 0 && h.steps_done >= h.d.steps) finished_one = true;
     }
-    if (finished_one) b->dirty = true;  // drop finished cases from the work lists
+    // drop finished cases from the work lists; their blocks only look at the
+    // done flag, which for a few steps costs less than a new graph (about a step)
+    drop |= finished_one;
+    if (drop && nsteps - s > kRebuildSteps) {
+      b->dirty = true;
+      drop = false;
+    }
   }
+  if (drop) b->dirty = true;
   return SNS_OK;
 }
 

@@ -236,7 +236,7 @@ inline double poisson_eigenvalue(double dy, int jtot, int J) {
 constexpr int kPartSeg = 32;
 constexpr int kPartLevels = 5;  // log2(kPartSeg)
 
-// doubles per line of the factor block written by partition_factors
+// doubles per line of the factor block written by partition_factors_tri
 inline size_t partition_stride(int n) { return 4 * (size_t)n + 2 * kPartLevels * kPartSeg + kPartSeg; }
 
 // Factors of one line of n rows with sub-diagonal a_i, diagonal d_i and
@@ -331,18 +331,6 @@ inline void partition_factors_tri(int n, const double *a_in, const double *d, co
     out[2 * (size_t)n + o] = v[i];
     out[3 * (size_t)n + o] = w[i];
   }
-}
-
-// The Poisson lines: diagonal d_i = -l_raw_i - u_raw_i + eig with the
-// Neumann closure (src/fluid/compute_potential.c:116-127: the first and last
-// diagonal entries absorb l_raw_0 and u_raw_{n-1}), a_0 = c_{n-1} = 0.
-inline void partition_factors(int n, const double *a, const double *c, const double *l_raw, const double *u_raw,
-                              double eig, bool pin_last, bool interleave, double *out) {
-  std::vector<double> d(n);
-  for (int i = 0; i < n; i++) d[i] = -l_raw[i] - u_raw[i] + eig;
-  d[0] += l_raw[0];
-  d[n - 1] += u_raw[n - 1];
-  partition_factors_tri(n, a, d.data(), c, false, pin_last, interleave, out);
 }
 
 // stage layout of the length-jtot/2 complex FFT: radix 2 first when

@@ -24,6 +24,7 @@
 #include "diag_internal.h"
 #include "host_common.h"
 #include "npy.h"
+#include "setup_internal.h"
 #include "sns_batch.h"
 #include "sns_gpu.h"
 #include "sns_internal.h"
@@ -1158,23 +1159,23 @@ static int parallel_prepare(Context *c) {
   // elimination's dependent chain
   const size_t base = partition_stride(nx), stride = base + nx;
   const int m = nx / kPartSeg;
-  std::vector<double> fac(stride * nh), blk(base), lo(nx), hi(nx);
+  std::vector<double> lo(nx), hi(nx), eig(nh);
   for (int x = 0; x < nx; x++) {
     lo[(size_t)(x % m) * kPartSeg + x / m] = a[x];
     hi[(size_t)(x % m) * kPartSeg + x / m] = cc[x];
   }
-  for (int J = 0; J < nh; J++) {
-    partition_factors(nx, a.data(), cc.data(), l_raw.data(), u_raw.data(), poisson_eigenvalue(c->g.dy, ny, J),
-                      J == 0, true, blk.data());
-    double *o = fac.data() + stride * J;
-    std::copy(blk.begin(), blk.begin() + nx, o);                         // inv
-    for (int i = 0; i < nx; i++) o[nx + i] = lo[i] * blk[i];            // g
-    std::copy(blk.begin() + nx, blk.end(), o + 2 * (size_t)nx);         // up v w alpha beta rD
-  }
+  for (int J = 0; J < nh; J++) eig[J] = poisson_eigenvalue(c->g.dy, ny, J);
   int rc = SNS_OK;
-  if ((rc = upload(c, &c->g.twx, fixed_twiddles(ny)))) return rc;
-  if ((rc = upload(c, &c->par.fac, fac)) || (rc = upload(c, &c->par.lo, lo)) || (rc = upload(c, &c->par.hi, hi)))
+  double *fac = nullptr;
+  const double *deig = nullptr;
+  if ((rc = upload(c, &c->g.twx, fixed_twiddles(ny))) || (rc = upload(c, &c->par.lo, lo)) ||
+      (rc = upload(c, &c->par.hi, hi)) || (rc = upload(c, &deig, eig)) || (rc = dev_alloc(c, &fac, stride * nh)))
     return rc;
+  SNS_CUDA(launch_partition_factors(PoissonLines{nx, nh, c->par.lo, c->par.hi, deig, l_raw[0], u_raw[nx - 1], fac,
+                                                 stride, true, true},
+                                    c->stream));
+  count_launches(1);
+  c->par.fac = fac;
   if ((rc = dev_alloc(c, &c->par.err, (size_t)1))) return rc;
   SNS_CUDA(cudaMemset(c->par.err, 0, sizeof(unsigned)));
   if (!c->par_err_host) SNS_CUDA(counted_malloc_host(&c->par_err_host, sizeof(unsigned)));

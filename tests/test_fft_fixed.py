@@ -95,3 +95,19 @@ def test_batched_steps_match_the_plain_path(nx, ny, stretch, compensated):
         w = want[k][1:-1, 1:-1]
         err = np.linalg.norm(got[k][1:-1, 1:-1] - w) / np.linalg.norm(w)
         assert err < (1e-10 if compensated else 1e-5), (k, err)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,ny,stretch", [(64, 8, 1e9), (96, 32, 3), (256, 128, 1e9)])
+@pytest.mark.parametrize("given", [False, True], ids=["seeded", "given"])
+def test_admitted_temperature_is_the_hosts(nx, ny, stretch, given):
+    """the device's seeded (or split) initial field against the host's, as the
+    pair of floats that holds it"""
+    from simplenavierstokessolver_gb300.batch import Batch, Desc, initial_temperature
+
+    d = Desc(nx, ny, ly=2.0, stretch=stretch, Ra=1e6, Pr=1.0, seed=11)
+    t = initial_temperature(d)
+    with Batch(256 << 20, max_cases=2) as b:
+        got = b.state(b.add(d, t if given else None))["temp"]
+    hi = t.astype(np.float32)
+    assert np.array_equal(got, hi.astype(np.float64) + (t - hi).astype(np.float32))
