@@ -7,9 +7,12 @@
 //  * FP64-throughput kernels (stencils, FFTs): FP64 instructions per cell at
 //    one warp instruction per kFp64CyclesPerWarpInst cycles per SM, at
 //    kStencilEfficiency of that rate;
-//  * serial line recurrences (Thomas sweeps): cycles per element of one line
-//    times the line length, or the FP64 throughput bound when the lines
-//    outnumber the SM sub-partitions;
+//  * serial line recurrences (the Poisson modes' Thomas sweeps): cycles per
+//    element of one line times the line length, or the FP64 throughput bound
+//    when the lines outnumber the SM sub-partitions;
+//  * Crank-Nicolson solves (segments swept side by side): FP64 instructions
+//    per cell, warm-up rows included, at kSweepEfficiency, their traffic, and
+//    kSweepSeconds for the factors' computation and upload and the launch;
 //  * memory-bound kernels: bytes over kHbmBytesPerSecond;
 //  * kLaunchSeconds per launch.
 // The same grid and device always give the same costs, hence the same
@@ -28,9 +31,10 @@ constexpr double kHbmBytesPerSecond = 6.0e12;
 constexpr double kLaunchSeconds = 2.5e-6;
 // cycles per element of one serial sweep (forward + backward), measured
 constexpr double kCyclesPoissonLine = 530.0;
-constexpr double kCyclesSolveX = 540.0;
-constexpr double kCyclesSolveY = 700.0;  // periodic: second pass over the line
 constexpr double kOpsPerLineElement = 6.0;
+constexpr double kOpsSolveX = 5.5, kOpsSolveY = 10.0;  // y: the closure's pass over the line
+constexpr double kSweepEfficiency = 0.6;
+constexpr double kSweepSeconds = 22.0e-6;
 
 // FP64 instructions per real sample of the length-ny real FFT of the Poisson
 // kernels (radix-2 first stage when log2(ny/2) is odd, radix-4 stages with
@@ -66,6 +70,9 @@ void cost_model(int nx, int ny, int sms, double clock_hz, bool with_t, double ou
     return std::max(latency, throughput) + kLaunchSeconds;
   };
   auto memory = [&](double bytes_per_cell) { return bytes_per_cell * cells / kHbmBytesPerSecond + kLaunchSeconds; };
+  auto solve = [&](double ops_per_cell) {
+    return ops_per_cell * cells / 32.0 / (warp_inst_rate * kSweepEfficiency) + memory(40.0) + kSweepSeconds;
+  };
   const int nh = ny / 2 + 1;
   double base = fp64(81.0)                                   // velocity
                 + fp64(fft_ops_per_sample(ny) + 6.0)         // divergence + forward FFT
@@ -77,8 +84,8 @@ void cost_model(int nx, int ny, int sms, double clock_hz, bool with_t, double ou
   for (int iy = 0; iy < 2; iy++)
     for (int ix = 0; ix < 2; ix++) {
       double t = base;
-      if (ix) t += fields * (lines(ny, nx, kCyclesSolveX) + memory(24.0));
-      if (iy) t += fields * (lines(nx, ny, kCyclesSolveY) + memory(24.0));
+      if (ix) t += fields * solve(kOpsSolveX);
+      if (iy) t += fields * solve(kOpsSolveY);
       out[iy][ix] = t;
     }
 }

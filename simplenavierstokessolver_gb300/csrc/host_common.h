@@ -61,6 +61,41 @@ inline void factorize(int n, const double *l, const double *d, const double *u, 
   }
 }
 
+// Rows of a Thomas sweep after which a change of its starting value has shrunk
+// below 2^-80 of it (the last 2^-27 let the roundings of two sweeps meet), in
+// either direction and from any row: a change of the previous value reaches
+// the next one times l_i inv_i (elimination) or up_i (substitution). n where
+// some row does not shrink it.
+constexpr double kForgotten = 0x1p-80;
+inline int warm_rows(int n, const double *l, const double *inv, const double *up) {
+  int worst = 0;
+  for (int dir = 0; dir < 2; dir++) {
+    double prod = 1.0;
+    int first = 1;  // the window first .. i
+    for (int i = 1; i < n; i++) {
+      const int a = dir ? n - 1 - i : i;
+      const double c = std::fabs(dir ? up[a] : l[a] * inv[a]);
+      if (!(c < 1.0)) return n;
+      if (c < kForgotten) {  // forgotten in this row
+        prod = 1.0;
+        first = i + 1;
+        worst = std::max(worst, 1);
+        continue;
+      }
+      prod *= c;
+      while (first < i) {  // the shortest window that still shrinks enough
+        const int b = dir ? n - 1 - first : first;
+        const double shorter = prod / std::fabs(dir ? up[b] : l[b] * inv[b]);
+        if (!(shorter < kForgotten)) break;
+        prod = shorter;
+        first++;
+      }
+      worst = std::max(worst, i - first + 1);
+    }
+  }
+  return worst;
+}
+
 // exp(-2 pi i t/n) with the CPU FFT's rule: exact at multiples of pi/2, libm
 // cos/sin evaluated only on [0, pi/4]
 inline void twiddle(int n, int t, double *re, double *im) {

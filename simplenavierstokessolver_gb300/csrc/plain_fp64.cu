@@ -497,6 +497,16 @@ __global__ void __launch_bounds__(128) k_vel(const VelArgs a, int rows) {
   }
 }
 
+__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 // ------------------------------------------------------- line recurrences
 // The recurrences below read each element once, in order, from memory that
 // only the same thread writes: the next chunk of kLineChunk elements (and
@@ -600,12 +610,8 @@ __device__ __forceinline__ void line_backward(double *q, size_t s, const double 
 //         update_velocity.c:509-516)
 // mode 1: ux rows x = 1..nx-1 of the (itot+1)-system whose rows 0 and itot are
 //         identity rows with zero right-hand side (update_velocity.c:249-253)
-__global__ void __launch_bounds__(32) k_solve_x(int nx, int ny, const SolveXSet set) {
-  const int y = blockIdx.x * blockDim.x + threadIdx.x;
-  if (y >= ny) return;
-  const LineFactors &f = set.f[blockIdx.y];
-  const int mode = set.mode[blockIdx.y];
-  double *row = set.q[blockIdx.y] + (size_t)y * nx;
+// one thread, the whole line
+__device__ __forceinline__ void row_serial(double *row, const LineFactors &f, int mode, int nx) {
   double prev = 0.0;
   if (mode == 0) {
     prev = row[0] / f.d0;
@@ -616,13 +622,14 @@ __global__ void __launch_bounds__(32) k_solve_x(int nx, int ny, const SolveXSet 
   line_backward<kSolveXChunk>(row, 1, f.up, nx - 2, mode == 0 ? 0 : 1, prev);
 }
 
+__global__ void __launch_bounds__(32) k_solve_x(int nx, int ny, const SolveXSet set) {
+  const int y = blockIdx.x * blockDim.x + threadIdx.x;
+  if (y >= ny) return;
+  row_serial(set.q[blockIdx.y] + (size_t)y * nx, set.f[blockIdx.y], set.mode[blockIdx.y], nx);
+}
+
 // src/linalg.c:52-108 applied per column along y (periodic), coalesced across x.
-__global__ void __launch_bounds__(32) k_solve_y(int nx, int ny, const SolveYSet set) {
-  const int x = set.first_col[blockIdx.y] + blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
-  const PeriodicFactors &f = set.f[blockIdx.y];
-  const int n = ny;
-  double *col = set.q[blockIdx.y] + x;
+__device__ __forceinline__ void column_serial(double *col, const PeriodicFactors &f, int nx, int n) {
   const size_t s = (size_t)nx;
   const LineFactors &sub = f.sub;
   double prev = col[0] / sub.d0;
@@ -658,6 +665,186 @@ __global__ void __launch_bounds__(32) k_solve_y(int nx, int ny, const SolveYSet 
       cq[k] = nq[k];
       c1[k] = n1[k];
     }
+  }
+}
+
+__global__ void __launch_bounds__(32) k_solve_y(int nx, int ny, const SolveYSet set) {
+  const int x = set.first_col[blockIdx.y] + blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= nx) return;
+  column_serial(set.q[blockIdx.y] + x, set.f[blockIdx.y], nx, ny);
+}
+
+// The same lines cut into segments that are swept side by side, with the
+// serial sweep's values bit for bit. A sweep forgets where it started: a
+// change of one row's value reaches the next one times l inv or up, well below
+// 1 for the step sizes that Crank-Nicolson runs at, and once two sweeps over
+// the same rows round to the same value they stay the same. So every segment
+// starts `warm` rows early from any value, and is right if its value just
+// before its first row equals the one that the segment before it computed
+// there -- which is checked for every segment, in both directions. A line
+// that fails the check (none did in any run here) is redone serially from its
+// right-hand side, which stays in global memory until the line is accepted.
+//
+// A block holds its lines in shared memory, thread t the segment t / lines of
+// line t mod lines; row e lies at e + e / S, and lines are kept so that 16
+// lanes of a double each fall on different banks. FP64 issue bounds it: 5
+// instructions a row (7 along y) and (1 + warm / S) times as many with the
+// warm-up rows; 4 lines a block, so that the blocks' number does not leave
+// part of the SMs a block short (8 lines: 169 instead of 135 us along x).
+// Three fields of 1024 x 2048 at dt 2.6e-3 (16 warm-up rows of segments of 64):
+// 257 -> 135 us along x and 687 -> 182 along y, 70 and 60% of the FP64 issue.
+struct SegArgs {
+  PeriodicFactors f[3];
+  double *q[3];
+  int first[3];  // x: mode; y: first column
+  int lgC;       // 2^lgC lines per block, at most 4
+  int lgS, nseg; // 2^lgS rows per segment, segments
+  int stride;    // x: doubles between rows of shared memory
+  int warm;
+};
+
+__device__ __forceinline__ bool same_value(double a, double b) {
+  const unsigned long long x = (unsigned long long)__double_as_longlong(a), y = (unsigned long long)__double_as_longlong(b);
+  return x == y || ((x | y) << 1) == 0ull;
+}
+
+constexpr int kSegThreads = 256;
+
+// the whole line in one thread, element stride es (few registers: it is there
+// for lines that fail the check)
+template <bool COLS>
+__device__ __noinline__ void line_again(double *q, size_t es, const PeriodicFactors &pf, int n, int low) {
+  const LineFactors &f = pf.sub;
+  double prev = 0.0;
+  if (low == 0) q[0] = prev = q[0] / f.d0;
+#pragma unroll 1
+  for (int e = 1; e < n; ++e) {
+    prev = is_zero_bits(f.inv[e]) ? 0.0 : f.inv[e] * (q[e * es] - f.l[e] * prev);
+    q[e * es] = prev;
+  }
+#pragma unroll 1
+  for (int e = n - 2; e >= low; --e) {
+    prev = q[e * es] - f.up[e] * prev;
+    q[e * es] = prev;
+  }
+  if constexpr (COLS) {
+    const double last = (q[n * es] - pf.u_last * q[0] - pf.l_last * q[(n - 1) * es]) / pf.den;
+    q[n * es] = last;
+#pragma unroll 1
+    for (int e = 0; e < n; ++e) q[e * es] = q[e * es] + last * pf.q1[e];
+  }
+}
+
+template <bool COLS>
+__global__ void __launch_bounds__(kSegThreads) k_solve_seg(int nx, int ny, const SegArgs a) {
+  extern __shared__ double sm[];
+  __shared__ int bad[8];
+  // selects, not an index into the parameters (which would copy them to the stack)
+  const int fi = blockIdx.y;
+  const PeriodicFactors &pf = fi == 0 ? a.f[0] : fi == 1 ? a.f[1] : a.f[2];
+  const LineFactors f = pf.sub;
+  double *q = fi == 0 ? a.q[0] : fi == 1 ? a.q[1] : a.q[2];
+  const int first = fi == 0 ? a.first[0] : fi == 1 ? a.first[1] : a.first[2];
+  const int C = 1 << a.lgC, S = 1 << a.lgS, W = a.warm, lgS = a.lgS, stride = a.stride;
+  const int n = COLS ? ny - 1 : nx;  // rows of the swept system
+  const int total = COLS ? ny : nx;  // rows of a line
+  const bool skip0 = !COLS && first == 1;  // ux: row 0 is a wall
+  const int line0 = (COLS ? first : 0) + blockIdx.x * C, nlines = COLS ? nx : ny;
+  auto idx = [&](int c, int e) { return COLS ? ((e + (e >> lgS)) << a.lgC) + c : c * stride + e + (e >> lgS); };
+  // the lines' elements, consecutive threads along the contiguous direction
+  auto each = [&](auto &&fn) {
+    if constexpr (COLS) {
+      for (int i = threadIdx.x; i < total << a.lgC; i += blockDim.x) {
+        const int c = i & (C - 1), e = i >> a.lgC;
+        if (line0 + c < nlines) fn(c, e, (size_t)e * nx + (line0 + c));
+      }
+    } else {
+      for (int c = 0; c < C && line0 + c < nlines; ++c)
+        for (int e = threadIdx.x; e < total; e += blockDim.x) fn(c, e, (size_t)(line0 + c) * nx + e);
+    }
+  };
+  if (threadIdx.x < 8) bad[threadIdx.x] = 0;
+  // asynchronously: loads through registers would wait for each other
+  each([&](int c, int e, size_t g) { cp_async8(sm + idx(c, e), q + g); });
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  const int c = threadIdx.x & (C - 1), k = threadIdx.x >> a.lgC;
+  const int s0 = k * S, s1 = min(s0 + S, n);
+  const bool live = k < a.nseg && line0 + c < nlines && s0 < n;
+  auto step = [&](int e, double prev) {
+    const double iv = __ldg(f.inv + e);
+    return is_zero_bits(iv) ? 0.0 : iv * (sm[idx(c, e)] - __ldg(f.l + e) * prev);
+  };
+  auto start = [&]() { return skip0 ? 0.0 : sm[idx(c, 0)] / f.d0; };  // row 0
+  // ---- forward elimination: warm-up, then the segment
+  double before = 0.0;  // the value at row s0 - 1
+  if (live && k > 0) {
+    int e = s0 - W;
+    if (e <= 0) {
+      before = start();
+      e = 1;
+    }
+#pragma unroll 4
+    for (; e < s0; ++e) before = step(e, before);
+  }
+  __syncthreads();
+  if (live) {
+    double v = before;
+    int e = s0;
+    if (k == 0) {
+      v = start();
+      if (!skip0) sm[idx(c, 0)] = v;
+      e = 1;
+    }
+#pragma unroll 4
+    for (; e < s1; ++e) {
+      v = step(e, v);
+      sm[idx(c, e)] = v;
+    }
+  }
+  __syncthreads();
+  if (live && k > 0 && !same_value(before, sm[idx(c, s0 - 1)])) bad[c] = 1;
+  // ---- back substitution
+  double after = 0.0;  // the value at row s1
+  if (live && s1 < n) {
+    int e = min(s1 + W, n - 1);
+    after = sm[idx(c, e)];  // final at row n-1, a guess elsewhere
+#pragma unroll 4
+    for (--e; e >= s1; --e) after = sm[idx(c, e)] - __ldg(f.up + e) * after;
+  }
+  __syncthreads();
+  const int low = skip0 ? 1 : 0;
+  if (live) {
+    double v = after;
+    int e = s1 - 1;
+    if (s1 == n) v = sm[idx(c, e--)];
+#pragma unroll 4
+    for (; e >= max(s0, low); --e) {
+      v = sm[idx(c, e)] - __ldg(f.up + e) * v;
+      sm[idx(c, e)] = v;
+    }
+  }
+  __syncthreads();
+  if (live && s1 < n && !same_value(after, sm[idx(c, s1)])) bad[c] = 1;
+  __syncthreads();
+  // ---- back to global memory (along y with the closure, src/linalg.c:95-107)
+  if constexpr (COLS) {
+    __shared__ double last[8];
+    if (threadIdx.x < C && line0 + (int)threadIdx.x < nlines) {
+      const int t = threadIdx.x;
+      last[t] = (sm[idx(t, n)] - pf.u_last * sm[idx(t, 0)] - pf.l_last * sm[idx(t, n - 1)]) / pf.den;
+    }
+    __syncthreads();
+    each([&](int cc, int e, size_t g) {
+      if (!bad[cc]) q[g] = e == n ? last[cc] : sm[idx(cc, e)] + last[cc] * __ldg(pf.q1 + e);
+    });
+    if (k == 0 && line0 + c < nlines && bad[c]) line_again<true>(q + line0 + c, (size_t)nx, pf, n, 0);
+  } else {
+    each([&](int cc, int e, size_t g) {
+      if (!bad[cc] && e >= low) q[g] = sm[idx(cc, e)];
+    });
+    if (k == 0 && line0 + c < nlines && bad[c]) line_again<false>(q + (size_t)(line0 + c) * nx, 1, pf, n, low);
   }
 }
 
@@ -748,16 +935,6 @@ struct TriRing {
   double v[kTriDepth][kTriStage][32];
   double f[kTriDepth][kTriStage][32];
 };
-
-__device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // stage elements x = x0 + dir*k (k < kTriStage) lying in [lo, hi]; always
 // commits one group so that the group count stays regular
@@ -1488,16 +1665,81 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
   return cudaGetLastError();
 }
 
+// Segments for nl lines of n rows (total with the closure's row), or false
+// where the serial sweep is the better one: a sweep that remembers more than
+// a quarter of its line, or lines too long for shared memory. The segment
+// length: the least of the FP64 issue of all rows, warm-up included, and one
+// thread's chain (in FP64 instructions of a sub-partition).
+static bool seg_shape(bool cols, int n, int total, int nl, int warm, SegArgs &a, size_t *smem, int *threads) {
+  a.warm = warm + 1;
+  if (n < 32 || a.warm > n / 4) return false;
+  double best = 1e300;
+  for (int lg = 4; lg <= 12; lg++) {
+    const double S = 1 << lg, issue = (double)nl * n / 32.0 / kMarchWarps * 2.0 * (1.0 + a.warm / S), chain = S + a.warm;
+    if ((32 << lg) >= n && issue + chain < best) {
+      best = issue + chain;
+      a.lgS = lg;
+    }
+  }
+  a.nseg = (n + (1 << a.lgS) - 1) >> a.lgS;
+  const int rows = total + (total >> a.lgS) + 1;
+  a.lgC = 2;
+  if (!cols)
+    while (a.lgC > 0 && sizeof(double) * (size_t)(rows << a.lgC) > 72 * 1024) a.lgC--;
+  // x: 16 / lines doubles modulo 16 between the lines
+  a.stride = rows + (((16 >> a.lgC) - rows) % 16 + 16) % 16;
+  const size_t line = sizeof(double) * (size_t)(cols ? rows : a.stride);
+  *smem = line << a.lgC;
+  *threads = ((a.nseg << a.lgC) + 31) / 32 * 32;
+  return *smem <= 200 * 1024 && *threads <= kSegThreads;
+}
+
 cudaError_t launch_solve_x_set(const DevGrid &g, const SolveXSet &set, cudaStream_t st) {
   if (set.n < 1 || set.n > 3) return cudaErrorInvalidValue;
-  k_solve_x<<<dim3((g.ny + 31) / 32, set.n), 32, 0, st>>>(g.nx, g.ny, set);
+  SegArgs a{};
+  int warm = 0, threads = 0;
+  size_t smem = 0;
+  for (int k = 0; k < set.n; ++k) {
+    a.f[k].sub = set.f[k];
+    a.q[k] = set.q[k];
+    a.first[k] = set.mode[k];
+    warm = std::max(warm, set.f[k].warm);
+  }
+  if (seg_shape(false, g.nx, g.nx, g.ny * set.n, warm, a, &smem, &threads)) {
+    static bool attr = false;
+    if (!attr) {
+      cudaFuncSetAttribute(k_solve_seg<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      attr = true;
+    }
+    k_solve_seg<false><<<dim3((g.ny + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st>>>(g.nx, g.ny, a);
+  } else {
+    k_solve_x<<<dim3((g.ny + 31) / 32, set.n), 32, 0, st>>>(g.nx, g.ny, set);
+  }
   count_launches(1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_solve_y_set(const DevGrid &g, const SolveYSet &set, cudaStream_t st) {
   if (set.n < 1 || set.n > 3) return cudaErrorInvalidValue;
-  k_solve_y<<<dim3((g.nx + 31) / 32, set.n), 32, 0, st>>>(g.nx, g.ny, set);
+  SegArgs a{};
+  int warm = 0, threads = 0;
+  size_t smem = 0;
+  for (int k = 0; k < set.n; ++k) {
+    a.f[k] = set.f[k];
+    a.q[k] = set.q[k];
+    a.first[k] = set.first_col[k];
+    warm = std::max(warm, set.f[k].sub.warm);
+  }
+  if (seg_shape(true, g.ny - 1, g.ny, g.nx * set.n, warm, a, &smem, &threads)) {
+    static bool attr = false;
+    if (!attr) {
+      cudaFuncSetAttribute(k_solve_seg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      attr = true;
+    }
+    k_solve_seg<true><<<dim3((g.nx + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st>>>(g.nx, g.ny, a);
+  } else {
+    k_solve_y<<<dim3((g.nx + 31) / 32, set.n), 32, 0, st>>>(g.nx, g.ny, set);
+  }
   count_launches(1);
   return cudaGetLastError();
 }

@@ -729,6 +729,7 @@ static int push_factors(Context *c, const HostFactors &hf, size_t off, LineFacto
   lf.inv = c->fac + off + n;
   lf.up = c->fac + off + 2 * n;
   lf.d0 = hf.d0;
+  lf.warm = warm_rows((int)n, hf.l.data(), hf.inv.data(), hf.up.data());
   return SNS_OK;
 }
 

@@ -61,6 +61,7 @@ struct LineFactors {
                         //     row 0 unused (first row divides by d0)
   const double *up;     // [n] normalised upper diagonal
   double d0;            // first pivot
+  int warm;             // rows after which a sweep has forgotten its start (warm_rows)
 };
 
 // Periodic y system (src/linalg.c:52-108): Thomas factors of the (n-1)
