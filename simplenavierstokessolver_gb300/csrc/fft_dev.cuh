@@ -9,6 +9,20 @@
 namespace sns {
 namespace fft {
 
+// the threads that work on one group of columns: the whole block, or (Part) a
+// part of it that meets at a named barrier of its own
+struct Block {
+  __device__ __forceinline__ int tid() const { return threadIdx.x; }
+  __device__ __forceinline__ int size() const { return blockDim.x; }
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+struct Part {
+  int t, n, bar;
+  __device__ __forceinline__ int tid() const { return t; }
+  __device__ __forceinline__ int size() const { return n; }
+  __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(n) : "memory"); }
+};
+
 // slot of element idx before the in-place decimation-in-time stages: digit
 // reversal over the stage radices (2 first when log2(M) is odd, then 4s)
 __device__ __forceinline__ int fft_slot(int idx, int M, int nst, int first2) {
@@ -29,14 +43,14 @@ __device__ __forceinline__ int fft_slot(int idx, int M, int nst, int first2) {
 
 // One in-place DIT stage on `cols` columns of length M held in shared memory;
 // the same floating-point operations as dit_stage() of the CPU FFT.
-template <bool FWD>
+template <bool FWD, typename Team = Block>
 __device__ __forceinline__ void fft_stages(double2 *z, int cols, int M, int N, int nst, int first2,
-                                           const double2 *tw) {
+                                           const double2 *tw, const Team team = Team()) {
   int L = 1, lg = 0;
   for (int st = 0; st < nst; ++st) {
     const int R = (st == 0 && first2) ? 2 : 4;
     const int span = R * L, tstep = N / span, nb = M / R;
-    for (int b = threadIdx.x; b < cols * nb; b += blockDim.x) {
+    for (int b = team.tid(); b < cols * nb; b += team.size()) {
       const int c = b / nb, bb = b - c * nb;
       const int k = bb & (L - 1);
       const int base = c * M + (bb >> lg) * span + k;
@@ -81,7 +95,7 @@ __device__ __forceinline__ void fft_stages(double2 *z, int cols, int M, int N, i
         z[base + 3 * L] = make_double2(t1r - sr, t1i - si);
       }
     }
-    __syncthreads();
+    team.sync();
     L *= R;
     lg += (R == 2) ? 1 : 2;
   }

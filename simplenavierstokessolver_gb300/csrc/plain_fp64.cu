@@ -873,13 +873,13 @@ using fft::fft_stages;
 // src/fluid/compute_potential.c:69-92: right-hand side (div u*)/(gamma dt)
 // and its real DFT along y (forward, FFTW conventions).
 // columns x0 .. x0+cols-1 by the whole block, z: cols * ny/2 complex in shared memory
-template <bool RCP>
-__device__ __forceinline__ void poisson_fwd_cols(const PoissonArgs &a, int x0, double2 *z) {
+template <bool RCP, typename Team>
+__device__ __forceinline__ void poisson_fwd_cols(const PoissonArgs &a, int x0, double2 *z, const Team team) {
   const int nx = a.g.nx, ny = a.g.ny, M = ny / 2, C = a.cols;
   double *zd = reinterpret_cast<double *>(z);
   const double dy = a.g.dy, rdy = a.g.rdy;
   const Spacing sy = spacing_y<RCP, true>(dy, rdy, a.g.rdyl);
-  for (int e = threadIdx.x; e < C * ny; e += blockDim.x) {
+  for (int e = team.tid(); e < C * ny; e += team.size()) {
     const int c = e % C, y = e / C, x = x0 + c;
     double d = 0.0;
     if (x < nx) {
@@ -900,11 +900,11 @@ __device__ __forceinline__ void poisson_fwd_cols(const PoissonArgs &a, int x0, d
     }
     zd[2 * (c * M + fft_slot(y >> 1, M, a.g.fft_nst, a.g.fft_first2)) + (y & 1)] = d;
   }
-  __syncthreads();
+  team.sync();
   const double2 *tw = reinterpret_cast<const double2 *>(a.g.tw);
-  fft_stages<true>(z, C, M, ny, a.g.fft_nst, a.g.fft_first2, tw);
+  fft_stages<true>(z, C, M, ny, a.g.fft_nst, a.g.fft_first2, tw, team);
   const int half = M / 2 + 1;
-  for (int e = threadIdx.x; e < C * half; e += blockDim.x) {
+  for (int e = team.tid(); e < C * half; e += team.size()) {
     const int c = e / half, k = e - c * half, x = x0 + c;
     if (x >= nx) continue;
     fft::rfft_post(z + c * M, a.spec + (size_t)x * a.g.jpitch, M, k, tw);
@@ -914,7 +914,7 @@ __device__ __forceinline__ void poisson_fwd_cols(const PoissonArgs &a, int x0, d
 template <bool RCP>
 __global__ void __launch_bounds__(256) k_poisson_fwd(const PoissonArgs a) {
   extern __shared__ double2 z[];
-  poisson_fwd_cols<RCP>(a, blockIdx.x * a.cols, z);
+  poisson_fwd_cols<RCP>(a, blockIdx.x * a.cols, z, fft::Block());
 }
 
 // Thomas sweeps of the Poisson modes. On this GPU an FP64 warp instruction
@@ -1023,12 +1023,12 @@ __global__ void __launch_bounds__(32) k_poisson_tri(const DevGrid g, double2 *sp
 // src/fluid/compute_potential.c:146-157: inverse real DFT along y and the
 // 1/jtot normalisation, psi on the interior (halo and walls implied).
 // CG: read the spectrum through L2 (written by other blocks of the same launch)
-template <bool CG>
-__device__ __forceinline__ void poisson_bwd_cols(const PoissonArgs &a, int x0, double2 *z) {
+template <bool CG, typename Team>
+__device__ __forceinline__ void poisson_bwd_cols(const PoissonArgs &a, int x0, double2 *z, const Team team) {
   const int nx = a.g.nx, ny = a.g.ny, M = ny / 2, C = a.cols;
   const double2 *tw = reinterpret_cast<const double2 *>(a.g.tw);
   const int half = M / 2 + 1;
-  for (int e = threadIdx.x; e < C * half; e += blockDim.x) {
+  for (int e = team.tid(); e < C * half; e += team.size()) {
     const int c = e / half, k = e - c * half, x = x0 + c;
     double2 *zc = z + c * M;
     if (x >= nx) {
@@ -1038,10 +1038,10 @@ __device__ __forceinline__ void poisson_bwd_cols(const PoissonArgs &a, int x0, d
     }
     fft::rfft_pre<CG>(a.spec + (size_t)x * a.g.jpitch, zc, M, k, tw, a.g.fft_nst, a.g.fft_first2);
   }
-  __syncthreads();
-  fft_stages<false>(z, C, M, ny, a.g.fft_nst, a.g.fft_first2, tw);
+  team.sync();
+  fft_stages<false>(z, C, M, ny, a.g.fft_nst, a.g.fft_first2, tw, team);
   const double *zd = reinterpret_cast<const double *>(z);
-  for (int e = threadIdx.x; e < C * ny; e += blockDim.x) {
+  for (int e = team.tid(); e < C * ny; e += team.size()) {
     const int c = e % C, y = e / C, x = x0 + c;
     if (x >= nx) continue;
     a.psi[(size_t)y * nx + x] = zd[2 * (c * M + (y >> 1)) + (y & 1)] * a.s.rny;
@@ -1050,7 +1050,7 @@ __device__ __forceinline__ void poisson_bwd_cols(const PoissonArgs &a, int x0, d
 
 __global__ void __launch_bounds__(256) k_poisson_bwd(const PoissonArgs a) {
   extern __shared__ double2 z[];
-  poisson_bwd_cols<false>(a, blockIdx.x * a.cols, z);
+  poisson_bwd_cols<false>(a, blockIdx.x * a.cols, z, fft::Block());
 }
 
 // ------------------------------------------- fused Poisson (+ temperature)
@@ -1066,15 +1066,28 @@ __global__ void __launch_bounds__(256) k_poisson_bwd(const PoissonArgs a) {
 // so the results are identical.
 //
 // Synchronisation: fwd_done[g] = epoch when group g's spectrum rows are
-// written (release: block barrier, fence, store); a sweep warp reads flags
+// written (release: the team's barrier, fence, store); a sweep warp reads flags
 // with relaxed loads and issues one fence before reading the rows it
 // verified (acquire). bwd_cnt[s] counts the sweep warps that finished span s
 // (span = 2^span_shift x elements), cumulative over launches, so a worker waits
 // for epoch * lines. Spectrum reads of data written in this launch go
 // through L2 (__ldcg). Every wait polls at most `spin` times (kFusedSpin by
 // default, about a second; the host may set fewer); a wait that gives up sets
-// *err and its warp or block stops, so the launch always ends.
+// *err and its warp or team stops, so the launch always ends.
 constexpr int kFusedThreads = 512;
+// Teams of a worker block, each with column groups and a named barrier of its
+// own. A long column's stages and its gathers from the fields leave the FP64
+// pipe idle around each barrier, which another team's column fills; but the
+// columns of a round then come out together and late, and the sweeps, which
+// bound the launch for short columns, start on them. Launch with 1 / 2 / 4
+// teams (CUDA events): 1024 x 2048 457 / 403 / 376 us, 768 x 2048 389 / 350 /
+// 333, 512 x 4096 561 / 514 / 523, 512 x 2048 237 / 208 / 234 (four teams take
+// every column in one round: nothing to sweep until all are done), but
+// 512 x 1024 140 / 149 / 166, 1024 x 1024 268 / 276 / 291, 1024 x 512 240 /
+// 242 / 249. So: teams from kTeamRows rows on, four where the columns still
+// make more than 1.25 rounds.
+constexpr int kFusedTeams = 4;
+constexpr int kTeamRows = 2048;
 // sweep warps per block, one per SM sub-partition. Dependent FP64 chains run
 // ~20% slower with four warps on one SM than with one, but every SM given to
 // the sweeps is taken from the DFT workers, whose FP64 throughput bounds the
@@ -1107,7 +1120,7 @@ struct FusedArgs {
   unsigned long long *bwd_cnt;     // [spans]
   unsigned *err;                   // 1: a sweep wait gave up, 2: a worker wait gave up
   unsigned epoch;
-  int tri_blocks, tri_warps, lines, groups;
+  int tri_blocks, tri_warps, lines, groups, teams;
   int span_shift;                  // span = 2^span_shift x elements
   unsigned spin;                   // polls of a wait before it gives up
   unsigned want;                   // the flag value a sweep waits for: epoch (epoch + 1 in tests of the waits)
@@ -1313,22 +1326,25 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_poisson_fused(const FusedA
     if (!ok && (threadIdx.x & 31) == 0) atomicOr(a.err, 1u);
     return;
   }
-  __shared__ int s_ok;
-  const int wk = blockIdx.x - a.tri_blocks, W = gridDim.x - a.tri_blocks;
+  __shared__ int s_ok[kFusedTeams];
+  const int tn = kFusedThreads / a.teams, th = threadIdx.x / tn;
+  const fft::Part team{(int)threadIdx.x - th * tn, tn, 1 + th};
+  double2 *z = fz + (size_t)th * (C * (g.ny / 2));
+  const int workers = gridDim.x - a.tri_blocks, wk = blockIdx.x - a.tri_blocks + th * workers, W = workers * a.teams;
   // forward DFT column groups, ascending x
   for (int gi = wk; gi < a.groups; gi += W) {
-    poisson_fwd_cols<RCP>(a.p, gi * C, fz);
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    poisson_fwd_cols<RCP>(a.p, gi * C, z, team);
+    team.sync();
+    if (team.tid() == 0) {
       __threadfence();
       st_relaxed_u32(a.fwd_done + gi, a.epoch);
     }
   }
   // explicit temperature update, while the sweeps run
   if (a.with_temp) {
-    const int xb = (nx + kFusedThreads - 1) / kFusedThreads, yb = (g.ny + kRows - 1) / kRows;
+    const int xb = (nx + tn - 1) / tn, yb = (g.ny + kRows - 1) / kRows;
     for (int u = wk; u < xb * yb; u += W) {
-      const int x = (u % xb) * kFusedThreads + threadIdx.x;
+      const int x = (u % xb) * tn + team.tid();
       if (x < nx) {
         if (RCP ? g.p2 : g.dv2) {
           temp_column<0, 0, RCP, true>(a.t, x, (u / xb) * kRows, kRows);
@@ -1342,20 +1358,20 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_poisson_fused(const FusedA
   const unsigned long long target = (unsigned long long)a.epoch * (unsigned long long)a.lines;
   for (int k = wk; k < a.groups; k += W) {
     const int gi = a.groups - 1 - k;
-    if (threadIdx.x == 0) {
+    if (team.tid() == 0) {
       const int s = (gi * C) >> a.span_shift;
       unsigned spin = 0;
       unsigned long long v;
       while ((v = ld_relaxed_u64(a.bwd_cnt + s)) < target && ++spin < a.spin) {
       }
-      s_ok = v >= target;
-      if (!s_ok) atomicOr(a.err, 2u);
+      s_ok[th] = v >= target;
+      if (v < target) atomicOr(a.err, 2u);
       __threadfence();
     }
-    __syncthreads();
-    if (!s_ok) return;
-    poisson_bwd_cols<true>(a.p, gi * C, fz);
-    __syncthreads();
+    team.sync();
+    if (!s_ok[th]) return;
+    poisson_bwd_cols<true>(a.p, gi * C, z, team);
+    team.sync();
   }
 }
 
@@ -2024,8 +2040,17 @@ cudaError_t launch_poisson_fused(const DevGrid &g, const StageScalars &s, const 
   // two sweep warps per block when that still leaves kFusedMinWorkers workers
   const int tri_warps = sms - (lines + 1) / 2 >= kFusedMinWorkers ? 2 : kFusedTriWarps;
   const int tri_blocks = (lines + tri_warps - 1) / tri_warps;
-  const size_t smem = std::max({sizeof(double) * (size_t)g.nx, (size_t)C * g.ny * sizeof(double), kFusedMinSmem});
-  if (!coop || g.nx > kTriMaxNx || smem > 200 * 1024 || sms - tri_blocks < 8) return cudaErrorNotSupported;
+  const size_t cols = (size_t)C * g.ny * sizeof(double);  // shared memory of a team's columns
+  const size_t max_smem = 200 * 1024;
+  int groups = 0, spans = 0, teams = 1;
+  SNS_PLAIN_FORM::fused_layout(g, &groups, &spans);
+  if (g.ny >= kTeamRows) {
+    teams = 4 * groups > 5 * kFusedTeams * (sms - tri_blocks) && kFusedTeams * cols <= max_smem ? kFusedTeams
+            : 2 * cols <= max_smem                                                      ? 2
+                                                                                        : 1;
+  }
+  const size_t smem = std::max({sizeof(double) * (size_t)g.nx, teams * cols, kFusedMinSmem});
+  if (!coop || g.nx > kTriMaxNx || smem > max_smem || sms - tri_blocks < 8) return cudaErrorNotSupported;
   static bool attr = false;
   if (!attr) {
     cudaFuncSetAttribute(k_poisson_fused<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -2052,10 +2077,10 @@ cudaError_t launch_poisson_fused(const DevGrid &g, const StageScalars &s, const 
   a.tri_blocks = tri_blocks;
   a.tri_warps = tri_warps;
   a.lines = lines;
-  int spans = 0;
-  SNS_PLAIN_FORM::fused_layout(g, &a.groups, &spans);
+  a.teams = teams;
+  a.groups = groups;
   // the larger span when the workers can take all of its column groups at once
-  a.span_shift = ((1 << kFusedSpanShiftMax) / C <= sms - tri_blocks) ? kFusedSpanShiftMax : kFusedSpanShiftMax - 1;
+  a.span_shift = ((1 << kFusedSpanShiftMax) / C <= (sms - tri_blocks) * teams) ? kFusedSpanShiftMax : kFusedSpanShiftMax - 1;
   void *args[] = {&a};
   e = cudaLaunchCooperativeKernel(g.rcp ? (const void *)k_poisson_fused<true> : (const void *)k_poisson_fused<false>,
                                   dim3(sms), dim3(kFusedThreads), args, smem, st);
