@@ -20,6 +20,9 @@
 
 #include "fft_dev.cuh"
 #include "sns_internal.h"
+#ifdef SNS_PLAIN_CONTRACT
+#include "stencil_fixed.cuh"
+#endif
 
 // plain_fp64_contract.cu compiles this file a second time, with fused
 // multiply-add contraction, into namespace sns::contract (the parallel form)
@@ -263,13 +266,6 @@ __device__ __forceinline__ void temp_column(const TempArgs &a, int x, int y0, in
   }
 }
 
-template <int IMPX, int IMPY, bool RCP, bool FAST>
-__global__ void __launch_bounds__(128) k_temp(const TempArgs a, int rows) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= a.g.nx) return;
-  temp_column<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
-}
-
 // ------------------------------------------------------------------ velocity
 struct VelArgs {
   DevGrid g;
@@ -394,12 +390,10 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
   return m.ok;
 }
 
+// column x, rows y0 .. y0+rows-1
 template <int IMPX, int IMPY, bool RCP, bool FAST>
-__global__ void __launch_bounds__(128) k_vel(const VelArgs a, int rows) {
+__device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int rows) {
   const int nx = a.g.nx, ny = a.g.ny;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  if (x >= nx) return;
-  const int y0 = blockIdx.y * rows;
   const int y1 = min(y0 + rows, ny);
   const bool left = x == 0, right = x == nx - 1;
   const bool has_ux = x >= 1;  // ux is updated for i = 2..itot
@@ -496,6 +490,24 @@ __global__ void __launch_bounds__(128) k_vel(const VelArgs a, int rows) {
     in.pm = in.pc;
   }
 }
+
+#ifdef SNS_PLAIN_CONTRACT
+#include "stencil_fixed.inc"
+#else
+template <int IMPX, int IMPY, bool RCP, bool FAST>
+__global__ void __launch_bounds__(128) k_temp(const TempArgs a, int rows) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= a.g.nx) return;
+  temp_column<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
+}
+
+template <int IMPX, int IMPY, bool RCP, bool FAST>
+__global__ void __launch_bounds__(128) k_vel(const VelArgs a, int rows) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  if (x >= a.g.nx) return;
+  vel_march<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
+}
+#endif
 
 __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -1620,6 +1632,19 @@ cudaError_t launch_temp_update(const DevGrid &g, const StageScalars &s, int impx
   const TempArgs a{g, s, t_in, t_out, at, qt, ux, uy};
   const int rows = march_rows(g);
   const dim3 grid = march_grid(g, rows), block(kBlockX);
+#ifdef SNS_PLAIN_CONTRACT
+#define SNS_F(E)                                                     \
+  if (impx && impy) k_temp_fx<1, 1, E><<<grid, block, 0, st>>>(a, rows); \
+  else if (impx) k_temp_fx<1, 0, E><<<grid, block, 0, st>>>(a, rows);    \
+  else if (impy) k_temp_fx<0, 1, E><<<grid, block, 0, st>>>(a, rows);    \
+  else k_temp_fx<0, 0, E><<<grid, block, 0, st>>>(a, rows)
+  if (g.eq) {
+    SNS_F(true);
+  } else {
+    SNS_F(false);
+  }
+#undef SNS_F
+#else
 #define SNS_T(X, Y, R, F) k_temp<X, Y, R, F><<<grid, block, 0, st>>>(a, rows)
   if (g.p2) {
     if (impx && impy) SNS_T(1, 1, true, true);
@@ -1643,6 +1668,7 @@ cudaError_t launch_temp_update(const DevGrid &g, const StageScalars &s, int impx
     else SNS_T(0, 0, false, false);
   }
 #undef SNS_T
+#endif
   count_launches(1);
   return cudaGetLastError();
 }
@@ -1654,6 +1680,19 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
   const VelArgs a{g, s, ux, uy, p, tforce, ux_out, uy_out, aux, auy, qx, qy};
   const int rows = march_rows(g);
   const dim3 grid = march_grid(g, rows), block(kBlockX);
+#ifdef SNS_PLAIN_CONTRACT
+#define SNS_F(E)                                                     \
+  if (impx && impy) k_vel_fx<1, 1, E><<<grid, block, 0, st>>>(a, rows); \
+  else if (impx) k_vel_fx<1, 0, E><<<grid, block, 0, st>>>(a, rows);    \
+  else if (impy) k_vel_fx<0, 1, E><<<grid, block, 0, st>>>(a, rows);    \
+  else k_vel_fx<0, 0, E><<<grid, block, 0, st>>>(a, rows)
+  if (g.eq) {
+    SNS_F(true);
+  } else {
+    SNS_F(false);
+  }
+#undef SNS_F
+#else
 #define SNS_V(X, Y, R, F) k_vel<X, Y, R, F><<<grid, block, 0, st>>>(a, rows)
   if (g.p2) {
     if (impx && impy) SNS_V(1, 1, true, true);
@@ -1677,6 +1716,7 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
     else SNS_V(0, 0, false, false);
   }
 #undef SNS_V
+#endif
   count_launches(1);
   return cudaGetLastError();
 }

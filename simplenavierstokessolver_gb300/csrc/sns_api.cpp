@@ -330,6 +330,11 @@ static int build_context(Context *c, const param_t *param) {
     g.p2 = ok;
     g.p2u = ok;
     for (double v : c->dxf) g.p2u = g.p2u && v == c->dxf[0];
+    g.eq = rdxc[0] == 2.0 * rdxf[0] && rdxc[nx] == 2.0 * rdxf[0];
+    for (int i = 0; i < nx; i++) {
+      g.eq = g.eq && rdxf[i] == rdxf[0];
+      if (i > 0) g.eq = g.eq && rdxc[i] == rdxf[0] && cfm[i] == 0.5 && cfp[i] == 0.5;
+    }
   }
   int rc = SNS_OK;
   g.dv2 = false;

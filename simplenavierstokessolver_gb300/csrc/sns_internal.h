@@ -29,6 +29,7 @@ struct DevGrid {
   bool rcp;                // every metric divisor is a power of two
   bool p2;                 // rcp, and every reciprocal spacing, advective and Poisson coefficient is 2^e, |e| <= 64
   bool p2u;                // p2, and every DXF(i) is the same
+  bool eq;                 // every 1/DXF(i) is the same, 1/DXC(i) too or (at the walls) twice it, to the bit
   bool dv2;                // not rcp, and division by dy takes two instructions (invariant_divisor in host_common.h)
   double dy, rdy, rdyl;    // rdyl, rdxf_l, rdxc_l: with the reciprocal the pair that divides (NaN where none does)
   const double *dxf;    // [nx]    DXF(i)
