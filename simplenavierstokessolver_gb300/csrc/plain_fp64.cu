@@ -20,6 +20,7 @@
 
 #include "fft_dev.cuh"
 #include "sns_internal.h"
+#include "chain.cuh"
 #ifdef SNS_PLAIN_CONTRACT
 #include "stencil_fixed.cuh"
 #endif
@@ -496,6 +497,7 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
 #else
 template <int IMPX, int IMPY, bool RCP, bool FAST>
 __global__ void __launch_bounds__(128) k_temp(const TempArgs a, int rows) {
+  chain_begin();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.g.nx) return;
   temp_column<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
@@ -503,6 +505,7 @@ __global__ void __launch_bounds__(128) k_temp(const TempArgs a, int rows) {
 
 template <int IMPX, int IMPY, bool RCP, bool FAST>
 __global__ void __launch_bounds__(128) k_vel(const VelArgs a, int rows) {
+  chain_begin();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.g.nx) return;
   vel_march<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
@@ -635,6 +638,7 @@ __device__ __forceinline__ void row_serial(double *row, const LineFactors &f, in
 }
 
 __global__ void __launch_bounds__(32) k_solve_x(int nx, int ny, const SolveXSet set) {
+  chain_begin();
   const int y = blockIdx.x * blockDim.x + threadIdx.x;
   if (y >= ny) return;
   row_serial(set.q[blockIdx.y] + (size_t)y * nx, set.f[blockIdx.y], set.mode[blockIdx.y], nx);
@@ -681,6 +685,7 @@ __device__ __forceinline__ void column_serial(double *col, const PeriodicFactors
 }
 
 __global__ void __launch_bounds__(32) k_solve_y(int nx, int ny, const SolveYSet set) {
+  chain_begin();
   const int x = set.first_col[blockIdx.y] + blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= nx) return;
   column_serial(set.q[blockIdx.y] + x, set.f[blockIdx.y], nx, ny);
@@ -749,6 +754,7 @@ __device__ __noinline__ void line_again(double *q, size_t es, const PeriodicFact
 
 template <bool COLS>
 __global__ void __launch_bounds__(kSegThreads) k_solve_seg(int nx, int ny, const SegArgs a) {
+  chain_begin();
   extern __shared__ double sm[];
   __shared__ int bad[8];
   // selects, not an index into the parameters (which would copy them to the stack)
@@ -861,6 +867,7 @@ __global__ void __launch_bounds__(kSegThreads) k_solve_seg(int nx, int ny, const
 }
 
 __global__ void k_add_increment(int nx, int ny, int kind, const double *in, const double *q, double *out) {
+  chain_begin();
   const size_t n = (size_t)nx * ny;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
     const int x = (int)(k % nx);
@@ -925,6 +932,7 @@ __device__ __forceinline__ void poisson_fwd_cols(const PoissonArgs &a, int x0, d
 
 template <bool RCP>
 __global__ void __launch_bounds__(256) k_poisson_fwd(const PoissonArgs a) {
+  chain_begin();
   extern __shared__ double2 z[];
   poisson_fwd_cols<RCP>(a, blockIdx.x * a.cols, z, fft::Block());
 }
@@ -968,6 +976,7 @@ __device__ __forceinline__ void tri_issue(TriRing &R, int slot, const double *va
 // parts undergo identical real operations (real matrix), so they are solved
 // as independent real lines. blockIdx.y selects the component.
 __global__ void __launch_bounds__(32) k_poisson_tri(const DevGrid g, double2 *spec) {
+  chain_begin();
   extern __shared__ double tri_smem[];
   TriRing &R = *reinterpret_cast<TriRing *>(tri_smem);
   double *pl = tri_smem + sizeof(TriRing) / sizeof(double);
@@ -1061,6 +1070,7 @@ __device__ __forceinline__ void poisson_bwd_cols(const PoissonArgs &a, int x0, d
 }
 
 __global__ void __launch_bounds__(256) k_poisson_bwd(const PoissonArgs a) {
+  chain_begin();
   extern __shared__ double2 z[];
   poisson_bwd_cols<false>(a, blockIdx.x * a.cols, z, fft::Block());
 }
@@ -1477,6 +1487,7 @@ __device__ __forceinline__ bool corr_cell(const StageScalars &t, const CorrCol &
 // thread instead of CR.
 template <int IMPX, int IMPY, bool RCP, bool CORR, bool PRES, int CR>
 __global__ void __launch_bounds__(128) k_corr(const CorrArgs a) {
+  chain_begin();
   const int nx = a.g.nx, ny = a.g.ny;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const bool live = x < nx;
@@ -1576,6 +1587,7 @@ __global__ void __launch_bounds__(128) k_corr(const CorrArgs a) {
 
 __global__ void __launch_bounds__(128) k_umax(int nx, int ny, const double *ux, const double *uy,
                                               unsigned long long *colmax, unsigned long long *uymax) {
+  chain_begin();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long mx = 0ull, my = 0ull;
   bool nf = false;
@@ -1645,10 +1657,10 @@ cudaError_t launch_temp_update(const DevGrid &g, const StageScalars &s, int impx
   const dim3 grid = march_grid(g, rows), block(kBlockX);
 #ifdef SNS_PLAIN_CONTRACT
 #define SNS_F(E)                                                     \
-  if (impx && impy) k_temp_fx<1, 1, E><<<grid, block, 0, st>>>(a, rows); \
-  else if (impx) k_temp_fx<1, 0, E><<<grid, block, 0, st>>>(a, rows);    \
-  else if (impy) k_temp_fx<0, 1, E><<<grid, block, 0, st>>>(a, rows);    \
-  else k_temp_fx<0, 0, E><<<grid, block, 0, st>>>(a, rows)
+  if (impx && impy) chain_launch(k_temp_fx<1, 1, E>, grid, block, 0, st, a, rows); \
+  else if (impx) chain_launch(k_temp_fx<1, 0, E>, grid, block, 0, st, a, rows);    \
+  else if (impy) chain_launch(k_temp_fx<0, 1, E>, grid, block, 0, st, a, rows);    \
+  else chain_launch(k_temp_fx<0, 0, E>, grid, block, 0, st, a, rows)
   if (g.eq) {
     SNS_F(true);
   } else {
@@ -1656,7 +1668,7 @@ cudaError_t launch_temp_update(const DevGrid &g, const StageScalars &s, int impx
   }
 #undef SNS_F
 #else
-#define SNS_T(X, Y, R, F) k_temp<X, Y, R, F><<<grid, block, 0, st>>>(a, rows)
+#define SNS_T(X, Y, R, F) chain_launch(k_temp<X, Y, R, F>, grid, block, 0, st, a, rows)
   if (g.p2) {
     if (impx && impy) SNS_T(1, 1, true, true);
     else if (impx) SNS_T(1, 0, true, true);
@@ -1693,10 +1705,10 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
   const dim3 grid = march_grid(g, rows), block(kBlockX);
 #ifdef SNS_PLAIN_CONTRACT
 #define SNS_F(E)                                                     \
-  if (impx && impy) k_vel_fx<1, 1, E><<<grid, block, 0, st>>>(a, rows); \
-  else if (impx) k_vel_fx<1, 0, E><<<grid, block, 0, st>>>(a, rows);    \
-  else if (impy) k_vel_fx<0, 1, E><<<grid, block, 0, st>>>(a, rows);    \
-  else k_vel_fx<0, 0, E><<<grid, block, 0, st>>>(a, rows)
+  if (impx && impy) chain_launch(k_vel_fx<1, 1, E>, grid, block, 0, st, a, rows); \
+  else if (impx) chain_launch(k_vel_fx<1, 0, E>, grid, block, 0, st, a, rows);    \
+  else if (impy) chain_launch(k_vel_fx<0, 1, E>, grid, block, 0, st, a, rows);    \
+  else chain_launch(k_vel_fx<0, 0, E>, grid, block, 0, st, a, rows)
   if (g.eq) {
     SNS_F(true);
   } else {
@@ -1704,7 +1716,7 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
   }
 #undef SNS_F
 #else
-#define SNS_V(X, Y, R, F) k_vel<X, Y, R, F><<<grid, block, 0, st>>>(a, rows)
+#define SNS_V(X, Y, R, F) chain_launch(k_vel<X, Y, R, F>, grid, block, 0, st, a, rows)
   if (g.p2) {
     if (impx && impy) SNS_V(1, 1, true, true);
     else if (impx) SNS_V(1, 0, true, true);
@@ -1778,9 +1790,9 @@ cudaError_t launch_solve_x_set(const DevGrid &g, const SolveXSet &set, cudaStrea
       cudaFuncSetAttribute(k_solve_seg<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       attr = true;
     }
-    k_solve_seg<false><<<dim3((g.ny + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st>>>(g.nx, g.ny, a);
+    chain_launch(k_solve_seg<false>, dim3((g.ny + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st, g.nx, g.ny, a);
   } else {
-    k_solve_x<<<dim3((g.ny + 31) / 32, set.n), 32, 0, st>>>(g.nx, g.ny, set);
+    chain_launch(k_solve_x, dim3((g.ny + 31) / 32, set.n), 32, 0, st, g.nx, g.ny, set);
   }
   count_launches(1);
   return cudaGetLastError();
@@ -1803,9 +1815,9 @@ cudaError_t launch_solve_y_set(const DevGrid &g, const SolveYSet &set, cudaStrea
       cudaFuncSetAttribute(k_solve_seg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
       attr = true;
     }
-    k_solve_seg<true><<<dim3((g.nx + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st>>>(g.nx, g.ny, a);
+    chain_launch(k_solve_seg<true>, dim3((g.nx + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st, g.nx, g.ny, a);
   } else {
-    k_solve_y<<<dim3((g.nx + 31) / 32, set.n), 32, 0, st>>>(g.nx, g.ny, set);
+    chain_launch(k_solve_y, dim3((g.nx + 31) / 32, set.n), 32, 0, st, g.nx, g.ny, set);
   }
   count_launches(1);
   return cudaGetLastError();
@@ -1833,7 +1845,7 @@ cudaError_t launch_add_increment(const DevGrid &g, int kind, const double *in, c
                                  cudaStream_t st) {
   const size_t n = (size_t)g.nx * g.ny;
   const int blocks = (int)std::min<size_t>((n + 255) / 256, 152 * 16);
-  k_add_increment<<<blocks, 256, 0, st>>>(g.nx, g.ny, kind, in, q, out);
+  chain_launch(k_add_increment, blocks, 256, 0, st, g.nx, g.ny, kind, in, q, out);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -2047,9 +2059,9 @@ cudaError_t launch_poisson_fwd(const DevGrid &g, const StageScalars &s, const do
   const PoissonArgs a{g, s, ux, uy, spec, nullptr, C};
   const int blocks = (g.nx + C - 1) / C;
   if (g.rcp) {
-    k_poisson_fwd<true><<<blocks, poisson_threads(g, C), smem, st>>>(a);
+    chain_launch(k_poisson_fwd<true>, blocks, poisson_threads(g, C), smem, st, a);
   } else {
-    k_poisson_fwd<false><<<blocks, poisson_threads(g, C), smem, st>>>(a);
+    chain_launch(k_poisson_fwd<false>, blocks, poisson_threads(g, C), smem, st, a);
   }
   count_launches(1);
   return cudaGetLastError();
@@ -2063,7 +2075,7 @@ cudaError_t launch_poisson_tri(const DevGrid &g, double2 *spec, cudaStream_t st)
                          (int)(sizeof(TriRing) + sizeof(double) * (size_t)kTriMaxNx));
     attr = true;
   }
-  k_poisson_tri<<<dim3((g.nh + 31) / 32, 2), 32, smem, st>>>(g, spec);
+  chain_launch(k_poisson_tri, dim3((g.nh + 31) / 32, 2), 32, smem, st, g, spec);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -2149,7 +2161,7 @@ cudaError_t launch_poisson_bwd(const DevGrid &g, const StageScalars &s, const do
   const int C = poisson_setup(g, &smem);
   const PoissonArgs a{g, s, nullptr, nullptr, const_cast<double2 *>(spec), psi, C};
   const int blocks = (g.nx + C - 1) / C;
-  k_poisson_bwd<<<blocks, poisson_threads(g, C), smem, st>>>(a);
+  chain_launch(k_poisson_bwd, blocks, poisson_threads(g, C), smem, st, a);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -2165,8 +2177,8 @@ static cudaError_t launch_corr_t(const DevGrid &g, const StageScalars &s, int im
   const dim3 grid = march_grid(g, small ? 1 : kCorrRows), block(kBlockX);
 #define SNS_C(X, Y, R)                                                \
   do {                                                                \
-    if (small) k_corr<X, Y, R, CORR, PRES, 1><<<grid, block, 0, st>>>(a); \
-    else k_corr<X, Y, R, CORR, PRES, kCorrRows><<<grid, block, 0, st>>>(a); \
+    if (small) chain_launch(k_corr<X, Y, R, CORR, PRES, 1>, grid, block, 0, st, a); \
+    else chain_launch(k_corr<X, Y, R, CORR, PRES, kCorrRows>, grid, block, 0, st, a); \
   } while (0)
   if (g.rcp) {
     if (impx && impy) SNS_C(1, 1, true);
@@ -2202,7 +2214,7 @@ cudaError_t launch_correct_pressure(const DevGrid &g, const StageScalars &s, int
 
 cudaError_t launch_umax(const DevGrid &g, const double *ux, const double *uy, unsigned long long *colmax,
                         unsigned long long *uymax, cudaStream_t st) {
-  k_umax<<<march_grid(g, kRows), kBlockX, 0, st>>>(g.nx, g.ny, ux, uy, colmax, uymax);
+  chain_launch(k_umax, march_grid(g, kRows), kBlockX, 0, st, g.nx, g.ny, ux, uy, colmax, uymax);
   count_launches(1);
   return cudaGetLastError();
 }

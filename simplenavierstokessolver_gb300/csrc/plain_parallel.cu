@@ -36,6 +36,7 @@
 #include "host_common.h"
 #include "sns_gpu.h"
 #include "sns_internal.h"
+#include "chain.cuh"
 
 namespace sns {
 namespace {
@@ -60,6 +61,7 @@ __device__ __forceinline__ int par_p(int x, int m) { return (x % m) * kPartSeg +
 // along y, for the adjacent columns x0 .. x0+cols-1 (coalesced reads of the
 // velocity); each column's spectrum goes to its line position
 __global__ void __launch_bounds__(256) k_par_fwd(const ParArgs a) {
+  chain_begin();
   extern __shared__ double2 z[];
   const int nx = a.g.nx, ny = a.g.ny, M = ny / 2, C = a.cols;
   const int x0 = blockIdx.x * C;
@@ -90,6 +92,7 @@ __global__ void __launch_bounds__(256) k_par_fwd(const ParArgs a) {
 
 // src/fluid/compute_potential.c:146-157: inverse real DFT and 1/jtot
 __global__ void __launch_bounds__(256) k_par_bwd(const ParArgs a) {
+  chain_begin();
   extern __shared__ double2 z[];
   const int nx = a.g.nx, ny = a.g.ny, M = ny / 2, C = a.cols;
   const int x0 = blockIdx.x * C;
@@ -140,6 +143,7 @@ struct FixArgs {
 // the same bits in 3 FP64 instructions per value instead of 4.
 template <int V>
 __global__ void __launch_bounds__(512, 1) k_par_fwd_fx(const FixArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char fx_sm[];
   __shared__ fx::Slots slots;
   const int nx = a.g.nx, ny = a.g.ny, x0 = blockIdx.x << a.lgC;
@@ -177,6 +181,7 @@ __global__ void __launch_bounds__(512, 1) k_par_fwd_fx(const FixArgs a) {
 // src/fluid/compute_potential.c:146-157: the inverse into psi
 template <int V>
 __global__ void __launch_bounds__(512, 1) k_par_bwd_fx(const FixArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char fx_sm[];
   __shared__ fx::Slots slots;
   const int nx = a.g.nx, x0 = blockIdx.x << a.lgC;
@@ -238,6 +243,7 @@ constexpr int kParChunk = 8;
 // memory and writes it back.
 template <bool STAGED>
 __global__ void __launch_bounds__(32 * kParWarpsMax) k_par_tri(const ParTriArgs a) {
+  chain_begin();
   extern __shared__ __align__(128) unsigned char sm[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int li = w >> 1, comp = w & 1;  // line of the block, part (0 real, 1 imaginary)
@@ -457,6 +463,7 @@ __device__ __forceinline__ int cn_pos(int e, int m, int s) {
 // (odd, so that the 32 lanes' accesses at one row fall on distinct bank
 // pairs), solved there and written back, coalesced both ways.
 __global__ void __launch_bounds__(32 * kCnWarpsMax) k_par_cn(const ParCnArgs a) {
+  chain_begin();
   extern __shared__ __align__(16) double cn_sm[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   const ParCnField F = cn_field(a);
@@ -590,6 +597,7 @@ __global__ void __launch_bounds__(32 * kCnWarpsMax) k_par_cn(const ParCnArgs a) 
 constexpr int kCnCols = 4;
 
 __global__ void __launch_bounds__(32 * kCnCols) k_par_cn_cols(const ParCnArgs a) {
+  chain_begin();
   __shared__ double ex[3][kCnCols][kPartSeg];
   const ParCnField F = cn_field(a);
   const int n = a.n, m = a.m;
@@ -741,12 +749,12 @@ cudaError_t launch_par_fwd(const DevGrid &g, const StageScalars &s, const double
     const FixShape f = fix_shape(g);
     const FixArgs a{g, ux, uy, spec, nullptr, 0.0, f.lgC, g.nx / kPartSeg};
     const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
-    if (f.v == 8) k_par_fwd_fx<8><<<blocks, f.threads, f.smem, st>>>(a);
-    else k_par_fwd_fx<4><<<blocks, f.threads, f.smem, st>>>(a);
+    if (f.v == 8) chain_launch(k_par_fwd_fx<8>, blocks, f.threads, f.smem, st, a);
+    else chain_launch(k_par_fwd_fx<4>, blocks, f.threads, f.smem, st, a);
   } else {
     const int C = par_cols(g);
     const ParArgs a{g, s, ux, uy, spec, nullptr, C, g.nx / kPartSeg};
-    k_par_fwd<<<(g.nx + C - 1) / C, par_threads(g, C), (size_t)C * g.ny * sizeof(double), st>>>(a);
+    chain_launch(k_par_fwd, (g.nx + C - 1) / C, par_threads(g, C), (size_t)C * g.ny * sizeof(double), st, a);
   }
   count_launches(1);
   return cudaGetLastError();
@@ -768,9 +776,9 @@ cudaError_t launch_par_tri(const DevGrid &g, double2 *spec, const ParFactors &pf
                      pf.stale};
   const size_t smem = 128 + (size_t)lpb * per_line;
   if (staged) {
-    k_par_tri<true><<<(g.nh + lpb - 1) / lpb, 64 * lpb, smem, st>>>(a);
+    chain_launch(k_par_tri<true>, (g.nh + lpb - 1) / lpb, 64 * lpb, smem, st, a);
   } else {
-    k_par_tri<false><<<(g.nh + lpb - 1) / lpb, 64 * lpb, smem, st>>>(a);
+    chain_launch(k_par_tri<false>, (g.nh + lpb - 1) / lpb, 64 * lpb, smem, st, a);
   }
   count_launches(1);
   return cudaGetLastError();
@@ -798,14 +806,14 @@ cudaError_t launch_par_cn(bool columns, ParCnArgs a, cudaStream_t st) {
   a.s = a.m | 1;
   if (columns) {
     const dim3 grid((a.lines + kCnCols - 1) / kCnCols, a.nf);
-    k_par_cn_cols<<<grid, 32 * kCnCols, 0, st>>>(a);
+    chain_launch(k_par_cn_cols, grid, 32 * kCnCols, 0, st, a);
   } else {
     const size_t per = cn_warp_doubles(a.n) * sizeof(double);
     // warps (rows) per block: two blocks per SM where the rows fit
     int wpb = (int)std::min<size_t>(kCnWarpsMax, (kParSmemMax / 2) / per);
     if (wpb < 1) wpb = 1;
     const dim3 grid((a.lines + wpb - 1) / wpb, a.nf);
-    k_par_cn<<<grid, 32 * wpb, wpb * per, st>>>(a);
+    chain_launch(k_par_cn, grid, 32 * wpb, wpb * per, st, a);
   }
   count_launches(1);
   return cudaGetLastError();
@@ -819,12 +827,12 @@ cudaError_t launch_par_bwd(const DevGrid &g, const StageScalars &s, const double
     const FixArgs a{g,     nullptr, nullptr, const_cast<double2 *>(spec), psi, s.rgdt * (0.5 * s.rny),
                     f.lgC, g.nx / kPartSeg};
     const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
-    if (f.v == 8) k_par_bwd_fx<8><<<blocks, f.threads, f.smem, st>>>(a);
-    else k_par_bwd_fx<4><<<blocks, f.threads, f.smem, st>>>(a);
+    if (f.v == 8) chain_launch(k_par_bwd_fx<8>, blocks, f.threads, f.smem, st, a);
+    else chain_launch(k_par_bwd_fx<4>, blocks, f.threads, f.smem, st, a);
   } else {
     const int C = par_cols(g);
     const ParArgs a{g, s, nullptr, nullptr, const_cast<double2 *>(spec), psi, C, g.nx / kPartSeg};
-    k_par_bwd<<<(g.nx + C - 1) / C, par_threads(g, C), (size_t)C * g.ny * sizeof(double), st>>>(a);
+    chain_launch(k_par_bwd, (g.nx + C - 1) / C, par_threads(g, C), (size_t)C * g.ny * sizeof(double), st, a);
   }
   count_launches(1);
   return cudaGetLastError();
