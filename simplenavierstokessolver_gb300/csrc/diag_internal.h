@@ -9,7 +9,7 @@
 namespace sns {
 
 constexpr int kDiagSums = 10;  // compensated sums per block
-constexpr int kDiagRows = 16;  // rows per thread
+constexpr int kDiagRows = 16;  // rows of diag_blocks
 
 // dense fields (x fastest, no halos), metrics as DXF(i) = dxf[i-1], DXC(i) = dxc[i-1]
 template <typename F>
@@ -37,7 +37,8 @@ cudaError_t launch_diag(const DiagArgs<F> &a, double *scratch, double **out, cud
 
 // allocation-free form: block partials in a fixed file-scope device array of
 // kDiagStaticBlocks blocks (672 KiB), the final sum on the device; grids with
-// more blocks (diag_blocks) are rejected. Blocks until done.
+// more blocks (diag_blocks: of kDiagRows rows and 64 ux points) are rejected.
+// Launches have no more blocks than that, or 1217. Blocks until done.
 constexpr int kDiagStaticBlocks = 4096;
 int diag_blocks(int nx, int ny);
 cudaError_t diag_static(const DiagArgs<double> &a, cudaStream_t st, double out[11]);

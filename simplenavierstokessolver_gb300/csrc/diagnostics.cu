@@ -3,29 +3,35 @@
 // stencils of src/analyses.c:8-121): maximum and sum of the divergence,
 // x/y momentum, kinetic (x, y) and thermal energy, and the Nusselt number
 // from the wall heat flux, the energy injection, the kinetic and the thermal
-// dissipation. All arithmetic is FP64; every sum is accumulated with
-// Neumaier's compensated summation per thread, merged per block and over the
+// dissipation. All arithmetic is FP64; every sum is accumulated
+// exactly per thread, rounded to a pair of doubles, merged per block and over the
 // blocks with the compensation carried along, so the result agrees with the
 // reference's sequential sums to their own round-off. Fields may be FP64
 // (plain path) or FP32 (batched form); FP32 values are widened exactly.
 //
 // FP64 issue bounds the pass (an FP64 instruction holds a sub-partition of
-// GB300 for ~70-80 cycles, an integer one for 1-2), so the terms are arranged
-// for few FP64 instructions per cell, about 62 instead of about 590:
-//  * the cell size and the constants are factors of a thread's column and
-//    multiply its sums once, at the end;
+// GB300 for ~65-80 cycles, an integer one for 1-2), so the terms are arranged
+// for few FP64 instructions per cell, 19 instead of about 590:
+//  * the sums of a thread are 128-bit integers (Sum128), ~30 integer
+//    instructions a term instead of the 4 FP64 additions of a compensated one;
+//  * the cell size, the constants and the weights of the squared differences
+//    are factors of a thread's column and multiply its sums once, at the end;
 //  * the reference adds every squared difference twice, with weight 1/2 to the
 //    two points it separates (weight 1 at a wall, from one side); here each
 //    difference is squared once, with the full weight;
 //  * divisions by spacings become products by reciprocals, except in the
 //    divergence, whose maximum is the reference's bit for bit: there they
 //    stay divisions unless the spacings are powers of two;
-//  * compensation tests compare the operands' bits with integer instructions;
 //  * the sums of a block's 64 threads are merged by 60 threads and then 10,
-//    not by one thread in turn (which took 0.5 ms whatever the grid).
-// sns_diagnostics, host time per call: 128 x 256 547 -> 117 us, 512 x 1024
-// 745 -> 167 us, 1024 x 2048 2690 -> 505 us. What is left at 512 x 1024 is
-// the FP64 issue of the 62 instructions (~137 us).
+//    not by one thread in turn (which took 0.5 ms whatever the grid);
+//  * a small grid's threads take fewer rows (diag_rows).
+// sns_diagnostics, host time per call: with compensated FP64 sums (62 FP64
+// instructions a cell, 16 rows per thread on every grid) against this, 64 x 128
+// 110 / 42 us, 128 x 256 stretched 127 / 50, 512 x 1024 168 / 91, 1024 x 2048
+// 507 / 201, 2048 x 4096 1728 / 720; ~20 us of each are the two launches, the
+// copy and the wait. The FP64 pipe is still the busiest (65 % of its cycles at
+// 512 x 1024): the merges of a thread's and a block's sums add as much as ten
+// rows.
 #include <cstdint>
 #include <mutex>
 
@@ -61,87 +67,172 @@ __device__ __forceinline__ bool pow2(double d) {
   return __double2loint(d) == 0 && (__double2hiint(d) & 0xfffff) == 0;
 }
 
+// A sum of doubles without rounding: a 128-bit integer in units of
+// 2^(e - 1132), so that the 53 bits of a term whose biased exponent is e reach
+// from bit 57 up and 16 bits are left above for 65536 terms. A term with a
+// larger exponent than e moves the sum down first, to an exponent 20 above its
+// own, so that few threads of a warp ever do it after their first row. Terms
+// are cut off at 2^-90 of the largest one or below. Infinities and NaN make the
+// sum NaN, as the compensated sum's (inf - inf).
+__device__ __forceinline__ long long shr(long long v, int s) {  // amounts of 64 and more leave the sign
+  long long r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+  return r;
+}
+__device__ __forceinline__ unsigned long long shl(long long v, int s) {  // amounts of 64 and more leave 0
+  unsigned long long r;
+  asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+  return r;
+}
+struct Sum128 {
+  static constexpr int kNan = 8192;  // e of a sum that is NaN
+  static constexpr int kMargin = 20;
+  unsigned long long lo;
+  long long hi;
+  int e;
+  __device__ __forceinline__ void raise(int ev) {
+    const int n = ev == 0x7ff ? kNan : ev + kMargin, d = n - e;
+    lo = d < 64 ? (d ? lo >> d | (unsigned long long)hi << (64 - d) : lo) : (unsigned long long)shr(hi, d - 64);
+    hi = shr(hi, d);
+    e = n;
+  }
+  template <bool NONNEG = false>
+  __device__ __forceinline__ void add(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int ev = (int)(b >> 52) & 0x7ff;
+    if (ev > e) raise(ev);
+    long long m = (long long)((b & 0xfffffffffffffull) | (ev ? 1ull << 52 : 0ull));
+    if (!NONNEG) {
+      const long long n = (long long)b >> 63;
+      m = (m ^ n) - n;
+    }
+    const int s = e - max(ev, 1);
+    const unsigned long long l = s <= 57 ? shl(m, 57 - s) : (unsigned long long)shr(m, s - 57);
+    const unsigned long long t = lo + l;
+    hi += shr(m, s + 7) + (t < l);
+    lo = t;
+  }
+  // times f, as a pair of doubles whose sum it is to 2^-106
+  __device__ __forceinline__ Neu pair(double f) const {
+    if (e >= kNan) return {__longlong_as_double(0x7ff8000000000000ll), 0.0};
+    const bool neg = hi < 0;
+    unsigned long long h = (unsigned long long)hi, l = lo;
+    if (neg) {
+      l = 0ull - l;
+      h = ~h + (l == 0ull);
+    }
+    if ((h | l) == 0ull) return {0.0, 0.0};
+    const int z = h ? __clzll((long long)h) : 64 + __clzll((long long)l);
+    // to the top: 53 bits for each double
+    if (z >= 64) {
+      h = l << (z - 64);
+      l = 0ull;
+    } else if (z) {
+      h = h << z | l >> (64 - z);
+      l <<= z;
+    }
+    const int k = e - 1132 + 75 - z;  // of the first double's last bit
+    const unsigned long long m0 = h >> 11, m1 = (h & 0x7ff) << 42 | l >> 22;
+    // m 2^q without FP64 instructions; m's top bit is bit 52 - up
+    auto value = [&](unsigned long long m, int q, int up) {
+      const int ex = q - up + 52 + 1023;
+      const unsigned long long b = (m << up) + ((unsigned long long)(ex - 1) << 52);
+      double d = __longlong_as_double((long long)(m ? b : 0ull));
+      if (m && (ex < 1 || ex > 2046)) d = scalbn((double)m, q);
+      return neg ? -d : d;
+    };
+    const int up = min(__clzll((long long)m1) - 11, 52);
+    return {value(m0, k, 0) * f, value(m1, k - 53, up) * f};
+  }
+};
+
 constexpr int kDiagThreads = 64;
+constexpr int kDiagWarps = 608;  // one per sub-partition
+constexpr int kDiagMarch = 32;   // rows per thread, at most
 constexpr int kDiagParts = 6;  // threads merging one sum of a block
 
-// One thread per ux point (column x, i = x+1 in [1, nx+1]) and kDiagRows rows.
+// One thread per column x (ux point i = x+1 and the cell behind it; the last
+// column also the wall's face) and `rows` rows.
 template <typename F>
-__global__ void __launch_bounds__(kDiagThreads) k_diag(DiagArgs<F> a, double *partials) {
+__global__ void __launch_bounds__(kDiagThreads, 8) k_diag(DiagArgs<F> a, double *partials, int rows) {
   const int nx = a.nx, ny = a.ny;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y0 = blockIdx.y * kDiagRows, y1 = min(y0 + kDiagRows, ny);
+  const int y0 = blockIdx.y * rows, y1 = min(y0 + rows, ny);
   Neu acc[kDiagSums];
 #pragma unroll
   for (int k = 0; k < kDiagSums; ++k) acc[k] = {0.0, 0.0};
   unsigned long long divmax = 0ull;
-  if (x <= nx) {
+  if (x < nx) {
     const double dy = a.dy, q = a.sqrt_pr_ra;
-    const bool cell = x < nx, inner = x > 0 && cell;  // cell centre i = x+1 <= nx; ux point off the walls
+    const bool first = x == 0, last = x == nx - 1;
     auto LD = [](const F *hi, const float *lo, size_t k) -> double {
       return lo ? (double)hi[k] + (double)lo[k] : (double)hi[k];
     };
-    auto UX = [&](int xi, int y) -> double {  // ux at i = xi+1; walls i = 1 and nx+1 are zero
-      return (xi <= 0 || xi >= nx) ? 0.0 : LD(a.ux, a.uxl, (size_t)y * nx + xi);
-    };
-    auto UY = [&](int xi, int y) -> double {  // uy at i = xi+1, zero at i = 0 and nx+1
-      return (xi < 0 || xi >= nx) ? 0.0 : LD(a.uy, a.uyl, (size_t)y * nx + xi);
-    };
-    auto TT = [&](int xi, int y) -> double {
-      return xi < 0 ? 0.5 : xi >= nx ? -0.5 : LD(a.t, a.tl, (size_t)y * nx + xi);
-    };
-    const double dxc = a.dxc[x];               // DXC(i), i = x+1 <= nx+1
-    const double dxf = cell ? a.dxf[x] : 1.0;  // DXF(i)
+    // ux at i = x+1 (zero at the walls i = 1 and nx+1), uy and T of the cell
+    const double dxc = a.dxc[x], dxf = a.dxf[x], dxw = a.dxc[nx];
     const double rdy = 1.0 / dy, rdxf = 1.0 / dxf;
     const bool p2 = pow2(dy) && pow2(dxf);  // products by the reciprocals are the divisions
-    // weights of the squared differences: along x across a cell (ux) and across
-    // a face (uy, T), along y at a ux point and at a cell
-    const double wcx = cell ? dy * rdxf : 0.0, wfx = dy / dxc;
-    const double wuy = inner ? dxc * rdy : 0.0, wcy = cell ? dxf * rdy : 0.0;
-    double u = UX(x, y0), v = UY(x, y0), t = TT(x, y0);
+    const double wall = last ? dxc / dxw : 0.0;  // the wall face's weight to the column's west face's
+    Sum128 su{0, 0, 1}, suu = su, inj = su, div = su, sv = su, svv = su, stt = su, flux = su;
+    Sum128 ux2 = su, uy2 = su, vx2 = su, vy2 = su, tx2 = su, ty2 = su;
+    size_t r = (size_t)y0 * nx + x;
+    double u = first ? 0.0 : LD(a.ux, a.uxl, r), v = LD(a.uy, a.uyl, r), t = LD(a.t, a.tl, r);
+#pragma unroll 1
     for (int y = y0; y < y1; ++y) {
-      const int yp = y + 1 == ny ? 0 : y + 1;
-      const double un = UX(x, yp), vn = UY(x, yp), tn = TT(x, yp);
-      const double ur = UX(x + 1, y), vl = UY(x - 1, y), tl = TT(x - 1, y);
+      const size_t rn = (y + 1 == ny ? 0 : (size_t)(y + 1) * nx) + x;
+      const double un = first ? 0.0 : LD(a.ux, a.uxl, rn), vn = LD(a.uy, a.uyl, rn), tn = LD(a.t, a.tl, rn);
+      const double ur = last ? 0.0 : LD(a.ux, a.uxl, r + 1);
+      const double vl = first ? 0.0 : LD(a.uy, a.uyl, r - 1), tl = first ? 0.5 : LD(a.t, a.tl, r - 1);
       const double dux = ur - u, dvy = vn - v, duy = un - u, dvx = v - vl, dtx = t - tl, dty = tn - t;
       // ux point i (src/logging.c:95-100, 139-144, 208-214)
-      acc[0].add(u);
-      acc[2].add(u * u);
-      acc[5].add(u * (tl + t));
+      su.add(u);
+      suu.add<true>(u * u);
+      inj.add(u * (tl + t));
       // cell centre i (src/logging.c:51-57 and its momentum and energies)
-      if (cell) {
-        const double div = p2 ? dux * rdxf + dvy * rdy : dux / dxf + dvy / dy;
-        divmax = max(divmax, div_key(div));
-        acc[7].add(div);
-        acc[1].add(v);
-        acc[3].add(v * v);
-        acc[4].add(t * t);
-      }
+      const double dv = p2 ? dux * rdxf + dvy * rdy : dux / dxf + dvy / dy;
+      divmax = max(divmax, div_key(dv));
+      div.add(dv);
+      sv.add(v);
+      svv.add<true>(v * v);
+      stt.add<true>(t * t);
       // dissipations (src/analyses.c:8-33, 35-72 and 74-110)
-      acc[6].add(((wcx * dux) * dux + (wuy * duy) * duy) + ((wfx * dvx) * dvx + (wcy * dvy) * dvy));
-      acc[8].add((wfx * dtx) * dtx + (wcy * dty) * dty);
-      if (x == 0) {  // wall heat flux (src/logging.c:195-199)
-        const double g0 = (t - tl) / a.dxc[0];
-        const double g1 = (TT(nx, y) - TT(nx - 1, y)) / a.dxc[nx];
-        acc[9].add(-(0.5 * (g0 + g1) * dy));
+      ux2.add<true>(dux * dux);
+      uy2.add<true>(duy * duy);
+      vx2.add<true>(dvx * dvx);
+      vy2.add<true>(dvy * dvy);
+      tx2.add<true>(dtx * dtx);
+      ty2.add<true>(dty * dty);
+      // wall heat flux (src/logging.c:195-199)
+      if (first) flux.add(dtx);
+      if (last) {
+        const double dtw = -0.5 - t;
+        vx2.add<true>(v * v * wall);
+        tx2.add<true>(dtw * dtw * wall);
+        flux.add(first ? dtw * wall : dtw);
       }
+      r = rn;
       u = un;
       v = vn;
       t = tn;
     }
     // the column's factors
-    auto scale = [&](int k, double f) {
-      acc[k].s *= f;
-      acc[k].c *= f;
-    };
-    const double cs_u = dxc * dy, cs_c = cell ? dxf * dy : 0.0;
-    scale(0, cs_u);
-    scale(1, cs_c);
-    scale(2, 0.5 * cs_u);
-    scale(3, 0.5 * cs_c);
-    scale(4, 0.5 * cs_c);
-    scale(5, 0.5 * q * cs_u);
-    scale(6, q * a.nu);
-    scale(8, q * a.kappa);
+    const double cs_u = dxc * dy, cs_c = dxf * dy, wfx = dy / dxc, wcy = dxf * rdy, e = q * a.nu, h = q * a.kappa;
+    acc[0] = su.pair(cs_u);
+    acc[1] = sv.pair(cs_c);
+    acc[2] = suu.pair(0.5 * cs_u);
+    acc[3] = svv.pair(0.5 * cs_c);
+    acc[4] = stt.pair(0.5 * cs_c);
+    acc[5] = inj.pair(0.5 * q * cs_u);
+    acc[6] = ux2.pair(dy * rdxf * e);
+    const Neu a1 = uy2.pair(first ? 0.0 : dxc * rdy * e), a2 = vx2.pair(wfx * e), a3 = vy2.pair(wcy * e);
+    acc[6].merge(a1.s, a1.c);
+    acc[6].merge(a2.s, a2.c);
+    acc[6].merge(a3.s, a3.c);
+    acc[7] = div.pair(1.0);
+    acc[8] = tx2.pair(wfx * h);
+    const Neu b1 = ty2.pair(wcy * h);
+    acc[8].merge(b1.s, b1.c);
+    if (first | last) acc[9] = flux.pair(-(0.5 * dy) / (first ? dxc : dxw));
   }
   // block merge: kDiagParts threads per sum, then one
   __shared__ double sh[2][kDiagSums][kDiagThreads + 1];
@@ -233,16 +324,37 @@ __global__ void __launch_bounds__(kFinishThreads) k_diag_finish(const double *pa
 
 }  // namespace
 
+namespace {
+// Rows per thread: a power of two that leaves one warp per sub-partition, since
+// one keeps the FP64 pipe busy and every thread ends with merges worth ten rows
+// or more (two per sub-partition: 400 x 512 70 against 66 us per call); at most
+// kDiagMarch (16 / 32 / 64 rows: 1024 x 2048 246 / 201 / 215, 2048 x 4096 796 /
+// 727 / 699).
+int diag_rows(int nx, int ny) {
+  const long warps1 = (long)((nx + 31) / 32) * ny;
+  int rows = 1;
+  while (rows < kDiagMarch && warps1 / (2 * rows) >= kDiagWarps) rows *= 2;
+  return rows;
+}
+dim3 diag_grid(int nx, int ny) {
+  const int rows = diag_rows(nx, ny);
+  return dim3((nx + kDiagThreads - 1) / kDiagThreads, (ny + rows - 1) / rows);
+}
+}  // namespace
+
 int diag_blocks(int nx, int ny) {
   return ((nx + 1 + kDiagThreads - 1) / kDiagThreads) * ((ny + kDiagRows - 1) / kDiagRows);
 }
 
-size_t diag_words(int nx, int ny) { return (size_t)diag_blocks(nx, ny) * (2 * kDiagSums + 1) + kDiagOut; }
+size_t diag_words(int nx, int ny) {
+  const dim3 g = diag_grid(nx, ny);
+  return (size_t)g.x * g.y * (2 * kDiagSums + 1) + kDiagOut;
+}
 
 template <typename F>
 cudaError_t launch_diag(const DiagArgs<F> &a, double *scratch, double **out, cudaStream_t st) {
-  const dim3 grid((a.nx + 1 + kDiagThreads - 1) / kDiagThreads, (a.ny + kDiagRows - 1) / kDiagRows);
-  k_diag<F><<<grid, kDiagThreads, 0, st>>>(a, scratch + kDiagOut);
+  const dim3 grid = diag_grid(a.nx, a.ny);
+  k_diag<F><<<grid, kDiagThreads, 0, st>>>(a, scratch + kDiagOut, diag_rows(a.nx, a.ny));
   k_diag_finish<<<kDiagSums + 1, kFinishThreads, 0, st>>>(scratch + kDiagOut, (int)(grid.x * grid.y), a.ly, scratch);
   *out = scratch;
   return cudaGetLastError();
