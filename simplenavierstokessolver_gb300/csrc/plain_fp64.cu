@@ -709,10 +709,12 @@ __global__ void __launch_bounds__(32) k_solve_y(int nx, int ny, const SolveYSet 
 // warm-up rows; 4 lines a block, so that the blocks' number does not leave
 // part of the SMs a block short (8 lines: 169 instead of 135 us along x).
 // Three fields of 1024 x 2048 at dt 2.6e-3 (16 warm-up rows of segments of 64):
-// 257 -> 135 us along x and 687 -> 182 along y, 70 and 60% of the FP64 issue.
+// 257 -> 135 us along x and 687 -> 182 along y, 70 and 60% of the FP64 issue;
+// with the increments, which took 39 us in launches of their own, 212 along y.
 struct SegArgs {
   PeriodicFactors f[3];
   double *q[3];
+  Increment add[3];
   int first[3];  // x: mode; y: first column
   int lgC;       // 2^lgC lines per block, at most 4
   int lgS, nseg; // 2^lgS rows per segment, segments
@@ -762,6 +764,7 @@ __global__ void __launch_bounds__(kSegThreads) k_solve_seg(int nx, int ny, const
   const PeriodicFactors &pf = fi == 0 ? a.f[0] : fi == 1 ? a.f[1] : a.f[2];
   const LineFactors f = pf.sub;
   double *q = fi == 0 ? a.q[0] : fi == 1 ? a.q[1] : a.q[2];
+  const Increment add = fi == 0 ? a.add[0] : fi == 1 ? a.add[1] : a.add[2];
   const int first = fi == 0 ? a.first[0] : fi == 1 ? a.first[1] : a.first[2];
   const int C = 1 << a.lgC, S = 1 << a.lgS, W = a.warm, lgS = a.lgS, stride = a.stride;
   const int n = COLS ? ny - 1 : nx;  // rows of the swept system
@@ -846,7 +849,41 @@ __global__ void __launch_bounds__(kSegThreads) k_solve_seg(int nx, int ny, const
   __syncthreads();
   if (live && s1 < n && !same_value(after, sm[idx(c, s1)])) bad[c] = 1;
   __syncthreads();
-  // ---- back to global memory (along y with the closure, src/linalg.c:95-107)
+  // ---- back to global memory (along y with the closure, src/linalg.c:95-107),
+  // with the field's increment where this is its last solve
+  // (src/temperature/update.c:221-226, src/fluid/update_velocity.c:436-441)
+  // the increments' loads are issued before the stores, which could alias them
+  // for the compiler: kPut elements of a thread at a time
+  constexpr int kPut = 8;
+  auto put = [&](auto &&wanted, auto &&value) {
+    const int count = COLS ? total << a.lgC : total;
+    for (int c0 = 0; c0 < (COLS ? 1 : C) && (COLS || line0 + c0 < nlines); ++c0)
+      for (int i0 = threadIdx.x; i0 < count; i0 += kPut * blockDim.x) {
+        double old[kPut];
+        size_t g[kPut];
+#pragma unroll
+        for (int j = 0; j < kPut; ++j) {
+          const int i = i0 + j * blockDim.x, cc = COLS ? i & (C - 1) : c0, e = COLS ? i >> a.lgC : i;
+          g[j] = COLS ? (size_t)e * nx + (line0 + cc) : (size_t)(line0 + cc) * nx + e;
+          if (add.out && i < count && wanted(cc, e)) old[j] = add.in[g[j]];
+        }
+#pragma unroll
+        for (int j = 0; j < kPut; ++j) {
+          const int i = i0 + j * blockDim.x, cc = COLS ? i & (C - 1) : c0, e = COLS ? i >> a.lgC : i;
+          if (i >= count || !wanted(cc, e)) continue;
+          if (add.out) {
+            add.out[g[j]] = old[j] + value(cc, e);
+          } else {
+            q[g[j]] = value(cc, e);
+          }
+        }
+      }
+  };
+  auto again = [&](double *line, size_t es) {  // a line that failed the check
+    line_again<COLS>(line, es, pf, n, COLS ? 0 : low);
+    if (add.out)
+      for (int e = COLS ? 0 : low; e < total; ++e) add.out[(line - q) + e * es] = add.in[(line - q) + e * es] + line[e * es];
+  };
   if constexpr (COLS) {
     __shared__ double last[8];
     if (threadIdx.x < C && line0 + (int)threadIdx.x < nlines) {
@@ -854,15 +891,12 @@ __global__ void __launch_bounds__(kSegThreads) k_solve_seg(int nx, int ny, const
       last[t] = (sm[idx(t, n)] - pf.u_last * sm[idx(t, 0)] - pf.l_last * sm[idx(t, n - 1)]) / pf.den;
     }
     __syncthreads();
-    each([&](int cc, int e, size_t g) {
-      if (!bad[cc]) q[g] = e == n ? last[cc] : sm[idx(cc, e)] + last[cc] * __ldg(pf.q1 + e);
-    });
-    if (k == 0 && line0 + c < nlines && bad[c]) line_again<true>(q + line0 + c, (size_t)nx, pf, n, 0);
+    put([&](int cc, int e) { return line0 + cc < nlines && !bad[cc]; },
+        [&](int cc, int e) { return e == n ? last[cc] : sm[idx(cc, e)] + last[cc] * __ldg(pf.q1 + e); });
+    if (k == 0 && line0 + c < nlines && bad[c]) again(q + line0 + c, (size_t)nx);
   } else {
-    each([&](int cc, int e, size_t g) {
-      if (!bad[cc] && e >= low) q[g] = sm[idx(cc, e)];
-    });
-    if (k == 0 && line0 + c < nlines && bad[c]) line_again<false>(q + (size_t)(line0 + c) * nx, 1, pf, n, low);
+    put([&](int cc, int e) { return !bad[cc] && e >= low; }, [&](int cc, int e) { return sm[idx(cc, e)]; });
+    if (k == 0 && line0 + c < nlines && bad[c]) again(q + (size_t)(line0 + c) * nx, 1);
   }
 }
 
@@ -1773,6 +1807,18 @@ static bool seg_shape(bool cols, int n, int total, int nl, int warm, SegArgs &a,
   return *smem <= 200 * 1024 && *threads <= kSegThreads;
 }
 
+// the increments of a set whose lines were swept serially
+static cudaError_t add_increments(const DevGrid &g, const Increment *add, const int *kind, double *const *q, int n,
+                                  cudaStream_t st) {
+  count_launches(1);
+  for (int k = 0; k < n; ++k)
+    if (add[k].out) {
+      const cudaError_t e = SNS_PLAIN_FORM::launch_add_increment(g, kind[k], add[k].in, q[k], add[k].out, st);
+      if (e != cudaSuccess) return e;
+    }
+  return cudaGetLastError();
+}
+
 cudaError_t launch_solve_x_set(const DevGrid &g, const SolveXSet &set, cudaStream_t st) {
   if (set.n < 1 || set.n > 3) return cudaErrorInvalidValue;
   SegArgs a{};
@@ -1781,6 +1827,7 @@ cudaError_t launch_solve_x_set(const DevGrid &g, const SolveXSet &set, cudaStrea
   for (int k = 0; k < set.n; ++k) {
     a.f[k].sub = set.f[k];
     a.q[k] = set.q[k];
+    a.add[k] = set.add[k];
     a.first[k] = set.mode[k];
     warm = std::max(warm, set.f[k].warm);
   }
@@ -1793,6 +1840,7 @@ cudaError_t launch_solve_x_set(const DevGrid &g, const SolveXSet &set, cudaStrea
     chain_launch(k_solve_seg<false>, dim3((g.ny + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st, g.nx, g.ny, a);
   } else {
     chain_launch(k_solve_x, dim3((g.ny + 31) / 32, set.n), 32, 0, st, g.nx, g.ny, set);
+    return add_increments(g, set.add, set.mode, set.q, set.n, st);
   }
   count_launches(1);
   return cudaGetLastError();
@@ -1806,6 +1854,7 @@ cudaError_t launch_solve_y_set(const DevGrid &g, const SolveYSet &set, cudaStrea
   for (int k = 0; k < set.n; ++k) {
     a.f[k] = set.f[k];
     a.q[k] = set.q[k];
+    a.add[k] = set.add[k];
     a.first[k] = set.first_col[k];
     warm = std::max(warm, set.f[k].sub.warm);
   }
@@ -1818,6 +1867,7 @@ cudaError_t launch_solve_y_set(const DevGrid &g, const SolveYSet &set, cudaStrea
     chain_launch(k_solve_seg<true>, dim3((g.nx + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st, g.nx, g.ny, a);
   } else {
     chain_launch(k_solve_y, dim3((g.nx + 31) / 32, set.n), 32, 0, st, g.nx, g.ny, set);
+    return add_increments(g, set.add, set.first_col, set.q, set.n, st);
   }
   count_launches(1);
   return cudaGetLastError();

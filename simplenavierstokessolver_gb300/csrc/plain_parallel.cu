@@ -461,7 +461,10 @@ __device__ __forceinline__ int cn_pos(int e, int m, int s) {
 // Rows along x (wall-bounded): one warp per row, one lane per segment; the
 // row is gathered into shared memory with each segment at a stride s = m | 1
 // (odd, so that the 32 lanes' accesses at one row fall on distinct bank
-// pairs), solved there and written back, coalesced both ways.
+// pairs), solved there and written back, coalesced both ways. FP64 issue
+// bounds it: three instructions a row and two more where the interface values
+// reach (three fields of 2048 x 4096: 357 us with the spikes over all rows, 313
+// at dt 0.035, 305 at 0.002).
 __global__ void __launch_bounds__(32 * kCnWarpsMax) k_par_cn(const ParCnArgs a) {
   chain_begin();
   extern __shared__ __align__(16) double cn_sm[];
@@ -564,37 +567,58 @@ __global__ void __launch_bounds__(32 * kCnWarpsMax) k_par_cn(const ParCnArgs a) 
   const double xe = R * __ldg(f.rD + lane);
   seg[m - 1] = xe;
   // 4) interiors: x_r = y_r + v_r x_{e(k-1)} + w_r x_{e(k)} (v = 0 in the
-  //    first segment)
+  //    first segment), where v and w reach
   const double xl = __shfl_sync(0xffffffffu, xe, (lane - 1) & 31);
+  auto spike = [&](const double *factor, double x, int r0, int r1) {
 #pragma unroll 1
-  for (int b = 0; b < m - 1; b += kParChunk) {
-    double cv[kParChunk], cw[kParChunk];
+    for (int b = r0; b < r1; b += kParChunk) {
+      double cf[kParChunk];
 #pragma unroll
-    for (int k = 0; k < kParChunk; ++k) {
-      const int r = b + k, i = r * kPartSeg + lane;
-      cv[k] = r < m - 1 ? __ldg(f.vv + i) : 0.0;
-      cw[k] = r < m - 1 ? __ldg(f.ww + i) : 0.0;
-    }
+      for (int k = 0; k < kParChunk; ++k) cf[k] = b + k < r1 ? __ldg(factor + (b + k) * kPartSeg + lane) : 0.0;
 #pragma unroll
-    for (int k = 0; k < kParChunk; ++k) {
-      const int r = b + k;
-      if (r < m - 1) seg[r] = fma(cw[k], xe, fma(cv[k], xl, seg[r]));
+      for (int k = 0; k < kParChunk; ++k)
+        if (b + k < r1) seg[b + k] = fma(cf[k], x, seg[b + k]);
     }
-  }
+  };
+  spike(f.vv, xl, 0, min(F.nv, m - 1));
+  spike(f.ww, xe, max(m - 1 - F.nw, 0), m - 1);
   __syncwarp();
-  double *dstq = F.q + (size_t)line * a.ls;
-  for (int e = lane; e < n; e += 32) dstq[e] = sl[cn_pos(e, m, s)];
+  const size_t g0 = (size_t)line * a.ls;
+  if (F.add.out) {
+    for (int e0 = lane; e0 < n; e0 += 32 * kCnLoad) {
+      double old[kCnLoad];
+#pragma unroll
+      for (int k = 0; k < kCnLoad; ++k)
+        if (e0 + 32 * k < n) old[k] = F.add.in[g0 + e0 + 32 * k];
+#pragma unroll
+      for (int k = 0; k < kCnLoad; ++k) {
+        const int e = e0 + 32 * k;
+        if (e < n && e >= F.low) F.add.out[g0 + e] = old[k] + sl[cn_pos(e, m, s)];
+      }
+    }
+  } else {
+    for (int e = lane; e < n; e += 32) F.q[g0 + e] = sl[cn_pos(e, m, s)];
+  }
 }
 
 // Columns along y (periodic): a block takes kCnCols adjacent columns and
 // all 32 segments of each, thread t column t % kCnCols and segment
 // t / kCnCols, and walks its segment in place in global memory; a warp's
-// access covers 8 rows of kCnCols columns (whole 32-byte sectors). The
+// access covers 4 rows of kCnCols columns (whole 64-byte pairs of sectors). The
 // first interior values, the interface right-hand sides and the interface
 // solutions pass between the threads of a column through shared memory;
 // warp c solves column c's cyclic interface system with lane = segment.
 // Same operations on every element as k_par_cn.
-constexpr int kCnCols = 4;
+//
+// Memory traffic bounds it at 2048 x 4096 (three fields of 67 MB, larger than
+// L2 together), so a row is read and written twice: once going forward, once
+// going back, where it takes its increment unless an interface value reaches it
+// (ParCnField::nv, nw). Solve and increments, us: in 4 columns per block, the
+// spikes over all rows and the increments in launches of their own 371 + 110,
+// now 384; 1024 x 2048 111 + 33, now 95; 512 x 1024 53 + 12, now 47. (4 / 16
+// columns with the rest as it is: 2048 x 4096 466 / 565, 1024 x 2048 100 / 173;
+// chunks of 12 or 16 rows instead of kParChunk: 2048 x 4096 513.)
+constexpr int kCnCols = 8;
 
 __global__ void __launch_bounds__(32 * kCnCols) k_par_cn_cols(const ParCnArgs a) {
   chain_begin();
@@ -606,6 +630,9 @@ __global__ void __launch_bounds__(32 * kCnCols) k_par_cn_cols(const ParCnArgs a)
   const bool live = col < a.lines;
   const size_t es = (size_t)a.es;
   double *q = F.q + (live ? col : 0);
+  const double *in = F.add.out ? F.add.in + (live ? col : 0) : nullptr;
+  double *out = F.add.out ? F.add.out + (live ? col : 0) : q;
+  const int mid0 = min(F.nv, m - 1), mid1 = max(m - 1 - F.nw, mid0);  // at most m - 2 (nw >= 1)
   const CnFac f(F.fac, n);
   const size_t e0 = (size_t)k * m;  // first row of the segment
   double y = 0.0, ylast = 0.0;
@@ -613,18 +640,41 @@ __global__ void __launch_bounds__(32 * kCnCols) k_par_cn_cols(const ParCnArgs a)
     // 1) interior rows r = 0 .. m-2: forward elimination, back substitution
     y = q[e0 * es] * __ldg(f.inv + k);
     q[e0 * es] = y;
-#pragma unroll 4
-    for (int r = 1; r < m - 1; ++r) {
-      const size_t o = (e0 + r) * es;
-      y = fma(-__ldg(f.gg + r * kPartSeg + k), y, __ldg(f.inv + r * kPartSeg + k) * q[o]);
-      q[o] = y;
+#pragma unroll 1
+    for (int b = 1; b < m - 1; b += kParChunk) {
+      double q_[kParChunk];
+#pragma unroll
+      for (int j = 0; j < kParChunk; ++j) q_[j] = b + j < m - 1 ? q[(e0 + b + j) * es] : 0.0;
+#pragma unroll
+      for (int j = 0; j < kParChunk; ++j) {
+        const int r = b + j;
+        if (r >= m - 1) break;
+        y = fma(-__ldg(f.gg + r * kPartSeg + k), y, __ldg(f.inv + r * kPartSeg + k) * q_[j]);
+        q[(e0 + r) * es] = y;
+      }
     }
     ylast = y;
-#pragma unroll 4
-    for (int r = m - 3; r >= 0; --r) {
-      const size_t o = (e0 + r) * es;
-      y = fma(-__ldg(f.up + r * kPartSeg + k), y, q[o]);
-      q[o] = y;
+    // rows that no interface value reaches are final now
+#pragma unroll 1
+    for (int b = m - 3; b >= 0; b -= kParChunk) {
+      double y_[kParChunk], old[kParChunk];
+#pragma unroll
+      for (int j = 0; j < kParChunk; ++j) {
+        const int r = b - j;
+        y_[j] = r >= 0 ? q[(e0 + r) * es] : 0.0;
+        old[j] = in && r >= mid0 && r < mid1 ? in[(e0 + r) * es] : 0.0;
+      }
+#pragma unroll
+      for (int j = 0; j < kParChunk; ++j) {
+        const int r = b - j;
+        if (r < 0) break;
+        y = fma(-__ldg(f.up + r * kPartSeg + k), y, y_[j]);
+        if (r >= mid0 && r < mid1) {
+          out[(e0 + r) * es] = in ? old[j] + y : y;
+        } else {
+          q[(e0 + r) * es] = y;
+        }
+      }
     }
   }
   ex[0][c][k] = y;  // the segment's first interior value
@@ -654,11 +704,30 @@ __global__ void __launch_bounds__(32 * kCnCols) k_par_cn_cols(const ParCnArgs a)
   if (!live) return;
   // 4) interiors from the spikes
   const double xe = ex[2][c][k], xl = ex[2][c][(k - 1) & 31];
-  q[(e0 + m - 1) * es] = xe;
-#pragma unroll 4
-  for (int r = 0; r < m - 1; ++r) {
-    const size_t o = (e0 + r) * es;
-    q[o] = fma(__ldg(f.ww + r * kPartSeg + k), xe, fma(__ldg(f.vv + r * kPartSeg + k), xl, q[o]));
+  // the others in order, loads before the stores, which could alias them for
+  // the compiler
+  const int gap = max(mid1 - mid0, 0);
+#pragma unroll 1
+  for (int b = 0; b < m - gap; b += kParChunk) {
+    double y_[kParChunk], old[kParChunk];
+#pragma unroll
+    for (int j = 0; j < kParChunk; ++j) {
+      const int r = b + j < mid0 ? b + j : b + j + gap;
+      y_[j] = r < m - 1 ? q[(e0 + r) * es] : 0.0;
+      old[j] = in && r < m ? in[(e0 + r) * es] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kParChunk; ++j) {
+      const int r = b + j < mid0 ? b + j : b + j + gap;
+      if (r >= m) break;
+      double v = xe;
+      if (r < m - 1) {
+        v = y_[j];
+        if (r < F.nv) v = fma(__ldg(f.vv + r * kPartSeg + k), xl, v);
+        if (r >= m - 1 - F.nw) v = fma(__ldg(f.ww + r * kPartSeg + k), xe, v);
+      }
+      out[(e0 + r) * es] = in ? old[j] + v : v;
+    }
   }
 }
 

@@ -103,17 +103,24 @@ struct TempFields {
 
 // ------------------------------------------------------------ launch types
 // up to three independent fields (temperature, ux, uy) in one launch: their
-// serial sweeps run side by side
+// serial sweeps run side by side; with add.out the solution becomes the
+// field's increment, out = in + solution, as it is written (q is scratch then)
+struct Increment {
+  const double *in = nullptr;
+  double *out = nullptr;
+};
 struct SolveXSet {
   LineFactors f[3];
   int mode[3];
   double *q[3];
+  Increment add[3];
   int n;
 };
 struct SolveYSet {
   PeriodicFactors f[3];
   int first_col[3];
   double *q[3];
+  Increment add[3];
   int n;
 };
 // strided field copies in one launch (host arrays are pinned and read or
@@ -194,6 +201,11 @@ struct ParCnField {
   double *q = nullptr;
   const double *fac = nullptr;
   int first = 0;
+  Increment add{};
+  int low = 0;              // first row of a line that takes its increment
+  // rows of a segment that the interface values at its start and at its end
+  // reach (v and w of the others are below 2^-80)
+  int nv = 1 << 30, nw = 1 << 30;
 };
 struct ParCnArgs {
   ParCnField f[3];
