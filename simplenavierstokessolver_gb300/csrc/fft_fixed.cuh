@@ -19,15 +19,15 @@
 // Accuracy: products and shifts are rounded at 2^-59 or less of the column's
 // largest value of the pass. Over transforms of 8 to 4096 complex values the
 // error is 0.2 to 0.6 of that of the FP64 transform it replaces (0.7 for
-// delta columns of 8192 rows inverted), for noise, smooth, single-mode, delta
+// delta columns of 8192 rows and, with radix 2, 64 rows inverted), for noise, smooth, single-mode, delta
 // and wide-range columns (tests/test_fft_fixed.py measures both against an
 // extended-precision DFT).
 //
-// Stockham passes of radix V = 8 or 4 (then one of radix 4 or 2), V values per
+// Stockham passes of radix V = 8, 4 or 2 (then one of radix 4 or 2), V values per
 // thread: thread t of a block handles column t mod C, group t / C of M / V. The
 // radix-8 form moves the data through shared memory fewer times, the radix-4
-// form has twice the warps, each with half the instructions (a rule and both
-// sides' times where the forms are launched).
+// and radix-2 forms have two and four times the warps, each with fewer
+// instructions (rules and both sides' times where the forms are launched).
 // Shared memory holds element i of column c at c stride + i + i / 8 (elements
 // of 16 bytes; one of padding per 8 spreads each pass's accesses over all
 // banks, the columns' stride the lanes of different columns).

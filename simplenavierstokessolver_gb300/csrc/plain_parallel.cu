@@ -792,7 +792,14 @@ void par_dft_attributes() {
 // (the FP64 radix-8 pair: 22.4 / 19.9 at 128 x 256, 45 / 30 at 512 x 1024,
 // 410 / 364 at 2048 x 4096). Columns per block 1, 2, 4: within 5% at 512 x 1024,
 // 2 the best from 256 x 512 to 1024 x 2048.
+// 2 values per thread (radix 2, more passes of half the work and half as many
+// values to load and to write) for short columns on small grids, us per step
+// with 4 against 2: 64 x 64 101 / 95, 128 x 256 119 / 111, 256 x 256 128 / 122,
+// but 512 x 256 146 / 147, 128 x 512 127 / 133, 64 x 1024 144 / 163 (a column's
+// threads meet at every pass).
 constexpr long kFix8Warps = 1024;
+constexpr long kFix2Warps = 512;  // of 4 values
+constexpr int kFix2Rows = 256;
 constexpr int kFixLg = 1;
 struct FixShape {
   int v, lgC, threads;
@@ -800,7 +807,9 @@ struct FixShape {
 };
 FixShape fix_shape(const DevGrid &g) {
   FixShape f;
-  f.v = (long)g.nx * (g.ny / 16) / 32 >= kFix8Warps || g.ny > 4096 ? 8 : 4;
+  f.v = (long)g.nx * (g.ny / 16) / 32 >= kFix8Warps || g.ny > 4096            ? 8
+        : (long)g.nx * (g.ny / 8) / 32 < kFix2Warps && g.ny <= kFix2Rows ? 2
+                                                                         : 4;
   f.lgC = kFixLg;
   const int n = g.ny / 2 / f.v;
   while (f.lgC < 4 && (n << f.lgC) < 32) f.lgC++;
@@ -819,6 +828,7 @@ cudaError_t launch_par_fwd(const DevGrid &g, const StageScalars &s, const double
     const FixArgs a{g, ux, uy, spec, nullptr, 0.0, f.lgC, g.nx / kPartSeg};
     const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
     if (f.v == 8) chain_launch(k_par_fwd_fx<8>, blocks, f.threads, f.smem, st, a);
+    else if (f.v == 2) chain_launch(k_par_fwd_fx<2>, blocks, f.threads, f.smem, st, a);
     else chain_launch(k_par_fwd_fx<4>, blocks, f.threads, f.smem, st, a);
   } else {
     const int C = par_cols(g);
@@ -897,6 +907,7 @@ cudaError_t launch_par_bwd(const DevGrid &g, const StageScalars &s, const double
                     f.lgC, g.nx / kPartSeg};
     const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
     if (f.v == 8) chain_launch(k_par_bwd_fx<8>, blocks, f.threads, f.smem, st, a);
+    else if (f.v == 2) chain_launch(k_par_bwd_fx<2>, blocks, f.threads, f.smem, st, a);
     else chain_launch(k_par_bwd_fx<4>, blocks, f.threads, f.smem, st, a);
   } else {
     const int C = par_cols(g);

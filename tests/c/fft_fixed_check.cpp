@@ -1,7 +1,8 @@
 // The fixed-point real DFT (csrc/fft_fixed.cuh) run on the CPU: the kernels'
 // own arithmetic (quantisation, passes, shifts, split steps, conversions) in
 // their order, one column at a time, against a DFT in long double, beside the
-// FP64 radix-8 transform it stands for (the same passes in double). For each
+// FP64 radix-8 transform it stands for (the same passes in double). With an
+// argument: passes of radix 2, to jtot 256. For each
 // length and kind of column prints: jtot, kind, forward error of the fixed
 // and of the FP64 transform, inverse errors of both (relative 2-norms).
 #include <cstdio>
@@ -41,9 +42,11 @@ static void pass_fixed(std::vector<C64> &z, int M, int Ns, int &S, unsigned &m) 
   }
   z.swap(o);
 }
+static bool radix2;  // two values per thread: passes of radix 2
 template <bool FWD>
 static void fixed_fft(std::vector<C64> &z, int M, int &S, unsigned &m) {
   int Ns = 1, rem = M;
+  for (; radix2 && rem >= 2; rem >>= 1, Ns <<= 1) pass_fixed<2, FWD>(z, M, Ns, S, m);
   for (; rem >= 8; rem >>= 3, Ns <<= 3) pass_fixed<8, FWD>(z, M, Ns, S, m);
   if (rem == 4) pass_fixed<4, FWD>(z, M, Ns, S, m);
   if (rem == 2) pass_fixed<2, FWD>(z, M, Ns, S, m);
@@ -185,10 +188,11 @@ static void dft_ld(std::vector<cl> &z, int sign) {
   }
 }
 
-int main() {
+int main(int argc, char **) {
+  radix2 = argc > 1;
   std::mt19937_64 g(7);
   std::uniform_real_distribution<double> U(-1, 1);
-  for (int n = 16; n <= 8192; n *= 2) {
+  for (int n = 16; n <= (radix2 ? 256 : 8192); n *= 2) {
     const int M = n / 2;
     const std::vector<int32_t> t = fixed_twiddles(n);
     tw.resize(n);

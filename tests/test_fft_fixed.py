@@ -13,9 +13,11 @@ import pytest
 ROOT = pathlib.Path(__file__).resolve().parents[1]
 
 
-def test_error_is_below_the_fp64_transforms(tmp_path):
-    """forward and inverse, jtot 16 to 8192, noise, smooth, single-mode, delta,
-    wide-range and mean-dominated columns of sizes from 2^-960 to 2^100"""
+@pytest.mark.parametrize("args,lengths", [([], 10), (["2"], 5)], ids=["radix8", "radix2"])
+def test_error_is_below_the_fp64_transforms(tmp_path, args, lengths):
+    """forward and inverse, jtot 16 to 8192 (256 with radix 2), noise, smooth,
+    single-mode, delta, wide-range and mean-dominated columns of sizes from
+    2^-960 to 2^100"""
     cxx = shutil.which("g++")
     if cxx is None:
         pytest.skip("no g++")
@@ -24,8 +26,8 @@ def test_error_is_below_the_fp64_transforms(tmp_path):
                     str(ROOT / "simplenavierstokessolver_gb300" / "csrc"),
                     str(ROOT / "tests" / "c" / "fft_fixed_check.cpp"), "-o", str(exe)], check=True)
     rows = [line.split() for line in
-            subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.splitlines()]
-    assert len(rows) == 10 * 6
+            subprocess.run([str(exe), *args], check=True, capture_output=True, text=True).stdout.splitlines()]
+    assert len(rows) == lengths * 6
     for jtot, kind, fwd, fwd64, inv, inv64 in rows:
         assert float(fwd) <= float(fwd64) and float(inv) <= float(inv64), (jtot, kind, fwd, fwd64, inv, inv64)
 
