@@ -111,6 +111,61 @@ struct Mul {
   }
 };
 
+// ------------------------------------------------- additions in the integer unit
+// RN(a + b) of normal numbers (or zeros) with integer instructions. An FP64
+// addition holds a sub-partition's pipe for ~65 to 80 cycles; these ~37
+// instructions (and ~13 per operand, shared by the sums that it enters) take
+// about as long in the integer pipes, beside it. Measured with 4 warps a
+// sub-partition: 24 FP64 operations 1540 cycles a warp, 16 and 8 of these 1240.
+//
+// An operand is m 2^(e - 1084), m signed with its 53 bits from bit 9 up, z the
+// zeros below its lowest one bit (or fewer): the sum is formed at the larger
+// exponent, the other operand shifted down with its lost bits, if any, marked
+// in the last bit. That is at least 6 bits below the result's last one after
+// normalisation (bits are lost only by a shift of more than 9, which leaves at
+// most two leading zeros more), so rounding to nearest, ties to even, sees the
+// exact sum.
+struct Num {
+  long long m;
+  int e, z;
+};
+__device__ __forceinline__ long long shr_s64(long long v, int s) {  // amounts of 64 and more leave the sign
+  long long r;
+  asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+  return r;
+}
+__device__ __forceinline__ Num num(double d) {
+  const int hi = __double2hiint(d);
+  const int e = (hi >> 20) & 0x7ff;
+  long long m = (long long)(((unsigned long long)((hi & 0xfffff) | (e ? 1 << 20 : 0)) << 32 |
+                             (unsigned)__double2loint(d))
+                            << 9);
+  const long long n = (long long)(hi >> 31);
+  m = (m ^ n) - n;
+  const unsigned ml = (unsigned)m, mh = (unsigned)(m >> 32);
+  return Num{m, e, ml ? __ffs(ml) - 1 : 31 + __ffs(mh)};
+}
+// zero, or normal and far enough from the ends of the range for every result
+__device__ __forceinline__ bool in_range(const Num &a) { return a.m == 0 || (unsigned)(a.e - 128) < 1792u; }
+__device__ __forceinline__ double round_sum(long long s, int e) {
+  const long long n = s >> 63;
+  const unsigned long long a = (unsigned long long)((s ^ n) - n);
+  const int lz = __clzll((long long)a);  // 1 or more
+  unsigned long long m = a << ((lz - 1) & 63);
+  m += 0x1ff + ((m >> 10) & 1);
+  const unsigned long long q = m >> 10;  // 53 bits, or 2^53
+  const unsigned hi = ((unsigned)(q >> 32) + ((unsigned)(e + 1 - lz) << 20)) | ((unsigned)n & 0x80000000u);
+  return a ? __hiloint2double((int)hi, (int)(unsigned)q) : 0.0;
+}
+// a + b or a - b, times 2^x
+template <bool SUB>
+__device__ __forceinline__ double num_sum(const Num &a, const Num &b, int x = 0) {
+  const int e = max(a.e, b.e), sa = e - a.e, sb = e - b.e;
+  const long long ta = shr_s64(a.m, sa) | (sa > a.z), tb = shr_s64(b.m, sb) | (sb > b.z);
+  return round_sum(SUB ? ta - tb : ta + tb, e + x);
+}
+__device__ __forceinline__ Num scaled(const Num &a, int field) { return Num{a.m, a.e + (field >> 20), a.z}; }
+
 // what a row's divisions by the spacings use: (d) the spacing, (r) its
 // reciprocal, (l) the pair's low word, (e) the exponent of a power of two
 struct Spacing {
@@ -292,6 +347,12 @@ struct VelIn {
   double u0n, u1n, v0n, vln, vr, pc, ul, pl, tfl, tfr, aux, auy;
 };
 
+// the velocities that enter several sums, as integers (FAST)
+struct VelNum {
+  Num u0, u1, um0, um1, v0, vl;
+  Num ul, u0n, v0n, vln, vr, pc, pl, pm;
+};
+
 struct VelOut {
   double ux, ax, qx, uy, ay, qy;
   double gym_u, pym_u, gym_v, pym_v;
@@ -301,9 +362,24 @@ struct VelOut {
 // :219-230 / :371-381 (RK3 increments) and :436-441 / :580-585 (update), for
 // one row of column x. Returns false when a FAST product was out of range.
 template <int IMPX, int IMPY, bool RCP, bool FAST>
-__device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const VelIn &in, bool has_ux,
-                                        VelOut &o) {
+__device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const VelIn &in, const VelNum &n,
+                                        bool has_ux, VelOut &o) {
   Mul<FAST> m;
+  // x - y and (x + y) 2^e
+  auto Sub = [&](double x, double y, const Num &nx, const Num &ny) {
+    if constexpr (FAST) {
+      return num_sum<true>(nx, ny);
+    } else {
+      return x - y;
+    }
+  };
+  auto Mean = [&](double x, double y, const Num &nx, const Num &ny) {
+    if constexpr (FAST) {
+      return num_sum<false>(nx, ny, -1);
+    } else {
+      return 0.5 * x + 0.5 * y;
+    }
+  };
   const double nu = a.s.nu;
   // difference / spacing
   auto D = [&](double v, const Spacing &s) { return over<RCP, FAST>(m, v, s); };
@@ -319,17 +395,22 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
   o.pym_u = in.pym_u;
   // ---- ux(i, j), i = x+1 >= 2
   if (has_ux) {
-    const double gxm = D(in.u0 - in.ul, k.f_m);
-    const double gxp = D(in.u1 - in.u0, k.f);
-    const double gyp = D(in.u0n - in.u0, k.y);
-    const double vxm = m.half(in.ul) + m.half(in.u0);
-    const double vxp = m.half(in.u0) + m.half(in.u1);
+    const double gxm = D(Sub(in.u0, in.ul, n.u0, n.ul), k.f_m);
+    const double gxp = D(Sub(in.u1, in.u0, n.u1, n.u0), k.f);
+    const double gyp = D(Sub(in.u0n, in.u0, n.u0n, n.u0), k.y);
+    const double vxm = Mean(in.ul, in.u0, n.ul, n.u0);
+    const double vxp = Mean(in.u0, in.u1, n.u0, n.u1);
     const double adv1 = -(C(k.fm, vxm, k.e_fm) * gxm) - (C(k.fp, vxp, k.e_fp) * gxp);
-    const double pyp = m.half(C(k.fm, in.vln, k.e_fm) + C(k.fp, in.v0n, k.e_fp)) * gyp;
+    double pyp;
+    if constexpr (FAST && RCP) {
+      pyp = num_sum<false>(scaled(n.vln, k.e_fm), scaled(n.v0n, k.e_fp), -1) * gyp;
+    } else {
+      pyp = m.half(C(k.fm, in.vln, k.e_fm) + C(k.fp, in.v0n, k.e_fp)) * gyp;
+    }
     const double adv2 = -in.pym_u - pyp;
     const double dif1 = D(nu * (gxp - gxm), k.c);
     const double dif2 = D(nu * (gyp - in.gym_u), k.y);
-    const double pre = -D(in.pc - in.pl, k.c);
+    const double pre = -D(Sub(in.pc, in.pl, n.pc, n.pl), k.c);
     double A = adv1 + adv2;
     if (!IMPX) A = A + dif1;
     if (!IMPY) A = A + dif2;
@@ -355,17 +436,17 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
   }
   // ---- uy(i, j), i = x+1 >= 1
   {
-    const double gxm = D(in.v0 - in.vl, k.c);
-    const double gxp = D(in.vr - in.v0, k.c_p);
-    const double gyp = D(in.v0n - in.v0, k.y);
-    const double wxm = m.half(in.um0) + m.half(in.u0);
-    const double wxp = m.half(in.um1) + m.half(in.u1);
+    const double gxm = D(Sub(in.v0, in.vl, n.v0, n.vl), k.c);
+    const double gxp = D(Sub(in.vr, in.v0, n.vr, n.v0), k.c_p);
+    const double gyp = D(Sub(in.v0n, in.v0, n.v0n, n.v0), k.y);
+    const double wxm = Mean(in.um0, in.u0, n.um0, n.u0);
+    const double wxp = Mean(in.um1, in.u1, n.um1, n.u1);
     const double adv1 = -(C(k.cm, wxm, k.e_cm) * gxm) - (C(k.cp, wxp, k.e_cp) * gxp);
-    const double pyp = m.half(m.half(in.v0) + m.half(in.v0n)) * gyp;
+    const double pyp = m.half(Mean(in.v0, in.v0n, n.v0, n.v0n)) * gyp;
     const double adv2 = -in.pym_v - pyp;
     const double dif1 = D(nu * (gxp - gxm), k.f);
     const double dif2 = D(nu * (gyp - in.gym_v), k.y);
-    const double pre = -D(in.pc - in.pm, k.y);
+    const double pre = -D(Sub(in.pc, in.pm, n.pc, n.pm), k.y);
     double A = adv1 + adv2;
     if (!IMPX) A = A + dif1;
     if (!IMPY) A = A + dif2;
@@ -437,6 +518,18 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
   in.gym_v = over_checked<RCP, FAST>(in.v0 - vm, k.y);
   in.pym_v = (0.5 * (0.5 * vm + 0.5 * in.v0)) * in.gym_v;
   in.ul = in.pl = in.tfl = in.tfr = in.aux = in.auy = 0.0;
+  VelNum n{};
+  bool ok1 = true, ok2 = true;  // of the values loaded one and two rows below
+  if constexpr (FAST) {
+    n.u0 = num(in.u0);
+    n.u1 = num(in.u1);
+    n.um0 = num(in.um0);
+    n.um1 = num(in.um1);
+    n.v0 = num(in.v0);
+    n.vl = num(in.vl);
+    n.pm = num(in.pm);
+    ok1 = in_range(n.pm) & in_range(n.u0) & in_range(n.u1) & in_range(n.um0) & in_range(n.um1) & in_range(n.v0) & in_range(n.vl);
+  }
 
   for (int y = y0; y < y1; ++y) {
     const int yp = wrap_up(y, ny);
@@ -459,10 +552,29 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
     if (a.s.has_b) in.auy = a.auy[r];
     VelOut o;
     if constexpr (FAST) {
-      if (!vel_row<IMPX, IMPY, RCP, true>(a, k, in, has_ux, o) || k.bad)
-        vel_row<IMPX, IMPY, RCP, false>(a, k, in, has_ux, o);
+      n.ul = num(in.ul);
+      n.u0n = num(in.u0n);
+      n.v0n = num(in.v0n);
+      n.vln = num(in.vln);
+      n.vr = num(in.vr);
+      n.pc = num(in.pc);
+      n.pl = num(in.pl);
+      const Num u1n = num(in.u1n);
+      const bool ok = in_range(n.ul) & in_range(n.u0n) & in_range(n.v0n) & in_range(n.vln) & in_range(n.vr) &
+                      in_range(u1n) & in_range(n.pc) & in_range(n.pl);
+      if (!vel_row<IMPX, IMPY, RCP, true>(a, k, in, n, has_ux, o) || k.bad || !(ok & ok1 & ok2))
+        vel_row<IMPX, IMPY, RCP, false>(a, k, in, n, has_ux, o);
+      ok2 = ok1;
+      ok1 = ok;
+      n.um0 = n.u0;
+      n.um1 = n.u1;
+      n.u0 = n.u0n;
+      n.u1 = u1n;
+      n.v0 = n.v0n;
+      n.vl = n.vln;
+      n.pm = n.pc;
     } else {
-      vel_row<IMPX, IMPY, RCP, false>(a, k, in, has_ux, o);
+      vel_row<IMPX, IMPY, RCP, false>(a, k, in, n, has_ux, o);
     }
     if (has_ux) {
       a.aux[r] = o.ax;
@@ -503,8 +615,14 @@ __global__ void __launch_bounds__(128) k_temp(const TempArgs a, int rows) {
   temp_column<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
 }
 
+// FP64 issue bounds it (52 instructions a cell on grids of powers of two, 15 of
+// them sums taken in the integer unit). 128 registers, so that 8 blocks fit an
+// SM (170 without the bound: 5, slower than no integer sums at all). Velocity
+// update, us, before the integer sums / with 13 of them / with the pressure's
+// two: 256 x 512 20.8 / 18.9 / 18.9, 400 x 512 45.4 / 41.4 / 41.3, 512 x 1024
+// 61.8 / 53.4 / 53.5, 1024 x 2048 237 / 188 / 183, 2048 x 4096 867 / 685 / 664.
 template <int IMPX, int IMPY, bool RCP, bool FAST>
-__global__ void __launch_bounds__(128) k_vel(const VelArgs a, int rows) {
+__global__ void __launch_bounds__(kBlockX, 8) k_vel(const VelArgs a, int rows) {
   chain_begin();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.g.nx) return;
