@@ -365,7 +365,7 @@ struct VelIn {
   double u0n, u1n, v0n, vln, vr, pc, ul, pl, tfl, tfr, aux, auy;
 };
 
-// the velocities that enter several sums, as integers (FAST)
+// the values that enter the row's sums, as integers (INT)
 struct VelNum {
   Num u0, u1, um0, um1, v0, vl;
   Num ul, u0n, v0n, vln, vr, pc, pl, pm;
@@ -379,23 +379,23 @@ struct VelOut {
 // src/fluid/update_velocity.c:11-104 (ux sources), :106-192 (uy sources),
 // :219-230 / :371-381 (RK3 increments) and :436-441 / :580-585 (update), for
 // one row of column x. Returns false when a FAST product was out of range.
-template <int IMPX, int IMPY, bool RCP, bool FAST>
+template <int IMPX, int IMPY, bool RCP, bool FAST, bool INT>
 __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const VelIn &in, const VelNum &n,
                                         bool has_ux, VelOut &o) {
   Mul<FAST> m;
   // x - y and (x + y) 2^e
   auto Sub = [&](double x, double y, const Num &nx, const Num &ny) {
-    if constexpr (FAST) {
+    if constexpr (INT) {
       return num_sum<true>(nx, ny);
     } else {
       return x - y;
     }
   };
   auto Mean = [&](double x, double y, const Num &nx, const Num &ny) {
-    if constexpr (FAST) {
+    if constexpr (INT) {
       return num_sum<false>(nx, ny, -1);
     } else {
-      return 0.5 * x + 0.5 * y;
+      return m.half(x) + m.half(y);
     }
   };
   const double nu = a.s.nu;
@@ -420,7 +420,7 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
     const double vxp = Mean(in.u0, in.u1, n.u0, n.u1);
     const double adv1 = -(C(k.fm, vxm, k.e_fm) * gxm) - (C(k.fp, vxp, k.e_fp) * gxp);
     double pyp;
-    if constexpr (FAST && RCP) {
+    if constexpr (INT && RCP) {
       pyp = num_sum<false>(scaled(n.vln, k.e_fm), scaled(n.v0n, k.e_fp), -1) * gyp;
     } else {
       pyp = m.half(C(k.fm, in.vln, k.e_fm) + C(k.fp, in.v0n, k.e_fp)) * gyp;
@@ -491,7 +491,7 @@ __device__ __forceinline__ bool vel_row(const VelArgs &a, const VelCol &k, const
 }
 
 // column x, rows y0 .. y0+rows-1
-template <int IMPX, int IMPY, bool RCP, bool FAST>
+template <int IMPX, int IMPY, bool RCP, bool FAST, bool INT>
 __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int rows) {
   const int nx = a.g.nx, ny = a.g.ny;
   const int y1 = min(y0 + rows, ny);
@@ -538,7 +538,7 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
   in.ul = in.pl = in.tfl = in.tfr = in.aux = in.auy = 0.0;
   VelNum n{};
   bool ok1 = true, ok2 = true;  // of the values loaded one and two rows below
-  if constexpr (FAST) {
+  if constexpr (INT) {
     n.u0 = num(in.u0);
     n.u1 = num(in.u1);
     n.um0 = num(in.um0);
@@ -569,7 +569,9 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
     }
     if (a.s.has_b) in.auy = a.auy[r];
     VelOut o;
-    if constexpr (FAST) {
+    bool ok = true;
+    [[maybe_unused]] Num u1n{};
+    if constexpr (INT) {
       n.ul = num(in.ul);
       n.u0n = num(in.u0n);
       n.v0n = num(in.v0n);
@@ -577,11 +579,17 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
       n.vr = num(in.vr);
       n.pc = num(in.pc);
       n.pl = num(in.pl);
-      const Num u1n = num(in.u1n);
-      const bool ok = in_range(n.ul) & in_range(n.u0n) & in_range(n.v0n) & in_range(n.vln) & in_range(n.vr) &
-                      in_range(u1n) & in_range(n.pc) & in_range(n.pl);
-      if (!vel_row<IMPX, IMPY, RCP, true>(a, k, in, n, has_ux, o) || k.bad || !(ok & ok1 & ok2))
-        vel_row<IMPX, IMPY, RCP, false>(a, k, in, n, has_ux, o);
+      u1n = num(in.u1n);
+      ok = in_range(n.ul) & in_range(n.u0n) & in_range(n.v0n) & in_range(n.vln) & in_range(n.vr) & in_range(u1n) &
+           in_range(n.pc) & in_range(n.pl);
+    }
+    if constexpr (FAST) {
+      if (!vel_row<IMPX, IMPY, RCP, true, INT>(a, k, in, n, has_ux, o) || k.bad || !(ok & ok1 & ok2))
+        vel_row<IMPX, IMPY, RCP, false, false>(a, k, in, n, has_ux, o);
+    } else {
+      vel_row<IMPX, IMPY, RCP, false, false>(a, k, in, n, has_ux, o);
+    }
+    if constexpr (INT) {
       ok2 = ok1;
       ok1 = ok;
       n.um0 = n.u0;
@@ -591,8 +599,6 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
       n.v0 = n.v0n;
       n.vl = n.vln;
       n.pm = n.pc;
-    } else {
-      vel_row<IMPX, IMPY, RCP, false>(a, k, in, n, has_ux, o);
     }
     if (has_ux) {
       a.aux[r] = o.ax;
@@ -642,12 +648,12 @@ __global__ void __launch_bounds__(128) k_temp(const TempArgs a, int rows) {
 // update, us, before the integer sums / with 13 of them / with the pressure's
 // two: 256 x 512 20.8 / 18.9 / 18.9, 400 x 512 45.4 / 41.4 / 41.3, 512 x 1024
 // 61.8 / 53.4 / 53.5, 1024 x 2048 237 / 188 / 183, 2048 x 4096 867 / 685 / 664.
-template <int IMPX, int IMPY, bool RCP, bool FAST>
+template <int IMPX, int IMPY, bool RCP, bool FAST, bool INT>
 __global__ void __launch_bounds__(kBlockX, 8) k_vel(const VelArgs a, int rows) {
   chain_begin();
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   if (x >= a.g.nx) return;
-  vel_march<IMPX, IMPY, RCP, FAST>(a, x, blockIdx.y * rows, rows);
+  vel_march<IMPX, IMPY, RCP, FAST, INT>(a, x, blockIdx.y * rows, rows);
 }
 #endif
 
@@ -1827,6 +1833,11 @@ dim3 march_grid(const DevGrid &g, int rows) {
   return dim3((g.nx + kBlockX - 1) / kBlockX, (g.ny + rows - 1) / rows);
 }
 
+// integer sums in the velocity update from this many rows a thread on: with one
+// row a warp's instruction latency is the launch's, and they are the longer way
+// (64 x 128 8.4 us without, 9.9 with; 100 x 128 10.5 / 12.3; with two rows
+// 256 x 512 20.8 / 19.1, with eight 512 x 1024 61.7 / 53.4)
+constexpr int kIntRows = 2;
 // Rows marched by a thread of the velocity and temperature updates. Fewer
 // rows form more y-faces twice (2 to 9 FP64 instructions a thread) but give
 // more warps; a sub-partition issues an FP64 instruction every ~70 cycles from
@@ -1928,7 +1939,11 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
   }
 #undef SNS_F
 #else
-#define SNS_V(X, Y, R, F) chain_launch(k_vel<X, Y, R, F>, grid, block, 0, st, a, rows)
+#define SNS_V(X, Y, R, F)                                                                    \
+  do {                                                                                       \
+    if (F && rows >= kIntRows) chain_launch(k_vel<X, Y, R, F, F>, grid, block, 0, st, a, rows); \
+    else chain_launch(k_vel<X, Y, R, F, false>, grid, block, 0, st, a, rows);                 \
+  } while (0)
   if (g.p2) {
     if (impx && impy) SNS_V(1, 1, true, true);
     else if (impx) SNS_V(1, 0, true, true);
