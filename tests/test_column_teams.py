@@ -1,6 +1,7 @@
 """The fused Poisson launch of the exact form with its worker blocks split into
 teams (csrc/plain_fp64.cu, kFusedTeams): bit for bit the oracle, at one, two and
-four teams, with fewer columns than teams and with a remainder in the last round."""
+four teams, with fewer columns than teams and with a remainder in the last round;
+and with DFT stages of 1 to 64 butterflies (csrc/fft_dev.cuh, butterfly4)."""
 import numpy as np
 import pytest
 
@@ -11,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("nx,ny,stretch", [(32, 1024, 1e9), (8, 2048, 1e9), (130, 2048, 3), (512, 2048, 1e9),
                                            (601, 2048, 1e9), (1025, 2048, 1e9), (33, 4096, 1e9), (24, 8192, 3),
-                                           (16, 16384, 1e9)])
+                                           (16, 16384, 1e9), (8, 8, 1e9), (9, 16, 3),
+                                           (16, 32, 1e9), (33, 64, 3), (64, 128, 1e9), (31, 256, 1e9), (40, 512, 3)])
 def test_teams_give_the_oracles_step(nx, ny, stretch):
     from simplenavierstokessolver_gb300 import Case
 
