@@ -10,7 +10,7 @@ three RK substages (temperature, momentum, Poisson, projection, pressure).
 Arms:
   default          the plain FP64 GPU path of libsns_gpu.so in the form --form
                    names (default parallel: partition-method line solves and
-                   radix-8 DFTs, within 1e-12 of the reference; exact: the
+                   fixed-point DFTs, within 1e-12 of the reference; exact: the
                    reference's operations, bit-identical), the other form's
                    figure beside it; inputs resident in HBM; per-step CUDA
                    events on the solver's stream; L2 flushed (256 MiB write)
@@ -53,9 +53,10 @@ KERNEL_MODEL = {
     # name: (bytes per cell, fp64 ops per cell)
     "temperature_update": (48.0, 27.0),
     "velocity_update": (80.0, 81.0),
-    # on grids whose spacings are powers of two, 29 of the 81 products (the 1/2
-    # weights, reciprocal spacings, advective coefficients) run in the integer unit
-    "velocity_update_p2": (80.0, 52.0),
+    # on grids whose spacings are powers of two, 29 of the 81 operations (the products by the 1/2
+    # weights, reciprocal spacings, advective coefficients) run in the integer
+    # unit, and 15 of the sums
+    "velocity_update_p2": (80.0, 37.0),
     "poisson_forward_fft": (24.0, None),
     "poisson_tridiagonal": (40.0, 5.0),
     # partition-method solve of the parallel form: the spectrum read and
@@ -75,36 +76,34 @@ KERNEL_MODEL = {
 
 
 # DRAM bytes (read + write) per launch from ncu captures of the default
-# workload, keyed by kernel and size: the fused launch from
-# profiles/plain_fp64_fused_512x1024_ncu.md; the velocity update (16.8-25.2 MB
-# per launch in either form; the larger figure is used) and the parallel
-# form's kernels from profiles/plain_parallel_fp64_counts_512x1024.md; the
-# exact form's three-kernel Poisson solve from an earlier capture of the same
-# size
+# workload with warm caches, keyed by kernel and size (the fields stay in L2
+# between kernels at this size): the parallel form's kernels and the exact
+# form's fused launch from profiles/plain_parallel_fp64_counts_512x1024.md, the
+# exact form's three-kernel Poisson solve from an earlier capture
 PROFILED_TRAFFIC = {
-    ("poisson_fused", 512, 1024): 29699840 + 19200,  # profiles/plain_fp64_fused_512x1024_ncu.md
+    ("poisson_fused", 512, 1024): 5625600 + 117760,
     ("poisson_tridiagonal", 512, 1024): 8665344,
-    ("velocity_update", 512, 1024): 25210880,
-    ("poisson_forward_fft", 512, 1024): 8440064,
-    ("temperature_update", 512, 1024): 12647168,
-    ("poisson_inverse_fft", 512, 1024): 4249088,
-    ("correct_and_pressure", 512, 1024): 16805376,
+    ("velocity_update", 512, 1024): 4151552 + 1280,
+    ("poisson_forward_fft", 512, 1024): 58624,
+    ("poisson_pcr", 512, 1024): 11863040,
+    ("temperature_update", 512, 1024): 4055552,
+    ("poisson_inverse_fft", 512, 1024): 1857280,
+    ("correct_and_pressure", 512, 1024): 36864,
 }
 
 
 # FP64 instructions per cell of the parallel form's kernels on a uniform
 # power-of-two grid (DADD + DMUL + DFMA thread instructions counted by ncu at
-# 512 x 1024: profiles/plain_parallel_fp64_counts_512x1024.md; the temperature
-# update's mean over the three substages, the first of which has no previous
-# source; the DFT counts grow with log2(jtot))
-PARALLEL_FP64_OPS = {"velocity_update": 47.45, "temperature_update": 17.17, "poisson_forward_fft": 20.63,
-                     "poisson_pcr": 5.39, "poisson_inverse_fft": 17.75, "correct_and_pressure": 9.0}
+# 512 x 1024: profiles/plain_parallel_fp64_counts_512x1024.md)
+PARALLEL_FP64_OPS = {"velocity_update": 13.12, "temperature_update": 3.0, "poisson_forward_fft": 4.06,
+                     "poisson_pcr": 5.45, "poisson_inverse_fft": 2.0, "correct_and_pressure": 5.5}
 
 # algorithmic DRAM bytes per cell of the plain path's implicit-scheme
 # launches (2048 x 4096 at Ra 1e10): each Crank-Nicolson launch solves the
 # temperature, ux and uy lines side by side (increment read and written per
-# field), the increment launch adds them to the three fields
-IMPLICIT_MODEL = {"cn_solve_x": 48.0, "cn_solve_y": 48.0, "add_increment": 72.0}
+# field); the last one, along y, reads increments and fields and writes the new
+# fields
+IMPLICIT_MODEL = {"cn_solve_x": 48.0, "cn_solve_y": 72.0, "add_increment": 72.0}
 
 
 def batched_bytes_per_cell_step(compensated: bool) -> float:
@@ -365,7 +364,7 @@ def hbm_roofline(cell_steps_per_s: float, compensated: bool) -> dict:
     gbs = cell_steps_per_s * bpc / 1e9
     return {"bytes_per_cell_step": bpc, "achieved": gbs, "peak": peak, "unit": "GB/s", "frac": gbs / peak,
             "peak_source": f"{kind} (MEASURED_PEAKS.json hbm_gbs)" if kind == "measured" else "fallback",
-            "note": "algorithmic bytes of the whole step over its event time; the FP64 DFTs bound the step"}
+            "note": "algorithmic bytes of the whole step over its event time; FP64 issue and latency bound the step"}
 
 
 def large_instance(args, torch, nx=2048, ny=4096, Ra=1e10, steps=500, acc_steps=200):
@@ -897,7 +896,7 @@ def gpu_arm(args, world, rank, local):
                 "traffic": PROFILED_TRAFFIC.get((dom, args.nx, args.ny)),
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback",
                 "algorithmic_bytes_per_launch": bpc * cells if bpc else None,
-                "note": "FP64-pipe bound on GB300: see fp64_roofline"}
+                "note": "instruction issue (FP64 and integer pipes) bounds it on GB300: see fp64_roofline"}
     fp64 = None
     if opc:
         ach = opc * cells / avg_s / 1e9

@@ -55,7 +55,7 @@ typedef struct sns_batch_tuning {
   int tile_x;          /* stencil / correction block width: 32, 64 or 128 columns */
   int tile_rows;       /* rows each stencil / correction thread marches: 1 .. 64 */
   int modes_per_block; /* tridiagonal mode lines (warps) per block: 2, 4 or 8 */
-  int fcols_shift;     /* DFT columns per block: the per-case default times 2^shift, -3 .. 3 */
+  int fcols_shift;     /* threads, and with them columns, per DFT block: the default times 2^shift, -3 .. 3 */
 } sns_batch_tuning;
 
 /* a batch with a device arena of hbm_bytes and room for max_cases cases */

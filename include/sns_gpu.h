@@ -340,14 +340,15 @@ extern int sns_set_fused(const fluid_t *fluid, int on);
  * per segment of itot/32 rows), the Crank-Nicolson lines (src/linalg.c:9-108)
  * by the same method (32 segments per row or column, the periodic y lines
  * with a cyclic interface system; the serial sweep where a line is not a
- * multiple of 32 rows of at least 64), the DFTs by a radix-8 Stockham FFT,
- * and every other kernel compiled with fused multiply-adds. Results differ
+ * multiple of 32 rows of at least 64), the DFTs in 64-bit block fixed point,
+ * the advective and diffusive terms in 64-bit integers, and every other
+ * kernel compiled with fused multiply-adds. Results differ
  * from the reference's by rounding, held to 1e-12 relative L2 per field
  * after the stated step counts. Needs itot in [64, 14048] and a grid on
  * which the mean mode's last Thomas pivot vanishes (uniform grids with a
  * power-of-two itot), otherwise SNS_ERR_UNSUPPORTED and the form is
- * unchanged. The first switch to it computes the Poisson factors (host,
- * O(itot * jtot)) and allocates them on the device; the Crank-Nicolson
+ * unchanged. The first switch to it allocates the Poisson factors on the
+ * device and computes them there; the Crank-Nicolson
  * factors are recomputed on the host every implicit substage (they depend
  * on dt). */
 #define SNS_FORM_EXACT 0
