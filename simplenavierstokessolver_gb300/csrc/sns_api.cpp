@@ -112,6 +112,8 @@ struct Context {
   unsigned fac_next = 0;        // next slot of the ring
   int fac_slot = 0;             // the slot being filled
   double *fac_stage = nullptr;  // its host words
+  bool fac_hold = false;        // uploads are gathered into one copy of words fac_lo .. fac_hi-1
+  size_t fac_lo = 0, fac_hi = 0;
   double *diag = nullptr;  // block partials of sns_diagnostics
   // fused Poisson (+ temperature) launches: flag words, on unless disabled
   // or unsupported for this size
@@ -715,10 +717,20 @@ static void y_system(const param_t *param, int rk, int is_temp, HostFactors &sub
 
 // copies n doubles at word offset `off` of the substage's pinned staging slot
 // into the device factor buffer (stream-ordered, asynchronous)
-static int stage_upload(Context *c, size_t off, const double *src, size_t n) {
-  std::memcpy(c->fac_stage + off, src, n * sizeof(double));
+// (while c->fac_hold: noted for the one copy of upload_held)
+static int send_staged(Context *c, size_t off, size_t n) {
+  if (c->fac_hold) {
+    c->fac_lo = std::min(c->fac_lo, off);
+    c->fac_hi = std::max(c->fac_hi, off + n);
+    return SNS_OK;
+  }
   SNS_CUDA(cudaMemcpyAsync(c->fac + off, c->fac_stage + off, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   return SNS_OK;
+}
+
+static int stage_upload(Context *c, size_t off, const double *src, size_t n) {
+  std::memcpy(c->fac_stage + off, src, n * sizeof(double));
+  return send_staged(c, off, n);
 }
 
 // copies factor arrays into the context's device buffer at word offset `off`
@@ -728,7 +740,7 @@ static int push_factors(Context *c, const HostFactors &hf, size_t off, LineFacto
   std::memcpy(st, hf.l.data(), n * sizeof(double));
   std::memcpy(st + n, hf.inv.data(), n * sizeof(double));  // 0 marks |pivot| < DBL_EPSILON rows
   std::memcpy(st + 2 * n, hf.up.data(), n * sizeof(double));
-  SNS_CUDA(cudaMemcpyAsync(c->fac + off, st, 3 * n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  if (int rc = send_staged(c, off, 3 * n)) return rc;
   lf.n = (int)n;
   lf.l = c->fac + off;
   lf.inv = c->fac + off + n;
@@ -1014,6 +1026,7 @@ static int implicit_updates(const param_t *param, int rk, FluidExt *fe, TempExt 
   const bool with_t = param->with_temperature && te;
   const StageScalars s = stage_scalars(param, rk);
   if (int rc = ensure_implicit_buffers(fe)) return rc;
+  SNS_CUDA(cudaEventRecord(c->ev_fwd, c->stream));  // the solves before are the last to read the factors
   int out = 0;
   if (with_t) {
     if (!te->f.qt)
@@ -1038,79 +1051,102 @@ static int implicit_updates(const param_t *param, int rk, FluidExt *fe, TempExt 
                              Increment{f.ux, f.ux_alt}, Increment{f.uy, f.uy_alt}};
   if (impx || impy)
     if (int rc = begin_factor_uploads(c)) return rc;
-  if (impx && cn_parallel(c, c->nx)) {
-    ParCnArgs a = cn_x_args(c);
-    for (int k = with_t ? 0 : 1; k < 3; k++) {
-      std::vector<double> blk;
-      cn_x_block(param, rk, kinds[k], blk);
-      if (int rc = stage_upload(c, cnx_off(c, k), blk.data(), blk.size())) return rc;
-      a.f[a.nf] = ParCnField{qs[k], c->fac + cnx_off(c, k), 0, impy ? Increment{} : adds[k], k == 1 ? 1 : 0};
-      cn_reach(blk, c->nx, a.f[a.nf++]);
+  // the factors of all systems go up in one copy on the side stream, beside the
+  // source kernels (one copy per array in the solver's stream: 128 x 256
+  // stretched 8 us per substage more)
+  c->fac_hold = true;
+  c->fac_lo = SIZE_MAX;
+  c->fac_hi = 0;
+  ParCnArgs pax{}, pay{};
+  SolveXSet setx{};
+  SolveYSet sety{};
+  const int staged = [&]() -> int {
+    if (impx && cn_parallel(c, c->nx)) {
+      ParCnArgs a = cn_x_args(c);
+      for (int k = with_t ? 0 : 1; k < 3; k++) {
+        std::vector<double> blk;
+        cn_x_block(param, rk, kinds[k], blk);
+        if (int rc = stage_upload(c, cnx_off(c, k), blk.data(), blk.size())) return rc;
+        a.f[a.nf] = ParCnField{qs[k], c->fac + cnx_off(c, k), 0, impy ? Increment{} : adds[k], k == 1 ? 1 : 0};
+        cn_reach(blk, c->nx, a.f[a.nf++]);
+      }
+      pax = a;
+    } else if (impx) {
+      SolveXSet set{};
+      for (int k = with_t ? 0 : 1; k < 3; k++) {
+        HostFactors hf;
+        x_system(param, rk, kinds[k], hf);
+        if (int rc = push_factors(c, hf, xset_off(c, k), set.f[set.n])) return rc;
+        set.mode[set.n] = kinds[k] == 1 ? 1 : 0;
+        set.q[set.n] = qs[k];
+        if (!impy) set.add[set.n] = adds[k];
+        set.n++;
+      }
+      setx = set;
     }
-    Prof pf(c, K_SOLVE_X);
-    SNS_CUDA(launch_par_cn(false, a, c->stream));
-  } else if (impx) {
-    SolveXSet set{};
-    for (int k = with_t ? 0 : 1; k < 3; k++) {
-      HostFactors hf;
-      x_system(param, rk, kinds[k], hf);
-      if (int rc = push_factors(c, hf, xset_off(c, k), set.f[set.n])) return rc;
-      set.mode[set.n] = kinds[k] == 1 ? 1 : 0;
-      set.q[set.n] = qs[k];
-      if (!impy) set.add[set.n] = adds[k];
-      set.n++;
+    if (impy && cn_parallel(c, c->ny)) {
+      ParCnArgs a = cn_y_args(c);
+      for (int sys = with_t ? 0 : 1; sys < 2; sys++) {  // y systems: temperature, velocity
+        std::vector<double> blk;
+        cn_y_block(param, rk, sys == 0 ? 1 : 0, blk);
+        if (int rc = stage_upload(c, cny_off(c, sys), blk.data(), blk.size())) return rc;
+        const double *fac = c->fac + cny_off(c, sys);
+        const int first = a.nf;
+        if (sys == 0) {
+          a.f[a.nf++] = ParCnField{te->f.qt, fac, 0, adds[0]};
+        } else {
+          a.f[a.nf++] = ParCnField{f.qx, fac, 1, adds[1]};  // ux: columns 1..itot-1
+          a.f[a.nf++] = ParCnField{f.qy, fac, 0, adds[2]};
+        }
+        for (int k = first; k < a.nf; k++) cn_reach(blk, c->ny, a.f[k]);
+      }
+      pay = a;
+    } else if (impy) {
+      SolveYSet set{};
+      for (int sys = with_t ? 0 : 1; sys < 2; sys++) {  // y systems: temperature, velocity
+        HostFactors sub;
+        std::vector<double> q1;
+        PeriodicFactors pf{};
+        y_system(param, rk, sys == 0 ? 1 : 0, sub, q1, pf.l_last, pf.u_last, pf.den);
+        const size_t off = yset_off(c, sys);
+        if (int rc = push_factors(c, sub, off, pf.sub)) return rc;
+        const size_t qoff = off + 3 * sub.l.size();
+        if (int rc = stage_upload(c, qoff, q1.data(), q1.size())) return rc;
+        pf.q1 = c->fac + qoff;
+        if (sys == 0) {
+          set.f[set.n] = pf;
+          set.first_col[set.n] = 0;
+          set.add[set.n] = adds[0];
+          set.q[set.n++] = te->f.qt;
+        } else {
+          set.f[set.n] = pf;
+          set.first_col[set.n] = 1;  // ux
+          set.add[set.n] = adds[1];
+          set.q[set.n++] = f.qx;
+          set.f[set.n] = pf;
+          set.first_col[set.n] = 0;  // uy
+          set.add[set.n] = adds[2];
+          set.q[set.n++] = f.qy;
+        }
+      }
+      sety = set;
     }
+    return SNS_OK;
+  }();
+  c->fac_hold = false;
+  if (staged != SNS_OK) return staged;
+  SNS_CUDA(cudaStreamWaitEvent(c->side, c->ev_fwd, 0));
+  SNS_CUDA(cudaMemcpyAsync(c->fac + c->fac_lo, c->fac_stage + c->fac_lo, (c->fac_hi - c->fac_lo) * sizeof(double),
+                           cudaMemcpyHostToDevice, c->side));
+  SNS_CUDA(cudaEventRecord(c->ev_temp, c->side));
+  SNS_CUDA(cudaStreamWaitEvent(c->stream, c->ev_temp, 0));
+  if (impx) {
     Prof pf(c, K_SOLVE_X);
-    SNS_CUDA(FORM(c, launch_solve_x_set)(c->g, set, c->stream));
+    SNS_CUDA(pax.nf ? launch_par_cn(false, pax, c->stream) : FORM(c, launch_solve_x_set)(c->g, setx, c->stream));
   }
-  if (impy && cn_parallel(c, c->ny)) {
-    ParCnArgs a = cn_y_args(c);
-    for (int sys = with_t ? 0 : 1; sys < 2; sys++) {  // y systems: temperature, velocity
-      std::vector<double> blk;
-      cn_y_block(param, rk, sys == 0 ? 1 : 0, blk);
-      if (int rc = stage_upload(c, cny_off(c, sys), blk.data(), blk.size())) return rc;
-      const double *fac = c->fac + cny_off(c, sys);
-      const int first = a.nf;
-      if (sys == 0) {
-        a.f[a.nf++] = ParCnField{te->f.qt, fac, 0, adds[0]};
-      } else {
-        a.f[a.nf++] = ParCnField{f.qx, fac, 1, adds[1]};  // ux: columns 1..itot-1
-        a.f[a.nf++] = ParCnField{f.qy, fac, 0, adds[2]};
-      }
-      for (int k = first; k < a.nf; k++) cn_reach(blk, c->ny, a.f[k]);
-    }
-    Prof pr(c, K_SOLVE_Y);
-    SNS_CUDA(launch_par_cn(true, a, c->stream));
-  } else if (impy) {
-    SolveYSet set{};
-    for (int sys = with_t ? 0 : 1; sys < 2; sys++) {  // y systems: temperature, velocity
-      HostFactors sub;
-      std::vector<double> q1;
-      PeriodicFactors pf{};
-      y_system(param, rk, sys == 0 ? 1 : 0, sub, q1, pf.l_last, pf.u_last, pf.den);
-      const size_t off = yset_off(c, sys);
-      if (int rc = push_factors(c, sub, off, pf.sub)) return rc;
-      const size_t qoff = off + 3 * sub.l.size();
-      if (int rc = stage_upload(c, qoff, q1.data(), q1.size())) return rc;
-      pf.q1 = c->fac + qoff;
-      if (sys == 0) {
-        set.f[set.n] = pf;
-        set.first_col[set.n] = 0;
-        set.add[set.n] = adds[0];
-        set.q[set.n++] = te->f.qt;
-      } else {
-        set.f[set.n] = pf;
-        set.first_col[set.n] = 1;  // ux
-        set.add[set.n] = adds[1];
-        set.q[set.n++] = f.qx;
-        set.f[set.n] = pf;
-        set.first_col[set.n] = 0;  // uy
-        set.add[set.n] = adds[2];
-        set.q[set.n++] = f.qy;
-      }
-    }
-    Prof pr(c, K_SOLVE_Y);
-    SNS_CUDA(FORM(c, launch_solve_y_set)(c->g, set, c->stream));
+  if (impy) {
+    Prof pf(c, K_SOLVE_Y);
+    SNS_CUDA(pay.nf ? launch_par_cn(true, pay, c->stream) : FORM(c, launch_solve_y_set)(c->g, sety, c->stream));
   }
   if (impx || impy)
     if (int rc = end_factor_uploads(c)) return rc;
