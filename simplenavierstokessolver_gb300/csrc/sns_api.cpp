@@ -1287,11 +1287,31 @@ static int fused_check(Context *c) {
               (code & 1) ? "sweep" : "worker", code);
 }
 
+// copies of the error words to the host, where no reduction goes with them
 static int fused_enqueue_err(Context *c) {
   if (c->fused_ready)
     SNS_CUDA(cudaMemcpyAsync(c->fz_err_host, c->fz.err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
   if (c->par_ready)
     SNS_CUDA(cudaMemcpyAsync(c->par_err_host, c->par.err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  return SNS_OK;
+}
+
+// enqueues the reduction's and the error words' way to the host. The device's
+// copy of the reduction is gone then: red_version is set again by the caller
+// once the host's copy is known to be good.
+static int publish(Context *c, Fields &f) {
+  SNS_CUDA(launch_publish(f.colmax, c->red_host, c->nx + 1, c->fused_ready ? c->fz.err : nullptr, c->fz_err_host,
+                          c->par_ready ? c->par.err : nullptr, c->par_err_host, c->stream));
+  f.red_zero = true;
+  c->red_version = 0;
+  return SNS_OK;
+}
+
+// before a reduction into colmax: its words are zero
+static int zero_reduction(Context *c, Fields &f) {
+  if (!f.red_zero)
+    SNS_CUDA(cudaMemsetAsync(f.colmax, 0, sizeof(unsigned long long) * (c->nx + 1), c->stream));
+  f.red_zero = false;
   return SNS_OK;
 }
 
@@ -1395,16 +1415,15 @@ static int nonfinite_check(const Context *c, const param_t *param) {
 static int reduce_to_host(Context *c, Fields &f, bool launch) {
   // copied to the host at the end of the call that computed it
   if (!launch && c->red_host_version == c->version) return SNS_OK;
-  if (launch) {
-    SNS_CUDA(cudaMemsetAsync(f.colmax, 0, sizeof(unsigned long long) * (c->nx + 1), c->stream));
+  if (launch || f.red_zero) {
+    if (int rc = zero_reduction(c, f)) return rc;
     Prof pf(c, K_UMAX);
     SNS_CUDA(launch_umax(c->g, f.ux, f.uy, f.colmax, f.uymax, c->stream));
   }
-  SNS_CUDA(cudaMemcpyAsync(c->red_host, f.colmax, sizeof(unsigned long long) * (c->nx + 1), cudaMemcpyDeviceToHost,
-                           c->stream));
-  if (int rc = fused_enqueue_err(c)) return rc;
+  if (int rc = publish(c, f)) return rc;
   SNS_CUDA(cudaStreamSynchronize(c->stream));
   if (int rc = fused_check(c)) return rc;
+  c->red_version = c->version;
   c->red_host_version = c->version;
   return SNS_OK;
 }
@@ -1835,7 +1854,8 @@ int fluid_update_pressure(const param_t *param, const parallel_t *parallel, cons
     // the last substage also leaves the max-|u| reduction for the next
     // param_decide_dt (the velocity is final for the step)
     const bool red = rkstep == RKSTEPMAX - 1;
-    if (red) SNS_CUDA(cudaMemsetAsync(fe->f.colmax, 0, sizeof(unsigned long long) * (c->nx + 1), c->stream));
+    if (red)
+      if (int rc = zero_reduction(c, fe->f)) return rc;
     {
       Prof pf(c, K_CORR_PRES);
       SNS_CUDA(FORM(c, launch_correct_pressure)(c->g, s, param->implicitx, param->implicity, fe->f.psi, fe->f.ux, fe->f.uy,
@@ -2115,13 +2135,12 @@ static int sync_to_device_impl(const param_t *param, fluid_t *fluid, temperature
   // call's wait: the next param_decide_dt / sns_run decides dt without a
   // launch and a round trip of its own
   if (fe) {
-    SNS_CUDA(cudaMemsetAsync(fe->f.colmax, 0, sizeof(unsigned long long) * (c->nx + 1), c->stream));
+    if (int rc = zero_reduction(c, fe->f)) return rc;
     {
       Prof pf(c, K_UMAX);
       SNS_CUDA(launch_umax(c->g, fe->f.ux, fe->f.uy, fe->f.colmax, fe->f.uymax, c->stream));
     }
-    SNS_CUDA(cudaMemcpyAsync(c->red_host, fe->f.colmax, sizeof(unsigned long long) * (c->nx + 1),
-                             cudaMemcpyDeviceToHost, c->stream));
+    if (int rc = publish(c, fe->f)) return rc;
   }
   SNS_CUDA(cudaStreamSynchronize(c->stream));
   if (fe) {
@@ -2708,7 +2727,8 @@ static int integrate_impl(const param_t *param, FluidExt *fe, TempExt *te, bool 
       }
     }
     const bool red = reduce_last && rk == RKSTEPMAX - 1;
-    if (red) SNS_CUDA(cudaMemsetAsync(f.colmax, 0, sizeof(unsigned long long) * (c->nx + 1), c->stream));
+    if (red)
+      if (int rc = zero_reduction(c, f)) return rc;
     {
       Prof pf(c, K_CORR_PRES);
       SNS_CUDA(FORM(c, launch_correct_pressure)(c->g, s, param->implicitx, param->implicity, f.psi, f.ux, f.uy, f.p,
@@ -2759,14 +2779,13 @@ int sns_run(param_t *param, const parallel_t *parallel, fluid_t *fluid, temperat
     // the last step's reduction to the host with this call's final wait, so
     // that the next call decides dt without a round trip; launch errors of
     // this call are reported by this call
-    SNS_CUDA(cudaMemcpyAsync(c->red_host, fe->f.colmax, sizeof(unsigned long long) * (c->nx + 1),
-                             cudaMemcpyDeviceToHost, c->stream));
-    if (int rc = fused_enqueue_err(c)) return rc;
+    if (int rc = publish(c, fe->f)) return rc;
   }
   SNS_CUDA(cudaStreamSynchronize(c->stream));
   if (nsteps > 0) {
     if (int rc = fused_check(c)) return rc;
-    c->red_host_version = c->red_version;
+    c->red_version = c->version;
+    c->red_host_version = c->version;
     return nonfinite_check(c, param);
   }
   return SNS_OK;

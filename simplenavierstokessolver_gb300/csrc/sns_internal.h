@@ -93,6 +93,7 @@ struct Fields {
   double2 *spec;               // Poisson spectrum [nx * jpitch]
   unsigned long long *colmax;  // [nx] max |ux| per column (bit patterns)
   unsigned long long *uymax;   // [1]
+  bool red_zero;               // colmax and uymax hold zeros: the last reduction went to the host
 };
 
 struct TempFields {
