@@ -28,12 +28,13 @@ struct DiagArgs {
 constexpr int kDiagOut = 16;  // words kept for the 11 results at the head of the scratch
 // words of device scratch for a grid
 size_t diag_words(int nx, int ny);
-// the block sums and their final sum; *out: the 11 results on the device:
+// the block sums and their final sum; *out: the 11 results, in host (pinned, if
+// given) or at the head of the device's scratch:
 // divergence max, sum; x, y momentum; kinetic x, y and thermal energy;
 // Nu from wall flux, injection, kinetic dissipation, thermal dissipation.
 // Two launches.
 template <typename F>
-cudaError_t launch_diag(const DiagArgs<F> &a, double *scratch, double **out, cudaStream_t st);
+cudaError_t launch_diag(const DiagArgs<F> &a, double *scratch, double **out, cudaStream_t st, double *host = nullptr);
 
 // allocation-free form: block partials in a fixed file-scope device array of
 // kDiagStaticBlocks blocks (672 KiB), the final sum on the device; grids with

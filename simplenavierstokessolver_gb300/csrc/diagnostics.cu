@@ -28,13 +28,16 @@
 // sns_diagnostics, host time per call: with compensated FP64 sums (62 FP64
 // instructions a cell, 16 rows per thread on every grid) against this, 64 x 128
 // 110 / 42 us, 128 x 256 stretched 127 / 50, 512 x 1024 168 / 91, 1024 x 2048
-// 507 / 201, 2048 x 4096 1728 / 720; ~20 us of each are the two launches, the
-// copy and the wait. The FP64 pipe is still the busiest (65 % of its cycles at
+// 507 / 201, 2048 x 4096 1728 / 720. The two launches, the results' way and the
+// wait were ~20 us of each; with the results stored straight into pinned host
+// memory and launches prepared ahead (chain.cuh) 64 x 128 takes 34, 128 x 256
+// uniform 42 (52 before), 512 x 1024 82, 1024 x 2048 196. The FP64 pipe is still the busiest (65 % of its cycles at
 // 512 x 1024): the merges of a thread's and a block's sums add as much as ten
 // rows.
 #include <cstdint>
 #include <mutex>
 
+#include "chain.cuh"
 #include "diag_internal.h"
 
 namespace sns {
@@ -155,6 +158,7 @@ constexpr int kDiagParts = 6;  // threads merging one sum of a block
 // column also the wall's face) and `rows` rows.
 template <typename F>
 __global__ void __launch_bounds__(kDiagThreads, 8) k_diag(DiagArgs<F> a, double *partials, int rows) {
+  chain_begin();
   const int nx = a.nx, ny = a.ny;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y0 = blockIdx.y * rows, y1 = min(y0 + rows, ny);
@@ -274,6 +278,7 @@ constexpr int kFinishThreads = 256;
 
 __global__ void __launch_bounds__(kFinishThreads) k_diag_finish(const double *partials, int nblocks, double ly,
                                                                double *out) {
+  chain_begin();
   __shared__ double ss[kFinishThreads], sc[kFinishThreads];
   const int k = blockIdx.x, t = threadIdx.x;
   const size_t stride = 2 * kDiagSums + 1;
@@ -352,16 +357,17 @@ size_t diag_words(int nx, int ny) {
 }
 
 template <typename F>
-cudaError_t launch_diag(const DiagArgs<F> &a, double *scratch, double **out, cudaStream_t st) {
+cudaError_t launch_diag(const DiagArgs<F> &a, double *scratch, double **out, cudaStream_t st, double *host) {
   const dim3 grid = diag_grid(a.nx, a.ny);
-  k_diag<F><<<grid, kDiagThreads, 0, st>>>(a, scratch + kDiagOut, diag_rows(a.nx, a.ny));
-  k_diag_finish<<<kDiagSums + 1, kFinishThreads, 0, st>>>(scratch + kDiagOut, (int)(grid.x * grid.y), a.ly, scratch);
-  *out = scratch;
+  *out = host ? host : scratch;
+  chain_launch(k_diag<F>, grid, kDiagThreads, 0, st, a, scratch + kDiagOut, diag_rows(a.nx, a.ny));
+  chain_launch(k_diag_finish, kDiagSums + 1, kFinishThreads, 0, st, scratch + kDiagOut, (int)(grid.x * grid.y), a.ly,
+               *out);
   return cudaGetLastError();
 }
 
-template cudaError_t launch_diag<double>(const DiagArgs<double> &, double *, double **, cudaStream_t);
-template cudaError_t launch_diag<float>(const DiagArgs<float> &, double *, double **, cudaStream_t);
+template cudaError_t launch_diag<double>(const DiagArgs<double> &, double *, double **, cudaStream_t, double *);
+template cudaError_t launch_diag<float>(const DiagArgs<float> &, double *, double **, cudaStream_t, double *);
 
 // ---------------------------------------------------------------------------
 // Allocation-free variant (sns_diagnostics_static in sns_api.cpp).

@@ -102,6 +102,8 @@ struct Context {
   std::vector<double> dxf, dxc;  // host copies of the reference arrays (0-based)
   double *staging = nullptr;     // pinned, nx*ny doubles
   unsigned long long *red_host = nullptr;  // pinned, nx+1 words
+  double *diag_host = nullptr;  // behind them: the results of sns_diagnostics
+  std::mutex diag_mu;           // over a call's launches, its wait and its reading of diag_host
   // factors for the implicit solves: device buffer, and a ring of pinned host
   // staging slots so that the uploads are asynchronous; a slot is rewritten
   // only after its previous upload completed (fac_ev)
@@ -395,7 +397,8 @@ static int build_context(Context *c, const param_t *param) {
   if ((rc = upload(c, &g.tw, tw))) return rc;
   fft_layout(ny, &g.fft_nst, &g.fft_first2);
   SNS_CUDA(counted_malloc_host(&c->staging, sizeof(double) * (size_t)nx * ny));
-  SNS_CUDA(counted_malloc_host(&c->red_host, sizeof(unsigned long long) * (size_t)(nx + 1)));
+  SNS_CUDA(counted_malloc_host(&c->red_host, sizeof(unsigned long long) * (size_t)(nx + 1 + kDiagOut)));
+  c->diag_host = reinterpret_cast<double *>(c->red_host + nx + 1);
   return SNS_OK;
 }
 
@@ -2171,10 +2174,11 @@ int sns_diagnostics(const param_t *param, const fluid_t *fluid, const temperatur
   const DiagArgs<double> a{nx, ny, param->dy, param->ly, sqrt(Pr) * sqrt(Ra), sqrt(Pr) / sqrt(Ra),
                            1. / sqrt(Pr) / sqrt(Ra), c->g.dxf, c->g.dxc, fe->f.ux, fe->f.uy, te->f.t[te->cur]};
   double *res = nullptr;
-  SNS_CUDA(launch_diag(a, c->diag, &res, c->stream));
+  std::lock_guard<std::mutex> lk(c->diag_mu);
+  SNS_CUDA(launch_diag(a, c->diag, &res, c->stream, c->diag_host));
   count_launches(2);
-  SNS_CUDA(cudaMemcpyAsync(out, res, 11 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   SNS_CUDA(cudaStreamSynchronize(c->stream));
+  std::memcpy(out, res, 11 * sizeof(double));
   return SNS_OK;
 }
 
