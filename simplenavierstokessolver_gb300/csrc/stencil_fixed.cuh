@@ -12,20 +12,28 @@
 //   A = - ax (sxm dxm + sxp dxp) - ay (sym dym + syp dyp)
 //       + cp dxp - cm dxm + cy (dyp - dym),
 // d the differences of the updated quantity f to its neighbours, s twice the
-// velocities of the faces. The values of f that a cell reads are taken at the
-// largest exponent among them, as integers below 2^60: exact for values from
-// 2^-7 of the largest one up, truncated at its 2^-60 below. So differences and
-// second differences are exact for the most part; the former are shifted up
-// together until the largest has 62 bits, the latter too, and the products'
-// top 64 bits are formed from there. The other velocity's values have an
-// exponent of their own. cp and cm are equal, or (at a wall) one is twice the other, up to
-// the rounding of the grid: what is left of cp dxp - cm dxm beside the second
-// difference is a term of its own (ex), zero on a grid of equal spacings. No
-// sum can overflow (bounds beside each line).
+// velocities of the faces. The three values of f along a direction are taken at
+// the largest exponent among them, as integers below 2^60: exact for values
+// from 2^-7 of the largest one up, truncated at its 2^-60 below. So differences
+// and second differences are exact for the most part; the two differences of a
+// direction are shifted up together until the larger one has 62 bits, the second
+// difference too, and the products' top 64 bits are formed from there. The
+// velocities of a direction's faces have an exponent of their own. Each
+// direction's advection and diffusion is a number with its own exponent until
+// the final sum: on cells that are not square the coefficients of the two
+// directions and their differences are the aspect and its square apart. (One
+// exponent and one shift for both lost two bits for each doubling of the
+// aspect: at 64 the error was 96 times the FP64 expressions', at 1/32 25 times.)
+// cp and cm are equal, or (at a wall) one is twice the other, up to the rounding
+// of the grid: what is left of cp dxp - cm dxm beside the second difference is a
+// term of its own (ex), zero on a grid of equal spacings. No sum can overflow
+// (bounds beside each line).
 //
 // Accuracy: the error of A is below that of the FP64 expressions, whose terms
-// are rounded at 2^-53 each (tests/test_stencil_fixed.py measures both against
-// long double: 0.4 to 0.6 of it).
+// are rounded at 2^-53 each: 0.4 to 0.6 of it on square cells
+// (tests/test_stencil_fixed.py), 0.8 or less at aspects from 1/512 to 512
+// (tests/test_stencil_aspect.py; both against long double). Diffusion alone, on
+// spacings that are powers of two, is the exact value rounded once either way.
 #pragma once
 
 #include "fft_fixed.cuh"
@@ -96,12 +104,12 @@ struct Val {
   long long v;
   int e;
 };
-// their sum at the larger exponent; |v| <= 2^62 together
+// their sum at the larger exponent; |v| < 2^63 together
 FX_HD Val add(Val a, Val b) {
   const int t = a.e - b.e;
   return Val{shr(a.v, imax(-t, 0)) + shr(b.v, imax(t, 0)), imax(a.e, b.e)};
 }
-// |v| <= 2^62, e - 62 and e + 1 exponents of normal numbers
+// |v| < 2^63, e - 62 and e + 1 exponents of normal numbers
 FX_HD double to_double(Val x) {
   const long long n = x.v >> 63;
   const unsigned long long a = (unsigned long long)((x.v ^ n) - n);
@@ -139,12 +147,11 @@ FX_HD Coef mul(Coef a, Coef b) {
 FX_HD Coef quarter(Coef a) { return Coef{a.m, a.e - 2}; }
 FX_HD long long down(long long m, int s) { return m >> imin(s, 63); }
 
-// the coefficients: the advective terms' at one exponent, the second
-// differences' at another, or (where only one direction is implicit, and they
-// go different ways) at one each
+// the coefficients, at an exponent for each direction: a cell of aspect a has
+// 1/dx and 1/dy a factor of a apart, the diffusive coefficients a^2
 struct Terms {
   Split ax, ay, cx, cy;
-  int ea, ecx, ecy;  // of the integers, without the exponents of s and f
+  int eax, eay, ecx, ecy;  // of the products' integers, without the exponents of s and f
   // cm is nearer to 2 cp (tm) or cp to 2 cm (tp) than they are to each other:
   // the second difference in x is dxp - dxm, or dxp / 2 - dxm, or dxp - dxm / 2
   bool tm, tp;
@@ -154,12 +161,12 @@ struct Terms {
 // false: cp and cm too far apart (|ex| could exceed cx / 2), or exponents that
 // a sum's double could not have
 constexpr int kCoefExp = 300;
-template <bool APART>
+template <bool EQ>
 FX_HD bool terms(Terms &k, Coef ax, Coef ay, Coef cp, Coef cm, Coef cy) {
-  const int ta = imax(ax.e, ay.e) + 1;
-  k.ax = split(down(ax.m, ta - ax.e));  // <= 2^62
-  k.ay = split(down(ay.m, ta - ay.e));
-  k.ea = ta - 55 - 2044;
+  k.ax = split(-(ax.m >> 1));  // > -2^62
+  k.ay = split(-(ay.m >> 1));
+  k.eax = ax.e - 54 - 2044;
+  k.eay = ay.e - 54 - 2044;
   // cp and cm at the larger exponent of the two, halved (< 2^62)
   const int eb = imax(cp.e, cm.e) + 1;
   const long long p = down(cp.m, eb - cp.e), m = down(cm.m, eb - cm.e);
@@ -168,15 +175,16 @@ FX_HD bool terms(Terms &k, Coef ax, Coef ay, Coef cp, Coef cm, Coef cy) {
   // cp dxp - cm dxm = cx (second difference) + ex (dxp or dxm)
   Coef cx = k.tp ? cm : cp;
   if (k.tp | k.tm) cx.e += 1;
-  const long long ex = k.tp ? p - 2 * m : k.tm ? 2 * p - m : p - m;
-  const int up = fx::clz64((unsigned long long)(ex ^ (ex >> 63)) | 1ull) - 2;
-  k.ex = split(fx::shl(ex, up));  // <= 2^62
-  k.ee = eb - 59 - 1022 - up;
-  const int tx = (APART ? cx.e : imax(cx.e, cy.e)) + 2, ty = APART ? cy.e + 2 : tx;
-  k.cx = split(down(cx.m, tx - cx.e));  // <= 2^61
-  k.cy = split(down(cy.m, ty - cy.e));
-  k.ecx = tx - 59 - 1022;
-  k.ecy = ty - 59 - 1022;
+  if (!EQ) {
+    const long long ex = k.tp ? p - 2 * m : k.tm ? 2 * p - m : p - m;
+    const int up = fx::clz64((unsigned long long)(ex ^ (ex >> 63)) | 1ull) - 2;
+    k.ex = split(fx::shl(ex, up));  // <= 2^62
+    k.ee = eb - 59 - 1022 - up;
+  }
+  k.cx = split(cx.m >> 1);  // < 2^62
+  k.cy = split(cy.m >> 1);
+  k.ecx = cx.e - 58 - 1022;
+  k.ecy = cy.e - 58 - 1022;
   auto in = [](Coef c) { return c.e >= -kCoefExp && c.e <= kCoefExp; };
   return m - p <= p + (p >> 1) && p - m <= m + (m >> 1) && in(ax) && in(ay) && in(cp) && in(cm) && in(cy);
 }
@@ -196,35 +204,38 @@ FX_HD int room(unsigned m) {
   return __builtin_clz(m | 1u) - 2;
 #endif
 }
-// f's differences at the exponent ef, s at exponents whose largest one is ec,
-// by tx and ty above those of sx and sy; |s|, |d| <= 2^61. EQ: equal spacings
-// (ex = 0)
+// a direction's advective term s_m d_m + s_p d_p times the coefficient -a, from
+// differences shifted up by g; |s| <= 2^61, |d| <= 2^62
+FX_HD Val advective(Split dm, Split dp, int g, long long sm, long long sp, Split a, int e) {
+  const long long t = fx::shl(prod2(split(sm), dm, split(sp), dp), 2);  // <= 2^62
+  return Val{prod(split(t), a), e - 2 - g};                             // <= 2^60
+}
+FX_HD Val diffusive(long long d2, Split c, int e) {  // |d2| < 2^62
+  const int g = fx::clz64((unsigned long long)(d2 ^ (d2 >> 63)) | 1ull) - 2;
+  return Val{prod(split(fx::shl(d2, g)), c), e - g};  // <= 2^60
+}
+// differences of f along x and y and the velocities of the faces in that
+// direction, at an exponent each; |s|, |d| <= 2^61
+struct Line {
+  long long dm, dp, sm, sp;
+  int ed, es;
+};
+// EQ: equal spacings (ex = 0)
 template <bool IMPX, bool IMPY, bool EQ>
-FX_HD Sum sum(const Terms &k, int ef, int ec, int tx, int ty, long long dxm, long long dxp, long long dym,
-              long long dyp, long long sxm, long long sxp, long long sym, long long syp) {
-  const int g = room(size(dxm) | size(dxp) | size(dym) | size(dyp));
-  const Split xm = split(fx::shl(dxm, g)), xp = split(fx::shl(dxp, g));
-  const Split ym = split(fx::shl(dym, g)), yp = split(fx::shl(dyp, g));
-  const long long sx = shr(prod2(split(sxm), xm, split(sxp), xp), tx);  // <= 2^60
-  const long long sy = shr(prod2(split(sym), ym, split(syp), yp), ty);
-  const Val adv{-prod2(split(sx), k.ax, split(sy), k.ay), k.ea + ec + ef - g};  // <= 2^59
-  const long long d1 = (k.tm ? dxp >> 1 : dxp) - (k.tp ? dxm >> 1 : dxm), d2 = dyp - dym;  // < 2^62
-  constexpr bool APART = IMPX != IMPY;
-  const int g1 = room(APART ? size(d1) : size(d1) | size(d2)), g2 = APART ? room(size(d2)) : g1;
-  const Split e1 = split(fx::shl(d1, g1)), e2 = split(fx::shl(d2, g2));
-  Val x{0, k.ecx + ef - g1}, y{0, k.ecy + ef - g2};
-  if (!APART) {
-    x.v = prod2(e1, k.cx, e2, k.cy);  // <= 2^60
-  } else {
-    x.v = prod(e1, k.cx);
-    y.v = prod(e2, k.cy);
-  }
-  if (!EQ) x = add(x, Val{prod(k.tp ? xp : xm, k.ex), k.ee + ef - g});  // <= 2^60 + 2^60
+FX_HD Sum sum(const Terms &k, const Line &X, const Line &Y) {
+  const int gx = room(size(X.dm) | size(X.dp)), gy = room(size(Y.dm) | size(Y.dp));
+  const Split xm = split(fx::shl(X.dm, gx)), xp = split(fx::shl(X.dp, gx));
+  const Split ym = split(fx::shl(Y.dm, gy)), yp = split(fx::shl(Y.dp, gy));
+  const Val adv = add(advective(xm, xp, gx, X.sm, X.sp, k.ax, k.eax + X.es + X.ed),
+                      advective(ym, yp, gy, Y.sm, Y.sp, k.ay, k.eay + Y.es + Y.ed));  // <= 2^61
+  Val x = diffusive((k.tm ? X.dp >> 1 : X.dp) - (k.tp ? X.dm >> 1 : X.dm), k.cx, k.ecx + X.ed);
+  const Val y = diffusive(Y.dp - Y.dm, k.cy, k.ecy + Y.ed);
+  if (!EQ) x = add(x, Val{prod(k.tp ? xp : xm, k.ex), k.ee + X.ed - gx});  // <= 2^61
   Sum r;
+  r.A = adv;
   r.G = Val{0, 0};
   if (IMPX && IMPY) {
-    r.A = adv;
-    r.G = x;
+    r.G = add(x, y);
   } else if (IMPX) {
     r.A = add(adv, y);
     r.G = x;
@@ -232,7 +243,7 @@ FX_HD Sum sum(const Terms &k, int ef, int ec, int tx, int ty, long long dxm, lon
     r.A = add(adv, x);
     r.G = y;
   } else {
-    r.A = add(adv, x);
+    r.A = add(adv, add(x, y));  // <= 2^61 + 2^61 + 2^60
   }
   return r;
 }
@@ -253,44 +264,54 @@ FX_HD long long twice_mean(const Weights &w, long long a, long long b) {
   return fx::shl(prod(split(fx::shl(a, 2)), w.m) + prod(split(fx::shl(b, 2)), w.p), 1);
 }
 
-FX_HD int exponent(Num a, Num b, Num c, Num d, Num e) { return imax(imax(imax(a.e, b.e), imax(c.e, d.e)), e.e); }
+FX_HD int top(Num a, Num b) { return imax(a.e, b.e); }
+FX_HD int top(Num a, Num b, Num c, Num d) { return imax(top(a, b), top(c, d)); }
+// three values along a direction at the largest exponent of theirs
+struct Three {
+  long long m, c, p;
+  int e;
+};
+FX_HD Three three(Num m, Num c, Num p) {
+  const int e = imax(imax(top(m, p), c.e), kExpLo);
+  return Three{at(m, e), at(c, e), at(p, e), e};
+}
 
 // the velocities that a cell reads (l: column x-1, r: x+1, m: row y-1, n: row
-// y+1), at one exponent each; false: out of range
+// y+1); false: out of range
 struct Vels {
-  long long ul, u0, u1, um0, um1, u0n, vl, v0, vr, vm, v0n, vln;
-  int eu, ev, ec, tu, tv;  // ec: the larger one, by tu and tv above theirs
+  Num ul, u0, u1, um0, um1, u0n, vl, v0, vr, vm, v0n, vln;
 };
 FX_HD bool vels(Vels &o, Num ul, Num u0, Num u1, Num um0, Num um1, Num u0n, Num vl, Num v0, Num vr, Num vm, Num v0n,
                 Num vln) {
-  const int a = imax(exponent(ul, u0, u1, um0, um1), u0n.e), b = imax(exponent(vl, v0, vr, vm, v0n), vln.e);
-  const int eu = imax(a, kExpLo), ev = imax(b, kExpLo);
-  o = Vels{at(ul, eu), at(u0, eu), at(u1, eu), at(um0, eu), at(um1, eu),       at(u0n, eu),      at(vl, ev),
-           at(v0, ev), at(vr, ev), at(vm, ev), at(v0n, ev), at(vln, ev),       eu,               ev,
-           imax(eu, ev), imax(ev - eu, 0), imax(eu - ev, 0)};
-  return usable(a) && usable(b);
+  o = Vels{ul, u0, u1, um0, um1, u0n, vl, v0, vr, vm, v0n, vln};
+  return usable(imax(top(ul, u0, u1, um0), top(um1, u0n))) && usable(imax(top(vl, v0, vr, vm), top(v0n, vln)));
 }
 template <bool IMPX, bool IMPY, bool EQ>
 FX_HD Sum sum_ux(const Terms &k, const Weights &w, const Vels &v) {
-  return sum<IMPX, IMPY, EQ>(k, v.eu, v.ec, v.tu, v.tv, v.u0 - v.ul, v.u1 - v.u0, v.u0 - v.um0, v.u0n - v.u0, v.ul + v.u0,
-                         v.u0 + v.u1, twice_mean<EQ>(w, v.vl, v.v0), twice_mean<EQ>(w, v.vln, v.v0n));
+  const Three x = three(v.ul, v.u0, v.u1), y = three(v.um0, v.u0, v.u0n);
+  const int e = imax(top(v.vl, v.v0, v.vln, v.v0n), kExpLo);
+  return sum<IMPX, IMPY, EQ>(k, Line{x.c - x.m, x.p - x.c, x.m + x.c, x.c + x.p, x.e, x.e},
+                             Line{y.c - y.m, y.p - y.c, twice_mean<EQ>(w, at(v.vl, e), at(v.v0, e)),
+                                  twice_mean<EQ>(w, at(v.vln, e), at(v.v0n, e)), y.e, e});
 }
 template <bool IMPX, bool IMPY, bool EQ>
 FX_HD Sum sum_uy(const Terms &k, const Vels &v) {
-  return sum<IMPX, IMPY, EQ>(k, v.ev, v.ec, v.tu, v.tv, v.v0 - v.vl, v.vr - v.v0, v.v0 - v.vm, v.v0n - v.v0, v.um0 + v.u0,
-                         v.um1 + v.u1, v.vm + v.v0, v.v0 + v.v0n);
+  const Three x = three(v.vl, v.v0, v.vr), y = three(v.vm, v.v0, v.v0n);
+  const int e = imax(top(v.um0, v.u0, v.um1, v.u1), kExpLo);
+  return sum<IMPX, IMPY, EQ>(
+      k, Line{x.c - x.m, x.p - x.c, at(v.um0, e) + at(v.u0, e), at(v.um1, e) + at(v.u1, e), x.e, e},
+      Line{y.c - y.m, y.p - y.c, y.m + y.c, y.c + y.p, y.e, y.e});
 }
 // temperature: left, here, right, below, above; the face velocities; false:
 // out of range
 template <bool IMPX, bool IMPY, bool EQ>
 FX_HD bool sum_temp(Sum &r, const Terms &k, Num l, Num c, Num rt, Num d, Num u, Num ul, Num ur, Num vd, Num vu) {
-  const int ef = exponent(l, c, rt, d, u), ev = imax(imax(ul.e, ur.e), imax(vd.e, vu.e));
-  const int E = imax(ef, kExpLo), ec = imax(ev, kExpLo);
-  const long long C = at(c, E);
-  r = sum<IMPX, IMPY, EQ>(k, E, ec, 0, 0, C - at(l, E), at(rt, E) - C, C - at(d, E), at(u, E) - C,
-                          fx::shl(at(ul, ec), 1), fx::shl(at(ur, ec), 1), fx::shl(at(vd, ec), 1),
-                          fx::shl(at(vu, ec), 1));
-  return usable(ef) && usable(ev);
+  const Three x = three(l, c, rt), y = three(d, c, u);
+  const int eu = top(ul, ur), ev = top(vd, vu), ex = imax(eu, kExpLo), ey = imax(ev, kExpLo);
+  r = sum<IMPX, IMPY, EQ>(
+      k, Line{x.c - x.m, x.p - x.c, fx::shl(at(ul, ex), 1), fx::shl(at(ur, ex), 1), x.e, ex},
+      Line{y.c - y.m, y.p - y.c, fx::shl(at(vd, ey), 1), fx::shl(at(vu, ey), 1), y.e, ey});
+  return usable(imax(top(l, c, rt, d), u.e)) && usable(eu) && usable(ev);
 }
 
 }  // namespace sfx
