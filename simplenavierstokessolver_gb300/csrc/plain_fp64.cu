@@ -119,7 +119,7 @@ struct Mul {
 // sub-partition: 24 FP64 operations 1540 cycles a warp, 16 and 8 of these 1240.
 //
 // An operand is m 2^(e - 1084), m signed with its 53 bits from bit 9 up, z the
-// zeros below its lowest one bit (or fewer): the sum is formed at the larger
+// zeros below its lowest one bit (31 for a zero): the sum is formed at the larger
 // exponent, the other operand shifted down with its lost bits, if any, marked
 // in the last bit. That is at least 6 bits below the result's last one after
 // normalisation (bits are lost only by a shift of more than 9, which leaves at
@@ -145,8 +145,12 @@ __device__ __forceinline__ Num num(double d) {
   const unsigned ml = (unsigned)m, mh = (unsigned)(m >> 32);
   return Num{m, e, ml ? __ffs(ml) - 1 : 31 + __ffs(mh)};
 }
-// zero, or normal and far enough from the ends of the range for every result
-__device__ __forceinline__ bool in_range(const Num &a) { return a.m == 0 || (unsigned)(a.e - 128) < 1792u; }
+// d is +0, or normal and far enough from the ends of the range for every
+// result (a holds no sign of a zero, so -0 is left to FP64: sums of two of it
+// are -0)
+__device__ __forceinline__ bool in_range(const Num &a, double d) {
+  return (__double2hiint(d) | __double2loint(d)) == 0 || (unsigned)(a.e - 128) < 1792u;
+}
 __device__ __forceinline__ double round_sum(long long s, int e) {
   const long long n = s >> 63;
   const unsigned long long a = (unsigned long long)((s ^ n) - n);
@@ -321,7 +325,7 @@ __device__ __forceinline__ void temp_column(const TempArgs &a, int x, int y0, in
       n.tl = num(tl);
       n.tr = num(tr);
       n.tp = num(tp);
-      const bool ok = in_range(n.tc) & in_range(n.tl) & in_range(n.tr) & in_range(n.tp);
+      const bool ok = in_range(n.tc, tc) & in_range(n.tl, tl) & in_range(n.tr, tr) & in_range(n.tp, tp);
       if (!temp_row<IMPX, IMPY, RCP, true>(a, k, n, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, o) || k.bad || !ok)
         temp_row<IMPX, IMPY, RCP, false>(a, k, n, tc, gym, pym, tp, tl, tr, uyp, uxm, uxp, atr, o);
       n.tc = n.tp;
@@ -546,7 +550,8 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
     n.v0 = num(in.v0);
     n.vl = num(in.vl);
     n.pm = num(in.pm);
-    ok1 = in_range(n.pm) & in_range(n.u0) & in_range(n.u1) & in_range(n.um0) & in_range(n.um1) & in_range(n.v0) & in_range(n.vl);
+    ok1 = in_range(n.pm, in.pm) & in_range(n.u0, in.u0) & in_range(n.u1, in.u1) & in_range(n.um0, in.um0) &
+          in_range(n.um1, in.um1) & in_range(n.v0, in.v0) & in_range(n.vl, in.vl);
   }
 
   for (int y = y0; y < y1; ++y) {
@@ -580,8 +585,8 @@ __device__ __forceinline__ void vel_march(const VelArgs &a, int x, int y0, int r
       n.pc = num(in.pc);
       n.pl = num(in.pl);
       u1n = num(in.u1n);
-      ok = in_range(n.ul) & in_range(n.u0n) & in_range(n.v0n) & in_range(n.vln) & in_range(n.vr) & in_range(u1n) &
-           in_range(n.pc) & in_range(n.pl);
+      ok = in_range(n.ul, in.ul) & in_range(n.u0n, in.u0n) & in_range(n.v0n, in.v0n) & in_range(n.vln, in.vln) &
+           in_range(n.vr, in.vr) & in_range(u1n, in.u1n) & in_range(n.pc, in.pc) & in_range(n.pl, in.pl);
     }
     if constexpr (FAST) {
       if (!vel_row<IMPX, IMPY, RCP, true, INT>(a, k, in, n, has_ux, o) || k.bad || !(ok & ok1 & ok2))
@@ -1783,7 +1788,7 @@ __global__ void __launch_bounds__(128) k_corr(const CorrArgs a) {
       if constexpr (F) {
         cn.s = num(s0);
         cn.c = num(ps[0]);
-        ok = in_range(cn.s) & in_range(cn.c);
+        ok = in_range(cn.s, s0) & in_range(cn.c, ps[0]);
       }
       if (IMPY) {
         Mul<F> m;
@@ -1799,16 +1804,16 @@ __global__ void __launch_bounds__(128) k_corr(const CorrArgs a) {
         const double sw = left ? sc : pw[i], se = IMPX && !right ? pe[i] : sc;
         if constexpr (F) {
           cn.w = num(sw);
-          ok &= in_range(cn.w);
+          ok &= in_range(cn.w, sw);
           if (IMPX) {
             cn.e = num(se);
-            ok &= in_range(cn.e);
+            ok &= in_range(cn.e, se);
           }
           // the row above, whose value is loaded for the thread's last row only
           // where it enters
           if (IMPY || i + 1 < n) {
             cn.n = num(ps[i + 1]);
-            ok &= in_range(cn.n);
+            ok &= in_range(cn.n, ps[i + 1]);
           }
         }
         ok &= corr_cell<IMPX, IMPY, RCP, F, CORR, PRES>(a.s, k, cn, sc, sw, se, sm, IMPY ? ps[i + 1] : 0.0, gm, o[i]);
