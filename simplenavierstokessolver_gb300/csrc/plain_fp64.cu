@@ -79,11 +79,11 @@ __device__ __forceinline__ int p2_field(double c) { return (((__double2hiint(c) 
 
 // Division by a spacing that is no power of two: x zh + RN(x zl) in one fused
 // multiply-add equals RN(x / y) for the pairs that the host has proven
-// (invariant_divisor): 2 FP64 instructions instead of a division's ~10. The
-// Measured with the marches below: 400 x 512, velocity update 80 -> 45 us. The
-// proof needs numerators away from the ends of the exponent range; others
-// (below 2^-723 and not zero, from 2^877 up, infinities, NaN) clear the row's
-// flag like the products above.
+// (invariant_divisor): 2 FP64 instructions instead of a division's ~10
+// (with the marches below: velocity update 400 x 512 80 -> 45 us). The proof
+// needs numerators away from the ends of the exponent range; others
+// (below 2^-723 and not +0, from 2^877 up, infinities, NaN) clear the row's
+// flag like the products above. (-0 with a negative zl would give +0.)
 constexpr unsigned kDivLo = 300u << 20;
 constexpr unsigned kDivSpan = 1600u << 20;
 
@@ -105,8 +105,8 @@ struct Mul {
   __device__ __forceinline__ double half(double x) { return by(x, 0.5, -(1 << 20)); }
   // x / y by its pair (zh, zl); FAST only
   __device__ __forceinline__ double div(double x, double zh, double zl) {
-    const unsigned m = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    ok &= ((m | (unsigned)__double2loint(x)) == 0u) | (m - kDivLo < kDivSpan);
+    const int hi = __double2hiint(x);
+    ok &= ((hi | __double2loint(x)) == 0) | (((unsigned)hi & 0x7fffffffu) - kDivLo < kDivSpan);
     return __fma_rn(x, zh, __dmul_rn(x, zl));
   }
 };
