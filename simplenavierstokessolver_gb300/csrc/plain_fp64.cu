@@ -19,6 +19,7 @@
 #include <type_traits>
 
 #include "fft_dev.cuh"
+#include "smem_grant.h"
 #include "sns_internal.h"
 #include "chain.cuh"
 #ifdef SNS_PLAIN_CONTRACT
@@ -2047,6 +2048,7 @@ cudaError_t launch_velocity_update(const DevGrid &g, const StageScalars &s, int 
 // a quarter of its line, or lines too long for shared memory. The segment
 // length: the least of the FP64 issue of all rows, warm-up included, and one
 // thread's chain (in FP64 instructions of a sub-partition).
+constexpr size_t kSegSmem = 200 * 1024;
 static bool seg_shape(bool cols, int n, int total, int nl, int warm, SegArgs &a, size_t *smem, int *threads) {
   a.warm = warm + 1;
   if (n < 32 || a.warm > n / 4) return false;
@@ -2068,7 +2070,7 @@ static bool seg_shape(bool cols, int n, int total, int nl, int warm, SegArgs &a,
   const size_t line = sizeof(double) * (size_t)(cols ? rows : a.stride);
   *smem = line << a.lgC;
   *threads = ((a.nseg << a.lgC) + 31) / 32 * 32;
-  return *smem <= 200 * 1024 && *threads <= kSegThreads;
+  return *smem <= kSegSmem && *threads <= kSegThreads;
 }
 
 // the increments of a set whose lines were swept serially
@@ -2096,11 +2098,7 @@ cudaError_t launch_solve_x_set(const DevGrid &g, const SolveXSet &set, cudaStrea
     warm = std::max(warm, set.f[k].warm);
   }
   if (seg_shape(false, g.nx, g.nx, g.ny * set.n, warm, a, &smem, &threads)) {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(k_solve_seg<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      attr = true;
-    }
+    if (cudaError_t e = allow_smem(k_solve_seg<false>, smem, kSegSmem)) return e;
     chain_launch(k_solve_seg<false>, dim3((g.ny + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st, g.nx, g.ny, a);
   } else {
     chain_launch(k_solve_x, dim3((g.ny + 31) / 32, set.n), 32, 0, st, g.nx, g.ny, set);
@@ -2123,11 +2121,7 @@ cudaError_t launch_solve_y_set(const DevGrid &g, const SolveYSet &set, cudaStrea
     warm = std::max(warm, set.f[k].sub.warm);
   }
   if (seg_shape(true, g.ny - 1, g.ny, g.nx * set.n, warm, a, &smem, &threads)) {
-    static bool attr = false;
-    if (!attr) {
-      cudaFuncSetAttribute(k_solve_seg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-      attr = true;
-    }
+    if (cudaError_t e = allow_smem(k_solve_seg<true>, smem, kSegSmem)) return e;
     chain_launch(k_solve_seg<true>, dim3((g.nx + (1 << a.lgC) - 1) >> a.lgC, set.n), threads, smem, st, g.nx, g.ny, a);
   } else {
     chain_launch(k_solve_y, dim3((g.nx + 31) / 32, set.n), 32, 0, st, g.nx, g.ny, set);
@@ -2352,43 +2346,24 @@ cudaError_t launch_tempforce_to_host(const DevGrid &g, const double *t, double *
   return cudaGetLastError();
 }
 
-static int poisson_setup(const DevGrid &g, size_t *smem) {
-  const int C = poisson_cols(g);
-  *smem = (size_t)C * g.ny * sizeof(double);
-  static bool attr_set = false;
-  if (!attr_set) {
-    const int lim = 160 * 1024;
-    cudaFuncSetAttribute(k_poisson_fwd<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_poisson_fwd<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    cudaFuncSetAttribute(k_poisson_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    attr_set = true;
-  }
-  return C;
-}
+constexpr size_t kPoissonSmem = 160 * 1024;
 
 cudaError_t launch_poisson_fwd(const DevGrid &g, const StageScalars &s, const double *ux, const double *uy,
                                double2 *spec, cudaStream_t st) {
-  size_t smem;
-  const int C = poisson_setup(g, &smem);
+  const int C = poisson_cols(g);
+  const size_t smem = (size_t)C * g.ny * sizeof(double);
   const PoissonArgs a{g, s, ux, uy, spec, nullptr, C};
   const int blocks = (g.nx + C - 1) / C;
-  if (g.rcp) {
-    chain_launch(k_poisson_fwd<true>, blocks, poisson_threads(g, C), smem, st, a);
-  } else {
-    chain_launch(k_poisson_fwd<false>, blocks, poisson_threads(g, C), smem, st, a);
-  }
+  const auto kernel = g.rcp ? k_poisson_fwd<true> : k_poisson_fwd<false>;
+  if (cudaError_t e = allow_smem(kernel, smem, kPoissonSmem)) return e;
+  chain_launch(kernel, blocks, poisson_threads(g, C), smem, st, a);
   count_launches(1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_poisson_tri(const DevGrid &g, double2 *spec, cudaStream_t st) {
-  static bool attr = false;
   const size_t smem = sizeof(TriRing) + sizeof(double) * (size_t)g.nx;
-  if (!attr) {
-    cudaFuncSetAttribute(k_poisson_tri, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(sizeof(TriRing) + sizeof(double) * (size_t)kTriMaxNx));
-    attr = true;
-  }
+  if (cudaError_t e = allow_smem(k_poisson_tri, smem, sizeof(TriRing) + sizeof(double) * (size_t)kTriMaxNx)) return e;
   chain_launch(k_poisson_tri, dim3((g.nh + 31) / 32, 2), 32, smem, st, g, spec);
   count_launches(1);
   return cudaGetLastError();
@@ -2428,16 +2403,14 @@ cudaError_t launch_poisson_fused(const DevGrid &g, const StageScalars &s, const 
   }
   const size_t smem = std::max({sizeof(double) * (size_t)g.nx, teams * cols, kFusedMinSmem});
   if (!coop || g.nx > kTriMaxNx || smem > max_smem || sms - tri_blocks < 8) return cudaErrorNotSupported;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_poisson_fused<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_poisson_fused<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
+  // both forms, which loads them one after the other: loaded each at its first
+  // launch, between other kernels, the second took 1 to 2 % longer (512 x 1024
+  // after a grid of the other kind 139.5 -> 141.9 us)
+  if ((e = allow_smem(k_poisson_fused<true>, smem, max_smem)) != cudaSuccess) return e;
+  if ((e = allow_smem(k_poisson_fused<false>, smem, max_smem)) != cudaSuccess) return e;
+  const auto kernel = g.rcp ? k_poisson_fused<true> : k_poisson_fused<false>;
   int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, g.rcp ? (const void *)k_poisson_fused<true>
-                                                                        : (const void *)k_poisson_fused<false>,
-                                                         kFusedThreads, smem)) != cudaSuccess)
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kFusedThreads, smem)) != cudaSuccess)
     return e;
   if (per_sm < 1) return cudaErrorNotSupported;
   FusedArgs a{};
@@ -2459,8 +2432,7 @@ cudaError_t launch_poisson_fused(const DevGrid &g, const StageScalars &s, const 
   // the larger span when the workers can take all of its column groups at once
   a.span_shift = ((1 << kFusedSpanShiftMax) / C <= (sms - tri_blocks) * teams) ? kFusedSpanShiftMax : kFusedSpanShiftMax - 1;
   void *args[] = {&a};
-  e = cudaLaunchCooperativeKernel(g.rcp ? (const void *)k_poisson_fused<true> : (const void *)k_poisson_fused<false>,
-                                  dim3(sms), dim3(kFusedThreads), args, smem, st);
+  e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(sms), dim3(kFusedThreads), args, smem, st);
   if (e != cudaSuccess) {
     --fs.epoch;
     return e;
@@ -2471,10 +2443,11 @@ cudaError_t launch_poisson_fused(const DevGrid &g, const StageScalars &s, const 
 
 cudaError_t launch_poisson_bwd(const DevGrid &g, const StageScalars &s, const double2 *spec, double *psi,
                                cudaStream_t st) {
-  size_t smem;
-  const int C = poisson_setup(g, &smem);
+  const int C = poisson_cols(g);
+  const size_t smem = (size_t)C * g.ny * sizeof(double);
   const PoissonArgs a{g, s, nullptr, nullptr, const_cast<double2 *>(spec), psi, C};
   const int blocks = (g.nx + C - 1) / C;
+  if (cudaError_t e = allow_smem(k_poisson_bwd, smem, kPoissonSmem)) return e;
   chain_launch(k_poisson_bwd, blocks, poisson_threads(g, C), smem, st, a);
   count_launches(1);
   return cudaGetLastError();

@@ -35,6 +35,7 @@
 #include "fft_fixed.cuh"
 #include "host_common.h"
 #include "sns_gpu.h"
+#include "smem_grant.h"
 #include "sns_internal.h"
 #include "chain.cuh"
 
@@ -768,18 +769,7 @@ namespace {
 // the fixed-point pair: 16 <= jtot <= 8192 (at most 512 threads a block)
 bool par_fixed(const DevGrid &g) { return g.ny >= 16 && g.ny <= 8192; }
 
-void par_dft_attributes() {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_par_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    cudaFuncSetAttribute(k_par_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
-    cudaFuncSetAttribute(k_par_fwd_fx<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
-    cudaFuncSetAttribute(k_par_bwd_fx<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
-    cudaFuncSetAttribute(k_par_fwd_fx<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
-    cudaFuncSetAttribute(k_par_bwd_fx<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024);
-    attr = true;
-  }
-}
+constexpr size_t kParDftSmem = 160 * 1024, kFixSmem = 80 * 1024;
 
 // values per thread, columns per block (log2) and threads of the fixed-point
 // pair: jtot / 2V threads a column. One warp's instruction latency bounds the
@@ -822,30 +812,25 @@ FixShape fix_shape(const DevGrid &g) {
 
 cudaError_t launch_par_fwd(const DevGrid &g, const StageScalars &s, const double *ux, const double *uy,
                            double2 *spec, cudaStream_t st) {
-  par_dft_attributes();
   if (par_fixed(g)) {
     const FixShape f = fix_shape(g);
     const FixArgs a{g, ux, uy, spec, nullptr, 0.0, f.lgC, g.nx / kPartSeg};
     const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
-    if (f.v == 8) chain_launch(k_par_fwd_fx<8>, blocks, f.threads, f.smem, st, a);
-    else if (f.v == 2) chain_launch(k_par_fwd_fx<2>, blocks, f.threads, f.smem, st, a);
-    else chain_launch(k_par_fwd_fx<4>, blocks, f.threads, f.smem, st, a);
+    const auto kernel = f.v == 8 ? k_par_fwd_fx<8> : f.v == 2 ? k_par_fwd_fx<2> : k_par_fwd_fx<4>;
+    if (cudaError_t e = allow_smem(kernel, f.smem, kFixSmem)) return e;
+    chain_launch(kernel, blocks, f.threads, f.smem, st, a);
   } else {
     const int C = par_cols(g);
     const ParArgs a{g, s, ux, uy, spec, nullptr, C, g.nx / kPartSeg};
-    chain_launch(k_par_fwd, (g.nx + C - 1) / C, par_threads(g, C), (size_t)C * g.ny * sizeof(double), st, a);
+    const size_t smem = (size_t)C * g.ny * sizeof(double);
+    if (cudaError_t e = allow_smem(k_par_fwd, smem, kParDftSmem)) return e;
+    chain_launch(k_par_fwd, (g.nx + C - 1) / C, par_threads(g, C), smem, st, a);
   }
   count_launches(1);
   return cudaGetLastError();
 }
 
 cudaError_t launch_par_tri(const DevGrid &g, double2 *spec, const ParFactors &pf, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_par_tri<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kParSmemMax);
-    cudaFuncSetAttribute(k_par_tri<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kParSmemMax);
-    attr = true;
-  }
   const bool staged = par_staged(g.nx, pf.stride);
   const size_t per_line = 16 * (size_t)g.nx + (staged ? 8 * pf.stride : 0);
   // mode lines per block, two warps each
@@ -854,11 +839,9 @@ cudaError_t launch_par_tri(const DevGrid &g, double2 *spec, const ParFactors &pf
   const ParTriArgs a{spec,  pf.fac, pf.lo, pf.hi, pf.stride, g.nx, g.nh, g.nx / kPartSeg, pf.err, pf.spin_limit,
                      pf.stale};
   const size_t smem = 128 + (size_t)lpb * per_line;
-  if (staged) {
-    chain_launch(k_par_tri<true>, (g.nh + lpb - 1) / lpb, 64 * lpb, smem, st, a);
-  } else {
-    chain_launch(k_par_tri<false>, (g.nh + lpb - 1) / lpb, 64 * lpb, smem, st, a);
-  }
+  const auto kernel = staged ? k_par_tri<true> : k_par_tri<false>;
+  if (cudaError_t e = allow_smem(kernel, smem, kParSmemMax)) return e;
+  chain_launch(kernel, (g.nh + lpb - 1) / lpb, 64 * lpb, smem, st, a);
   count_launches(1);
   return cudaGetLastError();
 }
@@ -875,11 +858,6 @@ bool parallel_cn_supported(int n) {
 }
 
 cudaError_t launch_par_cn(bool columns, ParCnArgs a, cudaStream_t st) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_par_cn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kParSmemMax);
-    attr = true;
-  }
   if (!parallel_cn_supported(a.n) || a.nf < 1 || a.nf > 3) return cudaErrorInvalidValue;
   a.m = a.n / kPartSeg;
   a.s = a.m | 1;
@@ -892,6 +870,7 @@ cudaError_t launch_par_cn(bool columns, ParCnArgs a, cudaStream_t st) {
     int wpb = (int)std::min<size_t>(kCnWarpsMax, (kParSmemMax / 2) / per);
     if (wpb < 1) wpb = 1;
     const dim3 grid((a.lines + wpb - 1) / wpb, a.nf);
+    if (cudaError_t e = allow_smem(k_par_cn, wpb * per, kParSmemMax)) return e;
     chain_launch(k_par_cn, grid, 32 * wpb, wpb * per, st, a);
   }
   count_launches(1);
@@ -900,19 +879,20 @@ cudaError_t launch_par_cn(bool columns, ParCnArgs a, cudaStream_t st) {
 
 cudaError_t launch_par_bwd(const DevGrid &g, const StageScalars &s, const double2 *spec, double *psi,
                            cudaStream_t st) {
-  par_dft_attributes();
   if (par_fixed(g)) {
     const FixShape f = fix_shape(g);
     const FixArgs a{g,     nullptr, nullptr, const_cast<double2 *>(spec), psi, s.rgdt * (0.5 * s.rny),
                     f.lgC, g.nx / kPartSeg};
     const int blocks = (g.nx + (1 << f.lgC) - 1) >> f.lgC;
-    if (f.v == 8) chain_launch(k_par_bwd_fx<8>, blocks, f.threads, f.smem, st, a);
-    else if (f.v == 2) chain_launch(k_par_bwd_fx<2>, blocks, f.threads, f.smem, st, a);
-    else chain_launch(k_par_bwd_fx<4>, blocks, f.threads, f.smem, st, a);
+    const auto kernel = f.v == 8 ? k_par_bwd_fx<8> : f.v == 2 ? k_par_bwd_fx<2> : k_par_bwd_fx<4>;
+    if (cudaError_t e = allow_smem(kernel, f.smem, kFixSmem)) return e;
+    chain_launch(kernel, blocks, f.threads, f.smem, st, a);
   } else {
     const int C = par_cols(g);
     const ParArgs a{g, s, nullptr, nullptr, const_cast<double2 *>(spec), psi, C, g.nx / kPartSeg};
-    chain_launch(k_par_bwd, (g.nx + C - 1) / C, par_threads(g, C), (size_t)C * g.ny * sizeof(double), st, a);
+    const size_t smem = (size_t)C * g.ny * sizeof(double);
+    if (cudaError_t e = allow_smem(k_par_bwd, smem, kParDftSmem)) return e;
+    chain_launch(k_par_bwd, (g.nx + C - 1) / C, par_threads(g, C), smem, st, a);
   }
   count_launches(1);
   return cudaGetLastError();
