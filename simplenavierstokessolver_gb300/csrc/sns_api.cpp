@@ -103,7 +103,7 @@ struct Context {
   double *staging = nullptr;     // pinned, nx*ny doubles
   unsigned long long *red_host = nullptr;  // pinned, nx+1 words
   double *diag_host = nullptr;  // behind them: the results of sns_diagnostics
-  std::mutex diag_mu;           // over a call's launches, its wait and its reading of diag_host
+  std::mutex diag_mu;           // over a call: the partials' allocation, launches, wait and reading of diag_host
   // factors for the implicit solves: device buffer, and a ring of pinned host
   // staging slots so that the uploads are asynchronous; a slot is rewritten
   // only after its previous upload completed (fac_ev)
@@ -2166,6 +2166,7 @@ int sns_diagnostics(const param_t *param, const fluid_t *fluid, const temperatur
   TempExt *te = as_temp(temperature);
   if (!param || !fe || !te || !out) return fail(SNS_ERR_ARG, "sns_diagnostics: bad argument");
   Context *c = fe->ctx;
+  std::lock_guard<std::mutex> lk(c->diag_mu);
   if (int rc = flush_pending(c)) return rc;
   const int nx = c->nx, ny = c->ny;
   if (!c->diag)
@@ -2174,7 +2175,6 @@ int sns_diagnostics(const param_t *param, const fluid_t *fluid, const temperatur
   const DiagArgs<double> a{nx, ny, param->dy, param->ly, sqrt(Pr) * sqrt(Ra), sqrt(Pr) / sqrt(Ra),
                            1. / sqrt(Pr) / sqrt(Ra), c->g.dxf, c->g.dxc, fe->f.ux, fe->f.uy, te->f.t[te->cur]};
   double *res = nullptr;
-  std::lock_guard<std::mutex> lk(c->diag_mu);
   SNS_CUDA(launch_diag(a, c->diag, &res, c->stream, c->diag_host));
   count_launches(2);
   SNS_CUDA(cudaStreamSynchronize(c->stream));
