@@ -86,8 +86,10 @@ static CaseLayout layout_for(int nx, int ny, bool x2) {
   L.dxi = take(sizeof(double) * (nx + 1));
   L.dxf = take(sizeof(double) * nx);
   L.dxc = take(sizeof(double) * (nx + 1));
-  L.tw = take(sizeof(double) * 2 * ny);
-  L.twx = take(sizeof(int32_t) * 4 * ny);
+  // jtot 8 takes the FP64 DFTs alone, 16 to 4096 the fixed-point ones alone, so
+  // one table serves both names; 8192 takes FP64 in the persistent launch
+  L.twx = L.tw = take(sizeof(double) * 2 * ny);
+  if (ny == 8192) L.twx = take(sizeof(int32_t) * 4 * ny);
   L.lo = take(sizeof(double) * nx);
   L.hi = take(sizeof(double) * nx);
   L.ccm = take(sizeof(double) * nx);
@@ -519,7 +521,7 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
     dxi[i - 1] = 1. / DXC(i);
   }
   const std::vector<double> tw = twiddle_table(ny);
-  const std::vector<int32_t> twx = fixed_twiddles(ny);
+  const std::vector<int32_t> twx = ny > 8 ? fixed_twiddles(ny) : std::vector<int32_t>();
   std::vector<char> small(L.small, 0);
   auto keep = [&](size_t o, const void *src, size_t bytes) { std::memcpy(small.data() + o, src, bytes); };
   keep(L.rdxf_f, rdxf_f.data(), sizeof(float) * nx);
@@ -534,8 +536,8 @@ static int admit(sns_batch *b, const sns_case_desc *d, const double *temp_init, 
   keep(L.dxi, dxi.data(), sizeof(double) * (nx + 1));
   keep(L.dxf, dxf.data(), sizeof(double) * nx);
   keep(L.dxc, dxc.data(), sizeof(double) * (nx + 1));
-  keep(L.tw, tw.data(), sizeof(double) * tw.size());
-  keep(L.twx, twx.data(), sizeof(int32_t) * twx.size());
+  if (ny == 8 || ny == 8192) keep(L.tw, tw.data(), sizeof(double) * tw.size());
+  if (ny > 8) keep(L.twx, twx.data(), sizeof(int32_t) * twx.size());
   keep(L.lo, lo.data(), sizeof(double) * nx);
   keep(L.hi, hi.data(), sizeof(double) * nx);
   keep(L.ccm, ccm_d.data(), sizeof(double) * nx);
