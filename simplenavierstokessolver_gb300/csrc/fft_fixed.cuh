@@ -20,7 +20,8 @@
 // largest value of the pass. Over transforms of 8 to 4096 complex values the
 // error is 0.2 to 0.6 of that of the FP64 transform it replaces (0.7 for
 // delta columns of 8192 rows and, with radix 2, 64 rows inverted), for noise, smooth, single-mode, delta
-// and wide-range columns (tests/test_fft_fixed.py measures both against an
+// and wide-range columns (tests/test_fft_fixed.py and, for radix 4, 0.1 to 0.73,
+// tests/test_fft_radix4.py measure both against an
 // extended-precision DFT).
 //
 // Stockham passes of radix V = 8, 4 or 2 (then one of radix 4 or 2), V values per
