@@ -9,7 +9,9 @@
 namespace sns {
 
 constexpr int kDiagSums = 10;  // compensated sums per block
-constexpr int kDiagRows = 16;  // rows of diag_blocks
+// rows of a block as diag_blocks counts them, which is what the static form
+// accepts grids by (launches take 1 to 32)
+constexpr int kDiagRows = 16;
 
 // dense fields (x fastest, no halos), metrics as DXF(i) = dxf[i-1], DXC(i) = dxc[i-1]
 template <typename F>

@@ -3,8 +3,9 @@
 // stencils of src/analyses.c:8-121): maximum and sum of the divergence,
 // x/y momentum, kinetic (x, y) and thermal energy, and the Nusselt number
 // from the wall heat flux, the energy injection, the kinetic and the thermal
-// dissipation. All arithmetic is FP64; every sum is accumulated
-// exactly per thread, rounded to a pair of doubles, merged per block and over the
+// dissipation. The terms are FP64; a thread's sums of them are 128-bit
+// integers, exact but for what terms below 2^-37 of the largest one hold beneath
+// 2^-89 of it, then rounded to a pair of doubles, merged per block and over the
 // blocks with the compensation carried along, so the result agrees with the
 // reference's sequential sums to their own round-off. Fields may be FP64
 // (plain path) or FP32 (batched form); FP32 values are widened exactly.
@@ -70,13 +71,15 @@ __device__ __forceinline__ bool pow2(double d) {
   return __double2loint(d) == 0 && (__double2hiint(d) & 0xfffff) == 0;
 }
 
-// A sum of doubles without rounding: a 128-bit integer in units of
-// 2^(e - 1132), so that the 53 bits of a term whose biased exponent is e reach
-// from bit 57 up and 16 bits are left above for 65536 terms. A term with a
-// larger exponent than e moves the sum down first, to an exponent 20 above its
-// own, so that few threads of a warp ever do it after their first row. Terms
-// are cut off at 2^-90 of the largest one or below. Infinities and NaN make the
-// sum NaN, as the compensated sum's (inf - inf).
+// A sum of doubles as a 128-bit integer in units of 2^(e - 1132), so that the 53
+// bits of a term whose biased exponent is e reach from bit 57 up and 16 bits are
+// left above for 65536 terms. A term with a larger exponent than e moves the sum
+// down first, to an exponent 20 above its own, so that few threads of a warp
+// ever do it after their first row. The unit is then 2^-89 of that term at most:
+// terms down to 2^-37 of the largest one enter whole, smaller ones and the sum
+// are cut off (towards minus infinity) at the unit, so a sum whose large terms
+// cancel to less than that loses them. Infinities and NaN make the sum NaN, as
+// the compensated sum's (inf - inf).
 __device__ __forceinline__ long long shr(long long v, int s) {  // amounts of 64 and more leave the sign
   long long r;
   asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
