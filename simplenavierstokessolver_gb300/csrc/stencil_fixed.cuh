@@ -104,10 +104,19 @@ struct Val {
   long long v;
   int e;
 };
-// their sum at the larger exponent; |v| < 2^63 together
+// their sum at the largest exponent; |v| < 2^63 together
 FX_HD Val add(Val a, Val b) {
   const int t = a.e - b.e;
   return Val{shr(a.v, imax(-t, 0)) + shr(b.v, imax(t, 0)), imax(a.e, b.e)};
+}
+// (four at once: 512 x 1024 velocity update 31.6 us, two by two 32.8)
+FX_HD Val add(Val a, Val b, Val c) {
+  const int e = imax(imax(a.e, b.e), c.e);
+  return Val{shr(a.v, e - a.e) + shr(b.v, e - b.e) + shr(c.v, e - c.e), e};
+}
+FX_HD Val add(Val a, Val b, Val c, Val d) {
+  const int e = imax(imax(a.e, b.e), imax(c.e, d.e));
+  return Val{shr(a.v, e - a.e) + shr(b.v, e - b.e) + (shr(c.v, e - c.e) + shr(d.v, e - d.e)), e};
 }
 // |v| < 2^63, e - 62 and e + 1 exponents of normal numbers
 FX_HD double to_double(Val x) {
@@ -226,26 +235,16 @@ FX_HD Sum sum(const Terms &k, const Line &X, const Line &Y) {
   const int gx = room(size(X.dm) | size(X.dp)), gy = room(size(Y.dm) | size(Y.dp));
   const Split xm = split(fx::shl(X.dm, gx)), xp = split(fx::shl(X.dp, gx));
   const Split ym = split(fx::shl(Y.dm, gy)), yp = split(fx::shl(Y.dp, gy));
-  const Val adv = add(advective(xm, xp, gx, X.sm, X.sp, k.ax, k.eax + X.es + X.ed),
-                      advective(ym, yp, gy, Y.sm, Y.sp, k.ay, k.eay + Y.es + Y.ed));  // <= 2^61
+  const Val ax = advective(xm, xp, gx, X.sm, X.sp, k.ax, k.eax + X.es + X.ed);
+  const Val ay = advective(ym, yp, gy, Y.sm, Y.sp, k.ay, k.eay + Y.es + Y.ed);  // <= 2^60
   Val x = diffusive((k.tm ? X.dp >> 1 : X.dp) - (k.tp ? X.dm >> 1 : X.dm), k.cx, k.ecx + X.ed);
   const Val y = diffusive(Y.dp - Y.dm, k.cy, k.ecy + Y.ed);
   if (!EQ) x = add(x, Val{prod(k.tp ? xp : xm, k.ex), k.ee + X.ed - gx});  // <= 2^61
-  Sum r;
-  r.A = adv;
-  r.G = Val{0, 0};
-  if (IMPX && IMPY) {
-    r.G = add(x, y);
-  } else if (IMPX) {
-    r.A = add(adv, y);
-    r.G = x;
-  } else if (IMPY) {
-    r.A = add(adv, x);
-    r.G = y;
-  } else {
-    r.A = add(adv, add(x, y));  // <= 2^61 + 2^61 + 2^60
-  }
-  return r;
+  // sums of at most 2^62 + 2^60
+  if (IMPX && IMPY) return Sum{add(ax, ay), add(x, y)};
+  if (IMPX) return Sum{add(ax, ay, y), x};
+  if (IMPY) return Sum{add(ax, ay, x), y};
+  return Sum{add(ax, ay, x, y), Val{0, 0}};
 }
 
 // the interpolation weights of a vertical velocity (in (0, 1)) times 2^62
