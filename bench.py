@@ -75,20 +75,21 @@ KERNEL_MODEL = {
 }
 
 
-# DRAM bytes (read + write) per launch from ncu captures of the default
-# workload with warm caches, keyed by kernel and size (the fields stay in L2
-# between kernels at this size): the parallel form's kernels and the exact
-# form's fused launch from profiles/plain_parallel_fp64_counts_512x1024.md, the
-# exact form's three-kernel Poisson solve from an earlier capture
+# DRAM bytes (read + write) per launch, mean of a step's three launches, from
+# ncu captures of this program's own steps with its L2 flush before each
+# (profiles/plain_dram_512x1024.md): the first substage reads the fields from
+# HBM, the other two from L2. Bytes written include the flush's own lines, which
+# L2 writes back as the step needs their place. Keyed by form, kernel and size.
 PROFILED_TRAFFIC = {
-    ("poisson_fused", 512, 1024): 5625600 + 117760,
-    ("poisson_tridiagonal", 512, 1024): 8665344,
-    ("velocity_update", 512, 1024): 4151552 + 1280,
-    ("poisson_forward_fft", 512, 1024): 58624,
-    ("poisson_pcr", 512, 1024): 11863040,
-    ("temperature_update", 512, 1024): 4055552,
-    ("poisson_inverse_fft", 512, 1024): 1857280,
-    ("correct_and_pressure", 512, 1024): 36864,
+    ("parallel", "velocity_update", 512, 1024): 12804181,
+    ("parallel", "temperature_update", 512, 1024): 3976832,
+    ("parallel", "poisson_forward_fft", 512, 1024): 3534805,
+    ("parallel", "poisson_pcr", 512, 1024): 5609002,
+    ("parallel", "poisson_inverse_fft", 512, 1024): 2640512,
+    ("parallel", "correct_and_pressure", 512, 1024): 1356288,
+    ("exact", "velocity_update", 512, 1024): 14614826,
+    ("exact", "poisson_fused", 512, 1024): 12513962,
+    ("exact", "correct_and_pressure", 512, 1024): 1312554,
 }
 
 
@@ -893,7 +894,7 @@ def gpu_arm(args, world, rank, local):
     achieved = bpc * cells / avg_s / 1e9 if bpc else None
     roofline = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if achieved else None,
-                "traffic": PROFILED_TRAFFIC.get((dom, args.nx, args.ny)),
+                "traffic": PROFILED_TRAFFIC.get((form, dom, args.nx, args.ny)),
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured" else "fallback",
                 "algorithmic_bytes_per_launch": bpc * cells if bpc else None,
                 "note": "instruction issue (FP64 and integer pipes) bounds it on GB300: see fp64_roofline"}
