@@ -4,8 +4,8 @@
 // x/y momentum, kinetic (x, y) and thermal energy, and the Nusselt number
 // from the wall heat flux, the energy injection, the kinetic and the thermal
 // dissipation. The terms are FP64; a thread's sums of them are 128-bit
-// integers, exact but for what terms below 2^-37 of the largest one hold beneath
-// 2^-89 of it, then rounded to a pair of doubles, merged per block and over the
+// integers, exact but for what terms below 2^-47 of the largest one hold beneath
+// 2^-99 of it, then rounded to a pair of doubles, merged per block and over the
 // blocks with the compensation carried along, so the result agrees with the
 // reference's sequential sums to their own round-off. Fields may be FP64
 // (plain path) or FP32 (batched form); FP32 values are widened exactly.
@@ -71,15 +71,15 @@ __device__ __forceinline__ bool pow2(double d) {
   return __double2loint(d) == 0 && (__double2hiint(d) & 0xfffff) == 0;
 }
 
-// A sum of doubles as a 128-bit integer in units of 2^(e - 1132), so that the 53
-// bits of a term whose biased exponent is e reach from bit 57 up and 16 bits are
-// left above for 65536 terms. A term with a larger exponent than e moves the sum
-// down first, to an exponent 20 above its own, so that few threads of a warp
-// ever do it after their first row. The unit is then 2^-89 of that term at most:
-// terms down to 2^-37 of the largest one enter whole, smaller ones and the sum
-// are cut off (towards minus infinity) at the unit, so a sum whose large terms
-// cancel to less than that loses them. Infinities and NaN make the sum NaN, as
-// the compensated sum's (inf - inf).
+// A sum of doubles as a 128-bit integer in units of 2^(e - 1142): a term's 53
+// bits reach from bit 67 - s up, s >= 3 its biased exponent's distance from e, so
+// that 10 bits are left above for 1023 terms (a thread adds 64 at most). A term
+// too close to e moves the sum down first, to an exponent 20 above its own, so
+// that few threads of a warp ever do it after their first row. The unit is then
+// 2^-99 of that term: terms down to 2^-47 of the largest one enter whole, smaller
+// ones and the sum are cut off (towards minus infinity) at the unit. A compensated
+// FP64 sum of a thread's terms holds 2^-98 of their magnitudes in the worst case.
+// Infinities and NaN make the sum NaN, as the compensated sum's (inf - inf).
 __device__ __forceinline__ long long shr(long long v, int s) {  // amounts of 64 and more leave the sign
   long long r;
   asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
@@ -93,6 +93,8 @@ __device__ __forceinline__ unsigned long long shl(long long v, int s) {  // amou
 struct Sum128 {
   static constexpr int kNan = 8192;  // e of a sum that is NaN
   static constexpr int kMargin = 20;
+  static constexpr int kRoom = 3;   // least distance of e from a term's exponent
+  static constexpr int kStart = 4;  // e of an empty sum (exponent 0 counts as 1)
   unsigned long long lo;
   long long hi;
   int e;
@@ -106,16 +108,16 @@ struct Sum128 {
   __device__ __forceinline__ void add(double v) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(v);
     const int ev = (int)(b >> 52) & 0x7ff;
-    if (ev > e) raise(ev);
+    if (ev + kRoom > e) raise(ev);
     long long m = (long long)((b & 0xfffffffffffffull) | (ev ? 1ull << 52 : 0ull));
     if (!NONNEG) {
       const long long n = (long long)b >> 63;
       m = (m ^ n) - n;
     }
     const int s = e - max(ev, 1);
-    const unsigned long long l = s <= 57 ? shl(m, 57 - s) : (unsigned long long)shr(m, s - 57);
+    const unsigned long long l = s <= 67 ? shl(m, 67 - s) : (unsigned long long)shr(m, s - 67);
     const unsigned long long t = lo + l;
-    hi += shr(m, s + 7) + (t < l);
+    hi += shr(m, s - kRoom) + (t < l);
     lo = t;
   }
   // times f, as a pair of doubles whose sum it is to 2^-106
@@ -137,7 +139,7 @@ struct Sum128 {
       h = h << z | l >> (64 - z);
       l <<= z;
     }
-    const int k = e - 1132 + 75 - z;  // of the first double's last bit
+    const int k = e - 1142 + 75 - z;  // of the first double's last bit
     const unsigned long long m0 = h >> 11, m1 = (h & 0x7ff) << 42 | l >> 22;
     // m 2^q without FP64 instructions; m's top bit is bit 52 - up
     auto value = [&](unsigned long long m, int q, int up) {
@@ -180,7 +182,7 @@ __global__ void __launch_bounds__(kDiagThreads, 8) k_diag(DiagArgs<F> a, double 
     const double rdy = 1.0 / dy, rdxf = 1.0 / dxf;
     const bool p2 = pow2(dy) && pow2(dxf);  // products by the reciprocals are the divisions
     const double wall = last ? dxc / dxw : 0.0;  // the wall face's weight to the column's west face's
-    Sum128 su{0, 0, 1}, suu = su, inj = su, div = su, sv = su, svv = su, stt = su, flux = su;
+    Sum128 su{0, 0, Sum128::kStart}, suu = su, inj = su, div = su, sv = su, svv = su, stt = su, flux = su;
     Sum128 ux2 = su, uy2 = su, vx2 = su, vy2 = su, tx2 = su, ty2 = su;
     size_t r = (size_t)y0 * nx + x;
     double u = first ? 0.0 : LD(a.ux, a.uxl, r), v = LD(a.uy, a.uyl, r), t = LD(a.t, a.tl, r);
